@@ -31,6 +31,7 @@
 #include "nbg_common.cuh"
 #include "nbg_internal.h"
 #include "nbg_query.cuh"
+#include "nbg_tie.cuh"
 
 namespace nbg {
 
@@ -182,10 +183,8 @@ __global__ void __launch_bounds__(128) knn_fused_kernel(const QueryArgs a) {
 }
 
 // Split form, pass 1 + pass 2: the row's exact neighbourhood sums, in sorted
-// order (cnt = 0 marks a row handed to the exact path).  With FINISH the row
-// is finished in place instead and its sums are not written (the handed-back
-// rows of the single-pass select, whose sums slot already holds cnt = 0).
-template <int KS, bool FINISH = false>
+// order (cnt = 0 marks a row handed to the exact path).
+template <int KS>
 __device__ __forceinline__ void select_row(const QueryArgs& a, const uint64_t i) {
     const GridParams g = *a.gp;
     const float4 q = __ldg(&a.gv.sorted[i]);
@@ -197,11 +196,9 @@ __device__ __forceinline__ void select_row(const QueryArgs& a, const uint64_t i)
         const int32_t qraw[3] = {__float2int_rz(q.x) + g.minx, __float2int_rz(q.y) + g.miny,
                                  __float2int_rz(q.z) + g.minz};
         nbg_finish_row(a.grp, a.tf, a.ex, id, 0, M, qraw);
-        if (!FINISH) {
-            RowSums z;
-            z.cnt = 0;
-            a.sums[i] = z;
-        }
+        RowSums z;
+        z.cnt = 0;
+        a.sums[i] = z;
         return;
     }
     QueryCell qc;
@@ -218,27 +215,14 @@ __device__ __forceinline__ void select_row(const QueryArgs& a, const uint64_t i)
     out.cnt = 0;
     if (!select_kth<KS>(a, g, qc, q, K, R, kk, tie)) {
         defer_row(a, id, tie, kk, R);
-        if (!FINISH) a.sums[i] = out;
+        a.sums[i] = out;
         return;
     }
     Pass2Fn f2{q.x, q.y, q.z, kk, 0, 0, 0, 0, 0, 0, 0, 0, 0, 0};
     for (int r = 0; r <= R; ++r) scan_shell(a.gv, g, qc, r, f2);
     if (f2.cnt != K) {
         defer_row(a, id, false, kk, R);
-        if (!FINISH) a.sums[i] = out;
-        return;
-    }
-    if (FINISH) {
-        const long long n = f2.cnt;
-        long long M[6];
-        M[0] = n * f2.sxx - (long long)f2.s1x * f2.s1x;
-        M[1] = n * f2.syx - (long long)f2.s1y * f2.s1x;
-        M[2] = n * f2.syy - (long long)f2.s1y * f2.s1y;
-        M[3] = n * f2.szx - (long long)f2.s1z * f2.s1x;
-        M[4] = n * f2.szy - (long long)f2.s1z * f2.s1y;
-        M[5] = n * f2.szz - (long long)f2.s1z * f2.s1z;
-        const int32_t qraw[3] = {qc.qx + g.minx, qc.qy + g.miny, qc.qz + g.minz};
-        nbg_finish_row(a.grp, a.tf, a.ex, id, (int)n, M, qraw);
+        a.sums[i] = out;
         return;
     }
     out.s[0] = f2.s1x;
@@ -656,84 +640,23 @@ __global__ void __launch_bounds__(128) knn_retry_kernel(const QueryArgs a) {
     }
 }
 
-// Rows the single-pass select handed back, answered by the per-thread ring
-// search and finished in place (their sums slots hold cnt = 0, so the finish
-// pass over the other rows, which may run at the same time, skips them).  A
-// few of these rows search far and set the launch's length, so it runs beside
-// that finish pass rather than before it.
-template <int KS>
-__global__ void __launch_bounds__(128) knn_retry_finish_kernel(const QueryArgs a) {
-    const uint32_t nr = *a.nq_dev;
-    for (uint32_t r = blockIdx.x * blockDim.x + threadIdx.x; r < nr; r += gridDim.x * blockDim.x)
-        select_row<KS, true>(a, __ldg(&a.rows[r]));
-}
-
-// ---------------------------------------------------------------------------
-// Tie-order resolver.
-//
-// In a tie row the points strictly inside the K-th distance D_K are the
-// reference's, and the remaining m = K - less slots go to points at integer
-// distance D_K.  Among those the reference keeps the smallest FP64 distances
-// and, at equal FP64 distance, the ones its depth-first search meets first
-// (nanoflann.hpp:178-205, :1191-1197): while fewer than m of them have been
-// admitted the result set holds fewer than K points within D_K, so its worst
-// distance exceeds D_K and no subtree holding one of them is pruned.  The
-// search meets points of one leaf in the tree's point order and, for points in
-// different leaves, first the side of their lowest common node that the query
-// visits first (nanoflann.hpp:1226-1236: child1 iff (q-divlow)+(q-divhigh) < 0).
-// Ordering that group therefore needs the replica's tree but not its search.
-static constexpr int TIE_CAP = 32;
-
-// True when the reference's search meets replica position pa before pb.
-__device__ __forceinline__ bool kd_meets_first(const KdOrder& kd, const double q[3], uint32_t pa,
-                                               uint32_t pb) {
-    int node = kd.root;
-    for (int depth = 0; depth < 64; ++depth) {
-        const int a = __ldg(&kd.c1[node]);
-        if (a < 0) break;
-        const uint32_t split = __ldg(&kd.ne[a]);
-        const bool la = pa < split, lb = pb < split;
-        if (la == lb) {
-            node = la ? a : __ldg(&kd.c2[node]);
-            continue;
-        }
-        const double val = q[__ldg(&kd.feat[node])];
-        const bool left_first =
-            __dadd_rn(__dsub_rn(val, __ldg(&kd.dlo[node])), __dsub_rn(val, __ldg(&kd.dhi[node]))) < 0;
-        return la == left_first;
-    }
-    return pa < pb;
-}
-
 struct TieFn {
     float qx, qy, qz;
     uint32_t kk;
-    int s1x, s1y, s1z, sxx, syx, syy, szx, szy, szz, less;
+    int less;
     int gcnt;
     uint32_t gid[TIE_CAP];
     int gd[TIE_CAP][3];
-    uint32_t* row;  // neighbour-set export: ids of the strictly closer points
+    uint32_t* row;  // ids of the strictly closer points
     int K;
     __device__ __forceinline__ unsigned long long limit() const {
         return (unsigned long long)(kk - KEY_BASE);
-    }
-    __device__ __forceinline__ void add(int ix, int iy, int iz) {
-        s1x += ix;
-        s1y += iy;
-        s1z += iz;
-        sxx += ix * ix;
-        syx += iy * ix;
-        syy += iy * iy;
-        szx += iz * ix;
-        szy += iz * iy;
-        szz += iz * iz;
     }
     __device__ __forceinline__ void operator()(const float4 p) {
         const float dx = p.x - qx, dy = p.y - qy, dz = p.z - qz;
         const uint32_t key = dist_key(dx, dy, dz);
         if (key < kk) {
-            add(small_int(dx), small_int(dy), small_int(dz));
-            if (row && less < K) row[less] = __float_as_uint(p.w);
+            if (less < K) row[less] = __float_as_uint(p.w);
             ++less;
         } else if (key == kk) {
             if (gcnt < TIE_CAP) {
@@ -747,28 +670,9 @@ struct TieFn {
     }
 };
 
-struct TieArgs {
-    GridView gv;
-    const GridParams* gp;
-    uint64_t n;
-    const double* row_k;
-    const int32_t* x;  // raw coordinates in caller order
-    const int32_t* y;
-    const int32_t* z;
-    int K;
-    StageGroup grp;
-    Transform tf;
-    ExceptionSink ex;
-    const uint2* ties;
-    uint32_t nties;
-    KdOrder kd;
-    uint32_t* exact_rows;
-    uint32_t* counters;
-    uint32_t* ids_out;
-};
-
-// One tie row r of a.ties.
-__device__ __forceinline__ void tie_row(const TieArgs& a, uint32_t r) {
+// One tie row r of a.ties, one thread: the neighbour-set export, which needs
+// the members' order (rows that only need sums: warp_tie).
+__device__ __forceinline__ void tie_ids_row(const TieArgs& a, uint32_t r) {
     const uint2 e = a.ties[r];
     const uint32_t id = e.x;
     const uint32_t kk = KEY_BASE + (e.y & 0xFFFFFFu);
@@ -788,10 +692,9 @@ __device__ __forceinline__ void tie_row(const TieArgs& a, uint32_t r) {
     f.qy = (float)qc.qy;
     f.qz = (float)qc.qz;
     f.kk = kk;
-    f.s1x = f.s1y = f.s1z = f.sxx = f.syx = f.syy = f.szx = f.szy = f.szz = 0;
     f.less = 0;
     f.gcnt = 0;
-    f.row = a.ids_out ? a.ids_out + (uint64_t)id * a.K : nullptr;
+    f.row = a.ids_out + (uint64_t)id * a.K;
     f.K = K;
     for (int ring = 0; ring <= R; ++ring) scan_shell(a.gv, g, qc, ring, f);
     const int m = K - f.less;
@@ -815,98 +718,36 @@ __device__ __forceinline__ void tie_row(const TieArgs& a, uint32_t r) {
         }
         d64[t] = acc;
     }
-    // Members at equal FP64 distance are taken in the search's visiting order.
-    // Without a neighbour-id export only their offsets reach the sums: when every
-    // member at the m-th smallest FP64 distance has the same offsets (duplicate
-    // points, most of a lidar tile's tie groups), any of them gives the same
-    // sums, and the row needs no walk down the tree.  (The test is per row: a
-    // member skipped as "equivalent" in a pairwise walk would stand in for its
-    // twin in later comparisons with the other members and break the order.)
-    bool any_order = f.row == nullptr;
-    if (any_order) {
-        double v = 0.0;  // the m-th smallest FP64 distance
-        for (int t = 0; t < f.gcnt; ++t) {
-            int less = 0, le = 0;
-            for (int u = 0; u < f.gcnt; ++u) {
-                less += d64[u] < d64[t];
-                le += d64[u] <= d64[t];
-            }
-            if (less < m && m <= le) v = d64[t];
-        }
-        int ref = -1;
-        for (int t = 0; t < f.gcnt && any_order; ++t) {
-            if (d64[t] != v) continue;
-            if (ref < 0) ref = t;
-            else if (f.gd[t][0] != f.gd[ref][0] || f.gd[t][1] != f.gd[ref][1] ||
-                     f.gd[t][2] != f.gd[ref][2])
-                any_order = false;
-        }
-    }
+    // members at equal FP64 distance are taken in the search's visiting order
     uint32_t taken = 0;
     for (int j = 0; j < m; ++j) {
         int best = -1;
         for (int t = 0; t < f.gcnt; ++t) {
             if ((taken >> t) & 1u) continue;
             if (best < 0 || d64[t] < d64[best] ||
-                (d64[t] == d64[best] && !any_order &&
+                (d64[t] == d64[best] &&
                  kd_meets_first(a.kd, q64, __ldg(&a.kd.kpos[a.kd.base + f.gid[t]]),
                                 __ldg(&a.kd.kpos[a.kd.base + f.gid[best]]))))
                 best = t;
         }
         taken |= 1u << best;
-        f.add(f.gd[best][0], f.gd[best][1], f.gd[best][2]);
-        if (f.row) f.row[f.less + j] = f.gid[best];
+        f.row[f.less + j] = f.gid[best];
     }
-    if (f.row) {
-        uint32_t* row = f.row;
-        for (int s = 1; s < K; ++s) {
-            const uint32_t v = row[s];
-            int t = s - 1;
-            while (t >= 0 && row[t] > v) {
-                row[t + 1] = row[t];
-                --t;
-            }
-            row[t + 1] = v;
+    uint32_t* row = f.row;
+    for (int s = 1; s < K; ++s) {
+        const uint32_t v = row[s];
+        int t = s - 1;
+        while (t >= 0 && row[t] > v) {
+            row[t + 1] = row[t];
+            --t;
         }
-        return;
+        row[t + 1] = v;
     }
-    const long long n = K;
-    long long M[6];
-    M[0] = n * f.sxx - (long long)f.s1x * f.s1x;
-    M[1] = n * f.syx - (long long)f.s1y * f.s1x;
-    M[2] = n * f.syy - (long long)f.s1y * f.s1y;
-    M[3] = n * f.szx - (long long)f.s1z * f.s1x;
-    M[4] = n * f.szy - (long long)f.s1z * f.s1y;
-    M[5] = n * f.szz - (long long)f.s1z * f.s1z;
-    nbg_finish_row(a.grp, a.tf, a.ex, id, (int)n, M, qraw);
 }
 
-__global__ void __launch_bounds__(128) knn_tie_kernel(const TieArgs a) {
+__global__ void __launch_bounds__(128) knn_tie_ids_kernel(const TieArgs a) {
     const uint32_t r = blockIdx.x * blockDim.x + threadIdx.x;
-    if (r < a.nties) tie_row(a, r);
-}
-
-// Tie rows counted on the device (a.nties: the list's capacity).
-__global__ void __launch_bounds__(128) knn_tie_counted_kernel(const TieArgs a, const uint32_t* count) {
-    const uint32_t nt = min(*count, a.nties);
-    for (uint32_t r = blockIdx.x * blockDim.x + threadIdx.x; r < nt; r += gridDim.x * blockDim.x)
-        tie_row(a, r);
-}
-
-// The tie rows of many tiles in one launch: jobs[j] is tile j's arguments,
-// its rows are entries first[j] .. first[j+1]-1 of the launch.
-__global__ void __launch_bounds__(128) knn_tie_batch_kernel(const TieArgs* __restrict__ jobs,
-                                                            const uint64_t* __restrict__ first,
-                                                            int njobs) {
-    const uint64_t t = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x;
-    if (t >= first[njobs]) return;
-    int lo = 0, hi = njobs;  // the job whose range holds t
-    while (hi - lo > 1) {
-        const int mid = (lo + hi) >> 1;
-        if (first[mid] <= t) lo = mid;
-        else hi = mid;
-    }
-    tie_row(jobs[lo], (uint32_t)(t - first[lo]));
+    if (r < a.nties) tie_ids_row(a, r);
 }
 
 static TieArgs tie_args(const TieLaunch& tl) {
@@ -931,56 +772,28 @@ static TieArgs tie_args(const TieLaunch& tl) {
     return a;
 }
 
-int launch_ties(Context* ctx, const TieLaunch& tl, cudaStream_t stream) {
-    (void)ctx;
-    if (!tl.nties) return NBG_OK;
-    knn_tie_kernel<<<(tl.nties + 127) / 128, 128, 0, stream>>>(tie_args(tl));
-    NBG_LAUNCHED(1);
-    return cudaGetLastError() == cudaSuccess ? NBG_OK : NBG_ERR_CUDA;
-}
+// nbg_rows.cu
+int launch_tie_rows(const TieArgs& a, const uint32_t* count, int sms, cudaStream_t stream);
+int launch_tie_batch(Context* ctx, const std::vector<TieArgs>& jobs, cudaStream_t stream);
+int launch_retry_finish(const QueryArgs& q, int slots, int sms, cudaStream_t stream);
 
-// The grid covers a few per cent of a tile at one row per thread (tie rows
-// are 3 % of the 32M-point stress tile); a longer list is walked in strides.
-static constexpr uint64_t kTieBlocksPerSm = 16;
+int launch_ties(Context* ctx, const TieLaunch& tl, cudaStream_t stream) {
+    return launch_ties_counted(ctx, tl, nullptr, stream);
+}
 
 int launch_ties_counted(Context* ctx, const TieLaunch& tl, const uint32_t* count, cudaStream_t stream) {
     if (!tl.nties) return NBG_OK;
-    const uint64_t sms = ctx ? (uint64_t)ctx->sm_count : 148;
-    const unsigned blocks = (unsigned)std::min<uint64_t>(((uint64_t)tl.nties + 127) / 128, sms * kTieBlocksPerSm);
-    knn_tie_counted_kernel<<<blocks, 128, 0, stream>>>(tie_args(tl), count);
+    if (!tl.ids_out) return launch_tie_rows(tie_args(tl), count, ctx ? ctx->sm_count : 148, stream);
+    knn_tie_ids_kernel<<<(tl.nties + 127) / 128, 128, 0, stream>>>(tie_args(tl));
     NBG_LAUNCHED(1);
     return cudaGetLastError() == cudaSuccess ? NBG_OK : NBG_ERR_CUDA;
 }
 
 int launch_ties_many(Context* ctx, const TieLaunch* tls, int count, cudaStream_t stream) {
     std::vector<TieArgs> jobs;
-    std::vector<uint64_t> first(1, 0);
-    for (int i = 0; i < count; ++i) {
-        if (!tls[i].nties) continue;
-        jobs.push_back(tie_args(tls[i]));
-        first.push_back(first.back() + tls[i].nties);
-    }
-    if (jobs.empty()) return NBG_OK;
-    TieArgs* djobs = nullptr;
-    uint64_t* dfirst = nullptr;
-    const size_t jb = jobs.size() * sizeof(TieArgs), fb = first.size() * sizeof(uint64_t);
-    int rc = ctx_alloc(ctx, (void**)&djobs, jb);
-    if (!rc) rc = ctx_alloc(ctx, (void**)&dfirst, fb);
-    // pageable sources: both copies complete before they return
-    if (!rc) rc = host_to_device(ctx, djobs, jobs.data(), jb, stream);
-    if (!rc) rc = host_to_device(ctx, dfirst, first.data(), fb, stream);
-    if (!rc) {
-        const uint64_t total = first.back();
-        knn_tie_batch_kernel<<<(unsigned)((total + 127) / 128), 128, 0, stream>>>(djobs, dfirst,
-                                                                               (int)jobs.size());
-        NBG_LAUNCHED(1);
-        if (cudaGetLastError() != cudaSuccess) rc = NBG_ERR_CUDA;
-    }
-    // the job table is read by the kernel: return it to the cache only after
-    if (cudaStreamSynchronize(stream) != cudaSuccess && !rc) rc = NBG_ERR_CUDA;
-    if (djobs) ctx_free(ctx, djobs, jb);
-    if (dfirst) ctx_free(ctx, dfirst, fb);
-    return rc;
+    for (int i = 0; i < count; ++i)
+        if (tls[i].nties) jobs.push_back(tie_args(tls[i]));
+    return launch_tie_batch(ctx, jobs, stream);
 }
 
 // ---------------------------------------------------------------------------
@@ -1358,11 +1171,12 @@ struct KnnLauncher {
             QueryArgs r = la.q;
             r.rows = la.q.retry_rows;
             r.nq_dev = la.q.counters + 6;
-            const unsigned rb = (unsigned)std::min<uint64_t>(blocks, (uint64_t)la.sms * kRetryBlocksPerSm);
+            r.nq = rows;
             if (!la.fork) {
-                knn_retry_kernel<KS><<<rb, threads, 0, la.stream>>>(r);
+                const int rc = launch_retry_finish(r, KS, la.sms, la.stream);
+                if (rc) return rc;
                 knn_finish_kernel<<<(unsigned)blocks, threads, 0, la.stream>>>(la.q);
-                NBG_LAUNCHED(3);
+                NBG_LAUNCHED(2);
                 return cudaGetLastError() == cudaSuccess ? NBG_OK : NBG_ERR_CUDA;
             }
             // the handed-back rows on the fork stream, queued first so their
@@ -1371,9 +1185,10 @@ struct KnnLauncher {
             cudaError_t e = cudaEventRecord(la.fev[0], la.stream);
             if (!e) e = cudaStreamWaitEvent(la.fork, la.fev[0], 0);
             if (e) return NBG_ERR_CUDA;
-            knn_retry_finish_kernel<KS><<<rb, threads, 0, la.fork>>>(r);
+            const int rc = launch_retry_finish(r, KS, la.sms, la.fork);
+            if (rc) return rc;
             knn_finish_kernel<<<(unsigned)blocks, threads, 0, la.stream>>>(la.q);
-            NBG_LAUNCHED(3);
+            NBG_LAUNCHED(2);
             if (la.done) {
                 // join on the fork stream: `stream` may go on to the next launch
                 e = cudaEventRecord(la.fev[2], la.stream);
