@@ -234,9 +234,10 @@ struct RadiusLaunch {
 int launch_radius(Context* ctx, const RadiusLaunch& rl, cudaStream_t stream);
 
 // Exact path: nanoflann replica build (lazy) + DFS for the listed rows.
-// beside_query: the build shares the SMs with a running query whose results
-// do not wait for it early; from 16M points its launches then keep to a few
-// blocks per SM (tiles and subtrees walked in strides)
+// beside_query: the build shares the SMs with a query just launched, whose
+// results do not wait for it early; from 16M points its level passes then keep
+// to a few blocks per SM, and its subtrees wait for the query's select pass
+// (ctx->fev[0])
 int kd_ensure(Context* ctx, Tile* t, cudaStream_t stream, bool beside_query = false);
 // One forest holding the replicas of every listed tile that has none.
 int kd_ensure_many(Context* ctx, Tile* const* tiles, int count, cudaStream_t stream,

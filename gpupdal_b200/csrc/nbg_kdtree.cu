@@ -38,44 +38,64 @@
 namespace nbg {
 
 static constexpr int KD_LEAF = 100;
-// Level passes: tiles of KD_TILE elements, KD_THREADS threads of KD_ITEMS
-// elements each (segments on the level passes hold more than 4096 points).
-static constexpr int KD_TILE = 1024;
+// Level passes: tiles of KD_TILE elements, KD_THREADS threads; each warp takes
+// KD_ROWS rows of 32 consecutive elements.  A tile this long keeps the tile
+// list of a 32M-point tree at 8k entries, which one block can scan.
+static constexpr int KD_TILE = 4096;
 static constexpr int KD_THREADS = 256;
-static constexpr int KD_ITEMS = KD_TILE / KD_THREADS;
-// Segments of at most this many points are finished, subtree and all, by
-// one warp (kd_warp_build_kernel) instead of level by level.
-static constexpr uint32_t KD_WARP_MAX = 4096;
-static constexpr int KD_WSTACK = 64;
-static constexpr int KD_WARPS = 4;
+static constexpr int KD_ROWS = KD_TILE / KD_THREADS;
+// Segments of at most this many points are finished, subtree and all, in the
+// shared memory of one block (kd_block_build_kernel).
+static constexpr uint32_t KD_BLOCK_MAX = 4096;
+static constexpr int KD_BTHREADS = 512;
+static constexpr int KD_BWARPS = KD_BTHREADS / 32;
+// a warp's pending subtrees: the smaller child is taken first, so at most
+// log2(KD_BLOCK_MAX) larger ones wait
+static constexpr int KD_BSTACK = 13;
 // A build beside a running query (the plain call's speculative replica) keeps
-// its level passes to 2 blocks of 256 threads per SM and the warp subtree
-// builder to 2 blocks of 128, walking tiles and subtrees in strides, so the
-// query keeps most of every SM while the build still streams its passes.
-// Uncapped, its one-block-per-tile launches take every slot a query block
-// frees.  Below 16M points the capped build outlasts the query, which then
-// waits for it; the cap applies from there up.
-static constexpr int kKdBesideBlocksPerSm = 2;
-static constexpr int kKdBesideWarpBlocksPerSm = 2;
+// its level passes to 4 blocks of 256 threads per SM, walking tiles in strides,
+// and starts its subtrees, whose blocks want most of an SM's shared memory, when
+// the query's select pass is through (beside its FP64 finish pass).  From 16M
+// points up; a smaller build would end after the query, which then waits for it.
+static constexpr int kKdBesideBlocksPerSm = 4;
 static constexpr uint64_t kKdBesideMinPoints = 16000000;
-static constexpr int KD_RETRY = -100;  // kd_build: redo without warp subtrees
+static constexpr int KD_RETRY = -100;  // kd_build: redo with room for every node
 static constexpr int KD_STACK = 96;
 static constexpr int KD_CAP = 66;
 
 struct KdSeg {
     uint32_t begin, end;
     int32_t node;
-    int32_t pad;
+    int32_t pad;   // tree
     double lo[3], hi[3];
 };
 
+// A level segment's cut and what its passes found.
 struct KdSplit {
     int32_t f;
-    uint32_t eq;  // points equal to the cut value (pass 2 has work only when > 0)
+    int32_t dims;  // dimensions (bits) whose extents the children need
+    // points with (uint32_t)(raw - org) below t1 are below the cut, those below
+    // t2 at or below it (org: the segment's least raw value in dimension f)
+    int32_t org;
+    uint32_t t1, t2;
+    uint32_t first;  // first tile
     double cutval;
-    uint32_t L, m;    // pass 1: count below, misplaced pairs
-    uint32_t L2, m2;  // pass 2 on [L, n)
-    int32_t mn[3], mx[3];
+    uint32_t L, eq;  // points below and at the cut
+    uint32_t m, m2;  // misplaced pairs of pass 1 and pass 2
+    // extents of the points below, at and above the cut (dimensions `dims`)
+    int32_t mn[3][3], mx[3][3];
+};
+
+// Device-side state of a build: the host queues levels without reading it.
+struct KdState {
+    uint32_t segs;    // segments of the current level
+    uint32_t tiles;   // their tiles
+    uint32_t nodes;
+    uint32_t errors;  // capacity overflows
+    uint32_t small;   // segments for the subtree builder
+    uint32_t any_eq;  // some segment of the level has points at its cut
+    uint32_t ticket;  // blocks of the running pass that have finished
+    uint32_t pad;
 };
 
 struct KdDev {
@@ -100,8 +120,8 @@ struct KdDev {
 // carry their tree in KdSeg::pad, nodes in ntree[].
 struct KdForest {
     uint64_t n = 0;
-    uint32_t grid_cap = 0;   // blocks of a level-pass launch (0: one per tile)
-    uint32_t wgrid_cap = 0;  // blocks of the warp subtree builder (0: one warp per subtree)
+    uint32_t grid_cap = 0;   // most blocks of a level-pass launch (0: no limit)
+    bool beside = false;     // shares the SMs with a query
     int ntrees = 0;
     std::vector<uint64_t> base, npts;
     std::vector<Transform> tfh;
@@ -127,26 +147,19 @@ struct KdForest {
     double* dhi = nullptr;
     int32_t* bmin = nullptr;  // 3 per node
     int32_t* bmax = nullptr;
-    // segments of the current and next level, pass-2 views
+    // segments of the current and next level
     KdSeg* seg[2] = {nullptr, nullptr};
-    KdSeg* seg2 = nullptr;
-    KdSplit* split = nullptr;
-    KdSplit* split2 = nullptr;     // pass-2 segments' split records
-    uint32_t* seg2_from = nullptr; // pass-2 segment -> its level segment
+    KdSplit* split[2] = {nullptr, nullptr};
     uint32_t seg_cap = 0;
-    KdSeg* small = nullptr;      // segments left for the warp builder
-    uint32_t* leaves = nullptr;  // leaves made by the level passes (bbox pending)
-    uint32_t leaf_cap = 0;
+    KdSeg* small = nullptr;      // segments left for the subtree builder
+    uint32_t small_cap = 0;
     // tiles
-    uint32_t* nt = nullptr;        // per segment tile count, then prefix (seg_cap+1)
     uint32_t* tile_seg = nullptr;
-    unsigned long long* tile_cnt = nullptr;  // per tile counts (lt | eq << 32), then prefix
+    unsigned long long* tile_cnt = nullptr;  // per tile counts (below | at << 32), then prefix
     uint32_t tile_cap = 0;
-    void* scan_tmp = nullptr;
-    size_t scan_bytes = 0;
-    uint32_t* counters = nullptr;  // [0] next segments, [1] nodes, [2] errors, [3] small
-                                   // segments, [4] leaves, [5] pass-2 segments
-    uint32_t dl_cap = 0;
+    KdState* state = nullptr;
+    uint32_t* counters = nullptr;  // [2] errors of the search replay
+    uint64_t* bases = nullptr;     // device, first position per tree
     uint64_t bytes = 0;
     std::vector<std::pair<void*, size_t>> blocks;  // device blocks owned
 };
@@ -169,85 +182,6 @@ __global__ void kd_init_kernel(const int32_t* x, const int32_t* y, const int32_t
         ry[i] = y[i];
         rz[i] = z[i];
         rid[i] = (uint32_t)i;
-    }
-}
-
-__global__ void kd_seg_tiles_kernel(const KdSeg* segs, uint32_t S, uint32_t* nt) {
-    uint32_t s = blockIdx.x * blockDim.x + threadIdx.x;
-    if (s < S) nt[s] = (segs[s].end - segs[s].begin + KD_TILE - 1) / KD_TILE;
-    if (s == S) nt[s] = 0;
-}
-
-__global__ void kd_fill_tiles_kernel(const uint32_t* tile_first, uint32_t S, uint32_t ntiles,
-                                     uint32_t* tile_seg) {
-    uint32_t t = blockIdx.x * blockDim.x + threadIdx.x;
-    if (t >= ntiles) return;
-    // last segment whose first tile <= t
-    uint32_t lo = 0, hi = S;  // answer in [lo, hi)
-    while (hi - lo > 1) {
-        uint32_t mid = (lo + hi) >> 1;
-        if (tile_first[mid] <= t) lo = mid;
-        else hi = mid;
-    }
-    tile_seg[t] = lo;
-}
-
-__global__ void kd_minmax_init_kernel(KdSplit* sp, uint32_t S) {
-    uint32_t s = blockIdx.x * blockDim.x + threadIdx.x;
-    if (s >= S) return;
-    for (int d = 0; d < 3; ++d) {
-        sp[s].mn[d] = INT32_MAX;
-        sp[s].mx[d] = INT32_MIN;
-    }
-}
-
-// Segment extents: each tile's block reduction folded into its segment's
-// split record with integer atomics (mn/mx start at INT32_MAX/INT32_MIN).
-__global__ void __launch_bounds__(KD_THREADS) kd_minmax_kernel(const KdSeg* segs, const uint32_t* tile_first,
-                                                               const uint32_t* tile_seg,
-                                                               const int32_t* rx, const int32_t* ry,
-                                                               const int32_t* rz, KdSplit* sp,
-                                                               uint32_t ntiles) {
-    __shared__ int32_t red[KD_THREADS / 32][6];
-    // tiles in strides of the grid (capped beside a query: see kd_grid)
-    for (uint32_t t = blockIdx.x; t < ntiles; t += gridDim.x) {
-        const uint32_t s = tile_seg[t];
-        const KdSeg sg = segs[s];
-        const uint32_t i0 = sg.begin + (t - tile_first[s]) * KD_TILE + threadIdx.x;
-        int32_t v[3] = {INT32_MAX, INT32_MAX, INT32_MAX}, w[3] = {INT32_MIN, INT32_MIN, INT32_MIN};
-#pragma unroll
-        for (int k = 0; k < KD_ITEMS; ++k) {
-            const uint32_t i = i0 + k * KD_THREADS;
-            if (i < sg.end) {
-                const int32_t c[3] = {rx[i], ry[i], rz[i]};
-#pragma unroll
-                for (int d = 0; d < 3; ++d) {
-                    v[d] = min(v[d], c[d]);
-                    w[d] = max(w[d], c[d]);
-                }
-            }
-        }
-#pragma unroll
-        for (int d = 0; d < 3; ++d) {
-            v[d] = __reduce_min_sync(0xffffffffu, v[d]);
-            w[d] = __reduce_max_sync(0xffffffffu, w[d]);
-        }
-        const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-        if (lane == 0) {
-            for (int d = 0; d < 3; ++d) {
-                red[warp][d] = v[d];
-                red[warp][3 + d] = w[d];
-            }
-        }
-        __syncthreads();
-        if (threadIdx.x < 6) {
-            int32_t r = red[0][threadIdx.x];
-            for (int k = 1; k < KD_THREADS / 32; ++k)
-                r = threadIdx.x < 3 ? min(r, red[k][threadIdx.x]) : max(r, red[k][threadIdx.x]);
-            if (threadIdx.x < 3) atomicMin(&sp[s].mn[threadIdx.x], r);
-            else atomicMax(&sp[s].mx[threadIdx.x - 3], r);
-        }
-        __syncthreads();
     }
 }
 
@@ -284,165 +218,389 @@ __device__ __forceinline__ void kd_choose_cut(const double lo[3], const double h
     else cutval = split_val;
 }
 
-__global__ void kd_split_kernel(const KdSeg* segs, uint32_t S, KdSplit* sp, const Transform* tfs,
-                                int32_t* bmin, int32_t* bmax) {
-    uint32_t s = blockIdx.x * blockDim.x + threadIdx.x;
-    if (s >= S) return;
-    const KdSeg sg = segs[s];
-    const Transform tf = tfs[sg.pad];
-    KdSplit p = sp[s];
-    // the node's extents are its points' extents
-    for (int d = 0; d < 3; ++d) {
-        bmin[3 * sg.node + d] = p.mn[d];
-        bmax[3 * sg.node + d] = p.mx[d];
-    }
-    int cutfeat;
-    double cutval;
-    kd_choose_cut(sg.lo, sg.hi, p.mn, p.mx, tf, cutfeat, cutval);
-    sp[s].f = cutfeat;
-    sp[s].cutval = cutval;
-}
-
-__device__ __forceinline__ int32_t kd_coord(const int32_t* rx, const int32_t* ry,
-                                            const int32_t* rz, int f, uint32_t i) {
-    return f == 0 ? rx[i] : (f == 1 ? ry[i] : rz[i]);
-}
-
-// pass 1: x < cutval; pass 2: x <= cutval
-template <int PASS>
-__device__ __forceinline__ bool kd_pred(double v, double cut) {
-    return PASS == 1 ? (v < cut) : (v <= cut);
-}
-
-// Per tile: predicate count in the low 32 bits and, on pass 1, the count of
-// points equal to the cut value in the high 32 bits.
-template <int PASS>
-__global__ void __launch_bounds__(KD_THREADS) kd_count_kernel(const KdSeg* segs, const uint32_t* tile_first,
-                                                              const uint32_t* tile_seg,
-                                                              const KdSplit* sp, const int32_t* rx,
-                                                              const int32_t* ry, const int32_t* rz,
-                                                              const Transform* tfs,
-                                                              unsigned long long* tile_cnt,
-                                                              uint32_t ntiles) {
-    __shared__ unsigned long long red[KD_THREADS / 32];
-    // tiles in strides of the grid (capped beside a query: see kd_grid)
-    for (uint32_t t = blockIdx.x; t < ntiles; t += gridDim.x) {
-        const uint32_t s = tile_seg[t];
-        const KdSeg sg = segs[s];
-        const Transform& tf = tfs[sg.pad];
-        const int f = sp[s].f;
-        const double cut = sp[s].cutval;
-        const int32_t* rc = f == 0 ? rx : (f == 1 ? ry : rz);
-        const uint32_t i0 = sg.begin + (t - tile_first[s]) * KD_TILE + threadIdx.x;
-        unsigned long long c = 0;
+// The reference's coordinate is monotone in the raw integer, so a comparison
+// with the cut value is one with an integer: t1 counts from mn to the smallest
+// raw value of [mn, mx + 1] whose coordinate is at or above the cut, t2 to the
+// smallest above it.  (The passes then read 4 bytes and compare, with no FP64
+// arithmetic; as offsets from mn the bounds fit at either end of int32.)
+__device__ __forceinline__ void kd_thresholds(double cut, double sc, double of, int32_t mn, int32_t mx,
+                                              uint32_t& t1, uint32_t& t2) {
+    const uint32_t range = (uint32_t)((long long)mx - mn) + 1u;
+    auto at = [&](uint32_t k) { return ref_coord((int32_t)((long long)mn + k), sc, of); };
+    const double est = (cut - of) / sc - (double)mn;
+    const uint32_t near = est <= 0.0 ? 0u : est >= (double)range ? range : (uint32_t)est;
+    uint32_t bound[2];
 #pragma unroll
-        for (int k = 0; k < KD_ITEMS; ++k) {
-            const uint32_t i = i0 + k * KD_THREADS;
-            if (i < sg.end) {
-                const double v = ref_coord(rc[i], tf.scale[f], tf.offset[f]);
-                c += kd_pred<PASS>(v, cut) ? 1ull : 0ull;
-                if (PASS == 1 && v == cut) c += 1ull << 32;
+    for (int q = 0; q < 2; ++q) {
+        uint32_t lo = q ? bound[0] : 0u, hi = range;  // the answer lies in [lo, hi]
+        uint32_t probe = max(lo, min(near, hi));
+        for (int step = 0; lo < hi; ++step) {
+            // a few steps around the estimate settle it unless many raw values
+            // share a coordinate (an offset far above the scale)
+            if (step > 3) probe = lo + (hi - lo) / 2;
+            probe = min(probe, hi - 1);
+            const double v = at(probe);
+            if (q ? v <= cut : v < cut) {
+                lo = probe + 1;
+                probe = lo;
+            } else {
+                hi = probe;
+                probe = hi > lo ? hi - 1 : lo;
             }
         }
+        bound[q] = lo;
+    }
+    t1 = bound[0];
+    t2 = bound[1];
+}
+
+// Hoare's pass swaps the t-th element from the left that fails the predicate
+// inside [0, L) with the t-th from the right that satisfies it inside [L, n);
+// with `prank` elements satisfying it before element li, a failing element's t
+// is li - prank, a satisfying one's L - 1 - prank.
+__device__ __forceinline__ uint32_t kd_split_index(uint32_t count, uint32_t L, uint32_t L2) {
+    const uint32_t lim1 = L, lim2 = L + L2;
+    return lim1 > count / 2 ? lim1 : lim2 < count / 2 ? lim2 : count / 2;
+}
+
+struct KdNodes {
+    int32_t *c1, *c2, *feat;
+    uint32_t *nb, *ne;
+    int32_t *bmin, *bmax;
+    int32_t* ntree;
+    uint32_t cap;
+};
+
+// Node arrays of one split: parent `node`, children cid and cid + 1.
+__device__ __forceinline__ void kd_write_children(const KdNodes& N, int32_t node, uint32_t cid, int f,
+                                                  uint32_t b, uint32_t mid, uint32_t e, int32_t tree) {
+    N.c1[node] = (int32_t)cid;
+    N.c2[node] = (int32_t)(cid + 1);
+    N.feat[node] = f;
 #pragma unroll
-        for (int o = 16; o > 0; o >>= 1) c += __shfl_xor_sync(0xffffffffu, c, o);
+    for (uint32_t side = 0; side < 2; ++side) {
+        N.nb[cid + side] = side ? mid : b;
+        N.ne[cid + side] = side ? e : mid;
+        N.c1[cid + side] = -1;
+        N.c2[cid + side] = -1;
+        N.feat[cid + side] = 0;
+        N.ntree[cid + side] = tree;
+    }
+}
+
+struct KdLevel {
+    const KdSeg* segs;
+    KdSplit* sp;
+    KdSeg* next;
+    KdSplit* next_sp;
+    KdSeg* small;
+    uint32_t* tile_seg;
+    unsigned long long* tile_cnt;
+    KdState* st;
+    int32_t *rx, *ry, *rz;
+    uint32_t* rid;
+    uint32_t *mlpos, *mrpos;
+    const Transform* tfs;
+    KdNodes N;
+    uint32_t seg_cap, small_cap, tile_cap;
+};
+
+// True in every thread of the block that finishes a pass last; what the other
+// blocks wrote is visible to it.
+__device__ __forceinline__ bool kd_last_block(KdState* st) {
+    __shared__ uint32_t s_last;
+    __threadfence();
+    __syncthreads();
+    if (threadIdx.x == 0) s_last = atomicAdd(&st->ticket, 1u) == gridDim.x - 1 ? 1u : 0u;
+    __syncthreads();
+    if (s_last) __threadfence();
+    return s_last != 0;
+}
+
+// Exclusive prefix of v[0 .. n] (n + 1 entries, v[n] written) by one block of
+// KD_THREADS threads.
+__device__ __forceinline__ void kd_block_prefix(unsigned long long* v, uint32_t n) {
+    typedef cub::BlockScan<unsigned long long, KD_THREADS> Scan;
+    __shared__ typename Scan::TempStorage tmp;
+    __shared__ unsigned long long s_carry;
+    if (threadIdx.x == 0) s_carry = 0;
+    __syncthreads();
+    for (uint32_t base = 0; base < n; base += KD_THREADS * 8) {
+        unsigned long long x[8];
+#pragma unroll
+        for (int k = 0; k < 8; ++k) {
+            const uint32_t i = base + threadIdx.x * 8 + k;
+            x[k] = i < n ? __ldcg(&v[i]) : 0ull;
+        }
+        unsigned long long total;
+        Scan(tmp).ExclusiveSum(x, x, total);
+        const unsigned long long c = s_carry;
+        __syncthreads();
+#pragma unroll
+        for (int k = 0; k < 8; ++k) {
+            const uint32_t i = base + threadIdx.x * 8 + k;
+            if (i < n) v[i] = c + x[k];
+        }
+        if (threadIdx.x == 0) s_carry = c + total;
+        __syncthreads();
+    }
+    if (threadIdx.x == 0) v[n] = s_carry;
+}
+
+// Rows of a tile: warp w's element of row k.
+__device__ __forceinline__ uint32_t kd_row(uint32_t begin, uint32_t tile, int k) {
+    return begin + tile * KD_TILE + ((threadIdx.x >> 5) * KD_ROWS + k) * 32 + (threadIdx.x & 31u);
+}
+
+// Per tile, pass 1: points below the cut in the low 32 bits, at it in the high
+// ones; pass 2: points at the cut at or after position L (segments that have
+// any).  The last block turns the counts into their prefix.
+template <int PASS>
+__global__ void __launch_bounds__(KD_THREADS) kd_count_kernel(const KdLevel lv) {
+    __shared__ unsigned long long red[KD_THREADS / 32];
+    const uint32_t ntiles = lv.st->tiles;
+    if (!ntiles || (PASS == 2 && !lv.st->any_eq)) return;
+    for (uint32_t t = blockIdx.x; t < ntiles; t += gridDim.x) {
+        const uint32_t s = lv.tile_seg[t];
+        const uint32_t b = lv.segs[s].begin, e = lv.segs[s].end;
+        const KdSplit* sp = &lv.sp[s];
+        const int f = sp->f, org = sp->org;
+        const uint32_t t1 = sp->t1, t2 = sp->t2;
+        const uint32_t from = PASS == 1 ? b : b + sp->L;
+        const int32_t* rc = f == 0 ? lv.rx : (f == 1 ? lv.ry : lv.rz);
+        uint32_t nlt = 0, neq = 0;
+        if (PASS == 1 || sp->eq) {
+            int32_t v[KD_ROWS];
+#pragma unroll
+            for (int k = 0; k < KD_ROWS; ++k) {
+                const uint32_t i = kd_row(b, t - sp->first, k);
+                v[k] = i >= from && i < e ? rc[i] - org : -1;
+            }
+#pragma unroll
+            for (int k = 0; k < KD_ROWS; ++k) {
+                const uint32_t x = (uint32_t)v[k];  // (outside the range: above every bound)
+                if (PASS == 1) nlt += x < t1;
+                neq += x >= t1 && x < t2;
+            }
+        }
+        unsigned long long c = (unsigned long long)__reduce_add_sync(0xffffffffu, nlt) |
+                               (unsigned long long)__reduce_add_sync(0xffffffffu, neq) << 32;
         if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = c;
         __syncthreads();
         if (threadIdx.x == 0) {
             unsigned long long r = 0;
             for (int k = 0; k < KD_THREADS / 32; ++k) r += red[k];
-            tile_cnt[t] = r;
+            lv.tile_cnt[t] = r;
         }
         __syncthreads();
     }
-}
-
-// L and the number of misplaced pairs m for each segment (one warp each: the
-// count before L inside L's tile is recounted by the warp).
-template <int PASS>
-__global__ void kd_seg_count_kernel(const KdSeg* segs, uint32_t S, const uint32_t* tile_first,
-                                    const unsigned long long* tile_pref, KdSplit* sp, const int32_t* rx,
-                                    const int32_t* ry, const int32_t* rz, const Transform* tfs) {
-    const uint32_t s = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
-    const int lane = threadIdx.x & 31;
-    if (s >= S) return;
-    const KdSeg sg = segs[s];
-    const Transform& tf = tfs[sg.pad];
-    const uint32_t first = tile_first[s], nt = tile_first[s + 1] - first;
-    const uint32_t len = sg.end - sg.begin;
-    const int f = sp[s].f;
-    const double cut = sp[s].cutval;
-    const int32_t* rc = f == 0 ? rx : (f == 1 ? ry : rz);
-    const unsigned long long tot = tile_pref[first + nt] - tile_pref[first];
-    const uint32_t L = (uint32_t)tot, eq = (uint32_t)(tot >> 32);
-    const uint32_t tl = L / KD_TILE;
-    uint32_t pleft = 0;
-    if (len) {
-        pleft = (uint32_t)(tile_pref[first + tl] - tile_pref[first]);
-        for (uint32_t base = sg.begin + tl * KD_TILE; base < sg.begin + L; base += 32) {
-            const uint32_t i = base + lane;
-            const bool p = i < sg.begin + L &&
-                           kd_pred<PASS>(ref_coord(rc[i], tf.scale[f], tf.offset[f]), cut);
-            pleft += __popc(__ballot_sync(0xffffffffu, p));
-        }
-    }
-    if (lane) return;
-    const uint32_t m = L - pleft;
+    if (!kd_last_block(lv.st)) return;
+    kd_block_prefix(lv.tile_cnt, ntiles);
+    __syncthreads();
+    if (threadIdx.x == 0) lv.st->ticket = 0;
     if (PASS == 1) {
-        sp[s].L = L;
-        sp[s].m = m;
-        sp[s].eq = eq;
-    } else {
-        sp[s].L2 = L;
-        sp[s].m2 = m;
+        // the segments' counts
+        const uint32_t S = lv.st->segs;
+        bool eq = false;
+        for (uint32_t s = threadIdx.x; s < S; s += KD_THREADS) {
+            KdSplit* sp = &lv.sp[s];
+            const uint32_t t0 = sp->first, t1 = s + 1 < S ? lv.sp[s + 1].first : ntiles;
+            const unsigned long long d = lv.tile_cnt[t1] - lv.tile_cnt[t0];
+            sp->L = (uint32_t)d;
+            sp->eq = (uint32_t)(d >> 32);
+            sp->m = 0;
+            sp->m2 = 0;
+            eq = eq || sp->eq;
+        }
+        eq = __syncthreads_or(eq);
+        if (threadIdx.x == 0) lv.st->any_eq = eq;
     }
 }
 
+// The positions of the misplaced elements (mlpos, mrpos: see kd_split_index's
+// note); pass 1 also takes the extents of the points below, at and above the
+// cut, the children's boxes.
 template <int PASS>
-__global__ void __launch_bounds__(KD_THREADS) kd_classify_kernel(const KdSeg* segs, const uint32_t* tile_first,
-                                                                 const uint32_t* tile_seg,
-                                                                 const unsigned long long* tile_pref,
-                                                                 const KdSplit* sp, const int32_t* rx,
-                                                                 const int32_t* ry, const int32_t* rz,
-                                                                 const Transform* tfs, uint32_t* mlpos,
-                                                                 uint32_t* mrpos,
-                                                                 uint32_t ntiles) {
-    typedef cub::BlockScan<uint32_t, KD_THREADS> Scan;
-    __shared__ typename Scan::TempStorage tmp;
-    // tiles in strides of the grid (capped beside a query: see kd_grid)
+__global__ void __launch_bounds__(KD_THREADS) kd_classify_kernel(const KdLevel lv) {
+    __shared__ uint32_t s_cnt[KD_THREADS / 32];
+    __shared__ int32_t s_ext[18];
+    const uint32_t ntiles = lv.st->tiles;
+    if (!ntiles || (PASS == 2 && !lv.st->any_eq)) return;
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const unsigned lt = (1u << lane) - 1u;
     for (uint32_t t = blockIdx.x; t < ntiles; t += gridDim.x) {
-        const uint32_t s = tile_seg[t];
-        const KdSeg sg = segs[s];
-        const Transform& tf = tfs[sg.pad];
-        const int f = sp[s].f;
-        const double cut = sp[s].cutval;
-        const int32_t* rc = f == 0 ? rx : (f == 1 ? ry : rz);
-        const uint32_t L = PASS == 1 ? sp[s].L : sp[s].L2;
-        const uint32_t m = PASS == 1 ? sp[s].m : sp[s].m2;
-        // blocked arrangement: thread j owns elements j*KD_ITEMS .. j*KD_ITEMS+KD_ITEMS-1
-        const uint32_t i0 = sg.begin + (t - tile_first[s]) * KD_TILE + threadIdx.x * KD_ITEMS;
-        uint32_t p[KD_ITEMS], rank[KD_ITEMS];
+        const uint32_t s = lv.tile_seg[t];
+        KdSplit* sp = &lv.sp[s];
+        if (PASS == 2 && !sp->eq) continue;
+        const uint32_t sb = lv.segs[s].begin, e = lv.segs[s].end;
+        const uint32_t L1 = sp->L;
+        const uint32_t b = PASS == 1 ? sb : sb + L1;      // the pass's range
+        const uint32_t L = PASS == 1 ? L1 : sp->eq;       // satisfying elements in it
+        const int f = sp->f, org = sp->org;
+        const uint32_t t1 = sp->t1, t2 = sp->t2;
+        const int dims = sp->dims;
+        const int32_t* rc = f == 0 ? lv.rx : (f == 1 ? lv.ry : lv.rz);
+        unsigned bal[KD_ROWS];
+        uint32_t n = 0;
+        if (PASS == 1) {
+            if (threadIdx.x < 18) s_ext[threadIdx.x] = threadIdx.x < 9 ? INT32_MAX : INT32_MIN;
+            int32_t mn[2][3], mx[2][3];  // below, at or above
 #pragma unroll
-        for (int k = 0; k < KD_ITEMS; ++k) {
-            const uint32_t i = i0 + k;
-            p[k] = i < sg.end && kd_pred<PASS>(ref_coord(rc[i], tf.scale[f], tf.offset[f]), cut);
-        }
-        Scan(tmp).ExclusiveSum(p, rank);
-        const uint32_t before = (uint32_t)(tile_pref[t] - tile_pref[tile_first[s]]);
+            for (int q = 0; q < 2; ++q)
 #pragma unroll
-        for (int k = 0; k < KD_ITEMS; ++k) {
-            const uint32_t i = i0 + k;
-            if (i >= sg.end) break;
-            const uint32_t prank = before + rank[k];  // predicate holders before i in the segment
-            const uint32_t li = i - sg.begin;
-            if (li < L) {
-                if (!p[k]) mlpos[sg.begin + (li - prank)] = i;
-            } else if (p[k]) {
-                const uint32_t rml = prank - (L - m);
-                mrpos[sg.begin + (m - 1 - rml)] = i;
+                for (int d = 0; d < 3; ++d) {
+                    mn[q][d] = INT32_MAX;
+                    mx[q][d] = INT32_MIN;
+                }
+            __syncthreads();
+#pragma unroll
+            for (int k = 0; k < KD_ROWS; ++k) {
+                const uint32_t i = kd_row(sb, t - sp->first, k);
+                const bool in = i < e;
+                const int32_t c[3] = {in && dims & 1 ? lv.rx[i] : 0, in && dims & 2 ? lv.ry[i] : 0,
+                                      in && dims & 4 ? lv.rz[i] : 0};
+                const uint32_t v = (uint32_t)((f == 0 ? c[0] : (f == 1 ? c[1] : c[2])) - org);
+                const bool p = in && v < t1;
+                bal[k] = __ballot_sync(0xffffffffu, p);
+                n += __popc(bal[k]);
+#pragma unroll
+                for (int d = 0; d < 3; ++d) {
+                    mn[0][d] = min(mn[0][d], p ? c[d] : INT32_MAX);
+                    mx[0][d] = max(mx[0][d], p ? c[d] : INT32_MIN);
+                    mn[1][d] = min(mn[1][d], in && v >= t2 ? c[d] : INT32_MAX);
+                    mx[1][d] = max(mx[1][d], in && v >= t2 ? c[d] : INT32_MIN);
+                }
+                if (in && v >= t1 && v < t2)  // at the cut: few
+#pragma unroll
+                    for (int d = 0; d < 3; ++d) {
+                        atomicMin(&s_ext[3 + d], c[d]);
+                        atomicMax(&s_ext[12 + d], c[d]);
+                    }
+            }
+#pragma unroll
+            for (int q = 0; q < 2; ++q)
+#pragma unroll
+                for (int d = 0; d < 3; ++d) {
+                    const int32_t a = __reduce_min_sync(0xffffffffu, mn[q][d]);
+                    const int32_t z = __reduce_max_sync(0xffffffffu, mx[q][d]);
+                    if (lane == 0) {
+                        atomicMin(&s_ext[6 * q + d], a);
+                        atomicMax(&s_ext[9 + 6 * q + d], z);
+                    }
+                }
+        } else {
+#pragma unroll
+            for (int k = 0; k < KD_ROWS; ++k) {
+                const uint32_t i = kd_row(sb, t - sp->first, k);
+                const bool in = i >= b && i < e;
+                bal[k] = __ballot_sync(0xffffffffu, in && (uint32_t)(rc[in ? i : b] - org) < t2);
+                n += __popc(bal[k]);
             }
         }
+        if (lane == 0) s_cnt[warp] = n;
         __syncthreads();
+        const unsigned long long pre = lv.tile_cnt[t] - lv.tile_cnt[sp->first];
+        uint32_t before = PASS == 1 ? (uint32_t)pre : (uint32_t)(pre >> 32);
+        for (int w = 0; w < warp; ++w) before += s_cnt[w];
+#pragma unroll
+        for (int k = 0; k < KD_ROWS; ++k) {
+            const uint32_t i = kd_row(sb, t - sp->first, k);
+            if (i >= b && i < e) {
+                const uint32_t prank = before + __popc(bal[k] & lt), li = i - b;
+                const bool p = bal[k] >> lane & 1u;
+                if (li < L) {
+                    if (!p) lv.mlpos[b + (li - prank)] = i;
+                } else {
+                    if (p) lv.mrpos[b + (L - 1 - prank)] = i;
+                    if (li == L) {
+                        if (PASS == 1) sp->m = L - prank;
+                        else sp->m2 = L - prank;
+                    }
+                }
+            }
+            before += __popc(bal[k]);
+        }
+        if (PASS == 1 && threadIdx.x < 18) {
+            const int q = (threadIdx.x % 9) / 3, d = threadIdx.x % 3;
+            if (threadIdx.x < 9) atomicMin(&sp->mn[q][d], s_ext[threadIdx.x]);
+            else atomicMax(&sp->mx[q][d], s_ext[threadIdx.x]);
+        }
+        __syncthreads();
+    }
+}
+
+// Cut, thresholds and fresh extents of a segment whose points' extents are
+// (mn, mx).
+__device__ __forceinline__ void kd_plan_segment(const KdSeg& sg, const int32_t mn[3], const int32_t mx[3],
+                                                const Transform& tf, KdSplit* sp) {
+    int f;
+    double cut;
+    kd_choose_cut(sg.lo, sg.hi, mn, mx, tf, f, cut);
+    KdSplit p;
+    p.f = f;
+    p.cutval = cut;
+    p.org = mn[f];
+    // a child's cut is chosen among the dimensions whose side of its box comes
+    // within 1e-5 of the longest; their extents decide, and the cut dimension's
+    // become divlow / divhigh: the classify pass reads no others
+    p.dims = 1 << f;
+    for (int side = 0; side < 2; ++side) {
+        double span[3], longest = 0.0;
+        for (int d = 0; d < 3; ++d) {
+            const double l = side && d == f ? cut : sg.lo[d], h = !side && d == f ? cut : sg.hi[d];
+            span[d] = __dsub_rn(h, l);
+            longest = fmax(longest, span[d]);
+        }
+        for (int d = 0; d < 3; ++d)
+            if (span[d] >= longest * (1.0 - 2e-5)) p.dims |= 1 << d;
+    }
+    kd_thresholds(cut, tf.scale[f], tf.offset[f], mn[f], mx[f], p.t1, p.t2);
+    p.first = 0;
+    p.L = p.eq = p.m = p.m2 = 0;
+#pragma unroll
+    for (int q = 0; q < 3; ++q)
+#pragma unroll
+        for (int d = 0; d < 3; ++d) {
+            p.mn[q][d] = INT32_MAX;
+            p.mx[q][d] = INT32_MIN;
+        }
+    *sp = p;
+}
+
+// One block: the tile list of the S segments in segs / sp.
+__device__ __forceinline__ void kd_tile_map(const KdSeg* segs, KdSplit* sp, uint32_t S, uint32_t* tile_seg,
+                                            uint32_t tile_cap, KdState* st) {
+    typedef cub::BlockScan<uint32_t, KD_THREADS> Scan;
+    __shared__ typename Scan::TempStorage tmp;
+    uint32_t carry = 0;
+    for (uint32_t base = 0; base < S; base += KD_THREADS) {
+        const uint32_t s = base + threadIdx.x;
+        const uint32_t nt = s < S ? (segs[s].end - segs[s].begin + KD_TILE - 1) / KD_TILE : 0u;
+        uint32_t first, total;
+        Scan(tmp).ExclusiveSum(nt, first, total);
+        if (s < S) sp[s].first = carry + first;
+        carry += total;
+        __syncthreads();
+    }
+    if (carry > tile_cap) {
+        if (threadIdx.x == 0) {
+            st->errors += 1;
+            st->segs = st->tiles = 0;
+        }
+        return;
+    }
+    for (uint32_t t = threadIdx.x; t < carry; t += KD_THREADS) {
+        uint32_t lo = 0, hi = S;  // last segment whose first tile <= t
+        while (hi - lo > 1) {
+            const uint32_t mid = (lo + hi) >> 1;
+            if (sp[mid].first <= t) lo = mid;
+            else hi = mid;
+        }
+        tile_seg[t] = lo;
+    }
+    if (threadIdx.x == 0) {
+        st->segs = S;
+        st->tiles = carry;
     }
 }
 
@@ -450,343 +608,426 @@ __global__ void __launch_bounds__(KD_THREADS) kd_classify_kernel(const KdSeg* se
 // before any store (each position belongs to exactly one pair of the level, so
 // the loads never read what a store of this launch writes), which keeps the
 // dependent position -> coordinate loads of all the thread's items in flight
-// together instead of one item at a time.
+// together instead of one item at a time.  After pass 2 the last block splits
+// the segments and plans the next level.
 template <int PASS>
-__global__ void __launch_bounds__(KD_THREADS) kd_swap_kernel(const KdSeg* __restrict__ segs,
-                                                             const uint32_t* __restrict__ tile_first,
-                                                             const uint32_t* __restrict__ tile_seg,
-                                                             const KdSplit* __restrict__ sp,
-                                                             const uint32_t* __restrict__ mlpos,
-                                                             const uint32_t* __restrict__ mrpos,
-                                                             int32_t* __restrict__ rx,
-                                                             int32_t* __restrict__ ry,
-                                                             int32_t* __restrict__ rz,
-                                                             uint32_t* __restrict__ rid,
-                                                             uint32_t ntiles) {
-    // tiles in strides of the grid (capped beside a query: see kd_grid)
-    for (uint32_t t = blockIdx.x; t < ntiles; t += gridDim.x) {
-        const uint32_t s = tile_seg[t];
-        const KdSeg sg = segs[s];
-        const uint32_t m = PASS == 1 ? sp[s].m : sp[s].m2;
-        const uint32_t l0 = (t - tile_first[s]) * KD_TILE + threadIdx.x;
-        if (l0 >= m) continue;
-        uint32_t a[KD_ITEMS], b[KD_ITEMS];
-        int32_t ax[KD_ITEMS], ay[KD_ITEMS], az[KD_ITEMS], bx[KD_ITEMS], by[KD_ITEMS], bz[KD_ITEMS];
-        uint32_t ai[KD_ITEMS], bi[KD_ITEMS];
+__global__ void __launch_bounds__(KD_THREADS) kd_swap_kernel(const KdLevel lv) {
+    const uint32_t ntiles = lv.st->tiles;
+    if (!ntiles) return;
+    constexpr int ITEMS = 4;
+    if (PASS == 1 || lv.st->any_eq) {
+        for (uint32_t t = blockIdx.x; t < ntiles; t += gridDim.x) {
+            const uint32_t s = lv.tile_seg[t];
+            const KdSplit* sp = &lv.sp[s];
+            const uint32_t m = PASS == 1 ? sp->m : sp->m2;
+            const uint32_t b = lv.segs[s].begin + (PASS == 1 ? 0u : sp->L);
+            const uint32_t end = min(m, (t - sp->first + 1) * KD_TILE);
+            for (uint32_t l0 = (t - sp->first) * KD_TILE + threadIdx.x; l0 < end; l0 += KD_THREADS * ITEMS) {
+                uint32_t a[ITEMS], z[ITEMS], ai[ITEMS], zi[ITEMS];
+                int32_t ax[ITEMS], ay[ITEMS], az[ITEMS], zx[ITEMS], zy[ITEMS], zz[ITEMS];
 #pragma unroll
-        for (int k = 0; k < KD_ITEMS; ++k) {
-            const uint32_t li = l0 + k * KD_THREADS;
-            if (li < m) {
-                a[k] = mlpos[sg.begin + li];
-                b[k] = mrpos[sg.begin + li];
-            }
-        }
-#pragma unroll
-        for (int k = 0; k < KD_ITEMS; ++k) {
-            if (l0 + k * KD_THREADS < m) {
-                ax[k] = rx[a[k]];
-                ay[k] = ry[a[k]];
-                az[k] = rz[a[k]];
-                ai[k] = rid[a[k]];
-                bx[k] = rx[b[k]];
-                by[k] = ry[b[k]];
-                bz[k] = rz[b[k]];
-                bi[k] = rid[b[k]];
-            }
-        }
-#pragma unroll
-        for (int k = 0; k < KD_ITEMS; ++k) {
-            if (l0 + k * KD_THREADS < m) {
-                rx[a[k]] = bx[k];
-                ry[a[k]] = by[k];
-                rz[a[k]] = bz[k];
-                rid[a[k]] = bi[k];
-                rx[b[k]] = ax[k];
-                ry[b[k]] = ay[k];
-                rz[b[k]] = az[k];
-                rid[b[k]] = ai[k];
-            }
-        }
-    }
-}
-
-// Pass 2 runs only on segments with points equal to the cut value: every
-// other segment has L2 = m2 = 0.  Listed segments start at their L and keep
-// their own split record (copied), written back after the pass.
-__global__ void kd_pass2_plan_kernel(const KdSeg* segs, uint32_t S, KdSplit* sp, KdSeg* seg2,
-                                     KdSplit* split2, uint32_t* seg2_from, uint32_t* count) {
-    const uint32_t s = blockIdx.x * blockDim.x + threadIdx.x;
-    if (s >= S) return;
-    const KdSplit p = sp[s];
-    sp[s].L2 = 0;
-    sp[s].m2 = 0;
-    if (p.eq == 0) return;
-    const uint32_t k = atomicAdd(count, 1u);
-    KdSeg g = segs[s];
-    g.begin = g.begin + p.L;
-    seg2[k] = g;
-    split2[k] = p;
-    seg2_from[k] = s;
-}
-
-__global__ void kd_pass2_done_kernel(uint32_t S2, const KdSplit* split2, const uint32_t* seg2_from,
-                                     KdSplit* sp) {
-    const uint32_t k = blockIdx.x * blockDim.x + threadIdx.x;
-    if (k >= S2) return;
-    sp[seg2_from[k]].L2 = split2[k].L2;
-    sp[seg2_from[k]].m2 = split2[k].m2;
-}
-
-__global__ void kd_children_kernel(const KdSeg* segs, uint32_t S, const KdSplit* sp, KdSeg* next,
-                                   uint32_t* counters, int32_t* c1, int32_t* c2, int32_t* feat,
-                                   uint32_t* nb, uint32_t* ne, uint32_t node_cap, uint32_t seg_cap,
-                                   KdSeg* small, uint32_t small_max, uint32_t* leaves,
-                                   uint32_t leaf_cap, int32_t* ntree) {
-    uint32_t s = blockIdx.x * blockDim.x + threadIdx.x;
-    if (s >= S) return;
-    const KdSeg sg = segs[s];
-    const KdSplit p = sp[s];
-    const uint32_t count = sg.end - sg.begin;
-    const uint32_t lim1 = p.L, lim2 = p.L + p.L2;
-    uint32_t index;
-    if (lim1 > count / 2) index = lim1;
-    else if (lim2 < count / 2) index = lim2;
-    else index = count / 2;
-    const uint32_t cid = atomicAdd(&counters[1], 2u);
-    if (cid + 2 > node_cap) {
-        atomicAdd(&counters[2], 1u);
-        return;
-    }
-    c1[sg.node] = (int32_t)cid;
-    c2[sg.node] = (int32_t)(cid + 1);
-    feat[sg.node] = p.f;
-    for (int side = 0; side < 2; ++side) {
-        const uint32_t node = cid + side;
-        KdSeg ch = sg;
-        if (side == 0) {
-            ch.end = sg.begin + index;
-            ch.hi[p.f] = p.cutval;
-        } else {
-            ch.begin = sg.begin + index;
-            ch.lo[p.f] = p.cutval;
-        }
-        ch.node = (int32_t)node;
-        nb[node] = ch.begin;
-        ne[node] = ch.end;
-        c1[node] = -1;
-        c2[node] = -1;
-        feat[node] = 0;
-        ntree[node] = sg.pad;
-        const uint32_t len = ch.end - ch.begin;
-        if (len <= (uint32_t)KD_LEAF) {
-            const uint32_t slot = atomicAdd(&counters[4], 1u);
-            if (slot < leaf_cap) leaves[slot] = node;
-            else atomicAdd(&counters[2], 1u);
-        } else if (len <= small_max) {
-            const uint32_t slot = atomicAdd(&counters[3], 1u);
-            if (slot < seg_cap) small[slot] = ch;
-            else atomicAdd(&counters[2], 1u);
-        } else {
-            const uint32_t slot = atomicAdd(&counters[0], 1u);
-            if (slot < seg_cap) next[slot] = ch;
-            else atomicAdd(&counters[2], 1u);
-        }
-    }
-}
-
-// Extents of [b, e) by one warp (INT32_MAX / INT32_MIN when empty).
-__device__ __forceinline__ void kd_warp_minmax(const int32_t* rx, const int32_t* ry, const int32_t* rz,
-                                               uint32_t b, uint32_t e, int lane, int32_t mn[3],
-                                               int32_t mx[3]) {
-    int32_t v[3] = {INT32_MAX, INT32_MAX, INT32_MAX}, w[3] = {INT32_MIN, INT32_MIN, INT32_MIN};
-    for (uint32_t i = b + lane; i < e; i += 32) {
-        const int32_t c[3] = {rx[i], ry[i], rz[i]};
-#pragma unroll
-        for (int d = 0; d < 3; ++d) {
-            v[d] = min(v[d], c[d]);
-            w[d] = max(w[d], c[d]);
-        }
-    }
-#pragma unroll
-    for (int d = 0; d < 3; ++d) {
-        mn[d] = __reduce_min_sync(0xffffffffu, v[d]);
-        mx[d] = __reduce_max_sync(0xffffffffu, w[d]);
-    }
-}
-
-// Leaves made by the level passes: their extents, one warp per leaf.
-__global__ void kd_leaf_bbox_kernel(const uint32_t* leaves, uint32_t nleaves, const uint32_t* nb,
-                                    const uint32_t* ne, const int32_t* rx, const int32_t* ry,
-                                    const int32_t* rz, int32_t* bmin, int32_t* bmax) {
-    const uint32_t w = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
-    const int lane = threadIdx.x & 31;
-    if (w >= nleaves) return;
-    const uint32_t node = leaves[w];
-    int32_t mn[3], mx[3];
-    kd_warp_minmax(rx, ry, rz, nb[node], ne[node], lane, mn, mx);
-    if (lane < 3) {
-        bmin[3 * node + lane] = mn[lane];
-        bmax[3 * node + lane] = mx[lane];
-    }
-}
-
-// One Hoare pass of nanoflann's planeSplit over [b, e) by one warp: with L
-// the count satisfying the predicate, the t-th element from the left failing
-// it inside [b, b+L) swaps with the t-th element from the right satisfying it
-// inside [b+L, e).  Returns L; *eq (pass 1) counts the elements equal to the
-// cut value, the only ones pass 2 can move.  mlpos/mrpos[b ...] are the
-// warp's scratch.
-template <int PASS>
-__device__ uint32_t kd_warp_pass(int32_t* rx, int32_t* ry, int32_t* rz, uint32_t* rid,
-                                 uint32_t* mlpos, uint32_t* mrpos, uint32_t b, uint32_t e, int f,
-                                 double cut, const Transform& tf, int lane, uint32_t* eq = nullptr) {
-    const int32_t* rc = f == 0 ? rx : (f == 1 ? ry : rz);
-    const double sc = tf.scale[f], of = tf.offset[f];
-    const unsigned lt = (1u << lane) - 1u;
-    uint32_t L = 0, neq = 0;
-    for (uint32_t base = b; base < e; base += 32) {
-        const uint32_t i = base + lane;
-        const double v = i < e ? ref_coord(rc[i], sc, of) : 0.0;
-        const bool p = i < e && kd_pred<PASS>(v, cut);
-        L += __popc(__ballot_sync(0xffffffffu, p));
-        if (PASS == 1) neq += __popc(__ballot_sync(0xffffffffu, i < e && v == cut));
-    }
-    if (eq) *eq = neq;
-    uint32_t m = 0;
-    for (uint32_t base = b; base < b + L; base += 32) {
-        const uint32_t i = base + lane;
-        const bool q = i < b + L && !kd_pred<PASS>(ref_coord(rc[i], sc, of), cut);
-        const unsigned mask = __ballot_sync(0xffffffffu, q);
-        if (q) mlpos[b + m + __popc(mask & lt)] = i;
-        m += __popc(mask);
-    }
-    uint32_t r = 0;
-    for (uint32_t base = b + L; base < e; base += 32) {
-        const uint32_t i = base + lane;
-        const bool q = i < e && kd_pred<PASS>(ref_coord(rc[i], sc, of), cut);
-        const unsigned mask = __ballot_sync(0xffffffffu, q);
-        if (q) {
-            const uint32_t k = r + __popc(mask & lt);
-            if (k < m) mrpos[b + (m - 1 - k)] = i;
-        }
-        r += __popc(mask);
-    }
-    __syncwarp();
-    for (uint32_t t = lane; t < m; t += 32) {
-        const uint32_t a = mlpos[b + t], c = mrpos[b + t];
-        const int32_t tx = rx[a], ty = ry[a], tz = rz[a];
-        const uint32_t ti = rid[a];
-        rx[a] = rx[c];
-        ry[a] = ry[c];
-        rz[a] = rz[c];
-        rid[a] = rid[c];
-        rx[c] = tx;
-        ry[c] = ty;
-        rz[c] = tz;
-        rid[c] = ti;
-    }
-    __syncwarp();
-    return L;
-}
-
-// Builds the whole subtree of each listed segment, one warp per segment,
-// depth first with an explicit stack in shared memory.  Same split rules as
-// the level passes; nodes are numbered by an atomic counter.  counters[2]
-// counts capacity or stack overflows (the host then rebuilds level by level).
-__global__ void __launch_bounds__(32 * KD_WARPS) kd_warp_build_kernel(
-    const KdSeg* small, uint32_t nsmall, int32_t* rx, int32_t* ry, int32_t* rz, uint32_t* rid,
-    uint32_t* mlpos, uint32_t* mrpos, int32_t* c1, int32_t* c2, int32_t* feat, uint32_t* nb,
-    uint32_t* ne, int32_t* bmin, int32_t* bmax, uint32_t* counters, uint32_t node_cap,
-    const Transform* tfs, int32_t* ntree) {
-    __shared__ KdSeg stk[KD_WARPS][KD_WSTACK];
-    const int wl = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    KdSeg* st = stk[wl];
-    // segments in strides of the grid's warps (capped beside a query)
-    for (uint32_t w = blockIdx.x * KD_WARPS + wl; w < nsmall; w += gridDim.x * KD_WARPS) {
-        if (lane == 0) st[0] = small[w];
-        int top = 1;
-        __syncwarp();
-        while (top > 0) {
-            const KdSeg sg = st[top - 1];
-            --top;
-            __syncwarp();
-            const uint32_t b = sg.begin, e = sg.end, count = e - b;
-            const int node = sg.node;
-            int32_t mn[3], mx[3];
-            kd_warp_minmax(rx, ry, rz, b, e, lane, mn, mx);
-            if (lane < 3) {
-                bmin[3 * node + lane] = mn[lane];
-                bmax[3 * node + lane] = mx[lane];
-            }
-            if (count <= (uint32_t)KD_LEAF) continue;
-            const Transform tf = tfs[sg.pad];
-            int f;
-            double cut;
-            kd_choose_cut(sg.lo, sg.hi, mn, mx, tf, f, cut);
-            uint32_t eq = 0;
-            const uint32_t L = kd_warp_pass<1>(rx, ry, rz, rid, mlpos, mrpos, b, e, f, cut, tf, lane, &eq);
-            // pass 2 (<= cut on [b+L, e), which pass 1 left holding the elements
-            // >= cut) moves only elements equal to the cut value: with none, its
-            // count is 0 and it swaps nothing
-            const uint32_t L2 =
-                eq ? kd_warp_pass<2>(rx, ry, rz, rid, mlpos, mrpos, b + L, e, f, cut, tf, lane) : 0u;
-            const uint32_t lim1 = L, lim2 = L + L2;
-            uint32_t index;
-            if (lim1 > count / 2) index = lim1;
-            else if (lim2 < count / 2) index = lim2;
-            else index = count / 2;
-            uint32_t cid = 0;
-            if (lane == 0) cid = atomicAdd(&counters[1], 2u);
-            cid = __shfl_sync(0xffffffffu, cid, 0);
-            if (cid + 2 > node_cap || top + 2 > KD_WSTACK) {
-                if (lane == 0) atomicAdd(&counters[2], 1u);
-                return;
-            }
-            if (lane == 0) {
-                c1[node] = (int32_t)cid;
-                c2[node] = (int32_t)(cid + 1);
-                feat[node] = f;
-                for (int side = 1; side >= 0; --side) {
-                    KdSeg ch = sg;
-                    if (side == 0) {
-                        ch.end = b + index;
-                        ch.hi[f] = cut;
-                    } else {
-                        ch.begin = b + index;
-                        ch.lo[f] = cut;
+                for (int k = 0; k < ITEMS; ++k)
+                    if (l0 + k * KD_THREADS < end) {
+                        a[k] = lv.mlpos[b + l0 + k * KD_THREADS];
+                        z[k] = lv.mrpos[b + l0 + k * KD_THREADS];
                     }
-                    ch.node = (int32_t)(cid + side);
-                    nb[cid + side] = ch.begin;
-                    ne[cid + side] = ch.end;
-                    c1[cid + side] = -1;
-                    c2[cid + side] = -1;
-                    feat[cid + side] = 0;
-                    ntree[cid + side] = sg.pad;
-                    st[top + (1 - side)] = ch;
+#pragma unroll
+                for (int k = 0; k < ITEMS; ++k)
+                    if (l0 + k * KD_THREADS < end) {
+                        ax[k] = lv.rx[a[k]];
+                        ay[k] = lv.ry[a[k]];
+                        az[k] = lv.rz[a[k]];
+                        ai[k] = lv.rid[a[k]];
+                        zx[k] = lv.rx[z[k]];
+                        zy[k] = lv.ry[z[k]];
+                        zz[k] = lv.rz[z[k]];
+                        zi[k] = lv.rid[z[k]];
+                    }
+#pragma unroll
+                for (int k = 0; k < ITEMS; ++k)
+                    if (l0 + k * KD_THREADS < end) {
+                        lv.rx[a[k]] = zx[k];
+                        lv.ry[a[k]] = zy[k];
+                        lv.rz[a[k]] = zz[k];
+                        lv.rid[a[k]] = zi[k];
+                        lv.rx[z[k]] = ax[k];
+                        lv.ry[z[k]] = ay[k];
+                        lv.rz[z[k]] = az[k];
+                        lv.rid[z[k]] = ai[k];
+                    }
+            }
+        }
+    }
+    if (PASS == 1 || !kd_last_block(lv.st)) return;
+    // ---- split the segments, plan the next level
+    __shared__ uint32_t s_next;
+    if (threadIdx.x == 0) s_next = 0;
+    __syncthreads();
+    const uint32_t S = lv.st->segs;
+    for (uint32_t s = threadIdx.x; s < S; s += KD_THREADS) {
+        const KdSeg sg = lv.segs[s];
+        const KdSplit p = lv.sp[s];
+        const uint32_t count = sg.end - sg.begin;
+        const uint32_t index = kd_split_index(count, p.L, p.eq);
+        const uint32_t cid = atomicAdd(&lv.st->nodes, 2u);
+        if (cid + 2 > lv.N.cap) {
+            atomicAdd(&lv.st->errors, 1u);
+            continue;
+        }
+        kd_write_children(lv.N, sg.node, cid, p.f, sg.begin, sg.begin + index, sg.end, sg.pad);
+        // the children's extents: the points at the cut go to one side, or (the
+        // split falls among them) their range is read
+        int32_t mn[2][3], mx[2][3];
+        for (int d = 0; d < 3; ++d) {
+            mn[0][d] = p.mn[0][d];
+            mx[0][d] = p.mx[0][d];
+            mn[1][d] = p.mn[2][d];
+            mx[1][d] = p.mx[2][d];
+        }
+        if (index == p.L || index == p.L + p.eq) {
+            const int side = index == p.L ? 1 : 0;
+            for (int d = 0; d < 3; ++d) {
+                mn[side][d] = min(mn[side][d], p.mn[1][d]);
+                mx[side][d] = max(mx[side][d], p.mx[1][d]);
+            }
+        } else {
+            for (uint32_t i = sg.begin + p.L; i < sg.begin + p.L + p.eq; ++i) {
+                const int side = i < sg.begin + index ? 0 : 1;
+                const int32_t c[3] = {__ldcg(&lv.rx[i]), __ldcg(&lv.ry[i]), __ldcg(&lv.rz[i])};
+                for (int d = 0; d < 3; ++d) {
+                    mn[side][d] = min(mn[side][d], c[d]);
+                    mx[side][d] = max(mx[side][d], c[d]);
                 }
             }
-            top += 2;
-            __syncwarp();
+        }
+        for (int side = 0; side < 2; ++side) {
+            const uint32_t node = cid + side;
+            for (int d = 0; d < 3; ++d) {
+                lv.N.bmin[3 * node + d] = mn[side][d];
+                lv.N.bmax[3 * node + d] = mx[side][d];
+            }
+            KdSeg ch = sg;
+            if (side == 0) {
+                ch.end = sg.begin + index;
+                ch.hi[p.f] = p.cutval;
+            } else {
+                ch.begin = sg.begin + index;
+                ch.lo[p.f] = p.cutval;
+            }
+            ch.node = (int32_t)node;
+            if (ch.end - ch.begin <= KD_BLOCK_MAX) {
+                const uint32_t slot = atomicAdd(&lv.st->small, 1u);
+                if (slot < lv.small_cap) lv.small[slot] = ch;
+                else atomicAdd(&lv.st->errors, 1u);
+            } else {
+                const uint32_t slot = atomicAdd(&s_next, 1u);
+                if (slot < lv.seg_cap) {
+                    lv.next[slot] = ch;
+                    kd_plan_segment(ch, mn[side], mx[side], lv.tfs[sg.pad], &lv.next_sp[slot]);
+                } else {
+                    atomicAdd(&lv.st->errors, 1u);
+                }
+            }
+        }
+    }
+    __syncthreads();
+    if (threadIdx.x == 0) lv.st->ticket = 0;
+    kd_tile_map(lv.next, lv.next_sp, min(s_next, lv.seg_cap), lv.tile_seg, lv.tile_cap, lv.st);
+}
+
+// The roots: extents, cuts and tile list of the first level (one block).
+__global__ void __launch_bounds__(KD_THREADS) kd_roots_kernel(const KdLevel lv, uint32_t S) {
+    for (uint32_t s = threadIdx.x; s < S; s += KD_THREADS) {
+        const KdSeg sg = lv.segs[s];
+        kd_plan_segment(sg, &lv.N.bmin[3 * sg.node], &lv.N.bmax[3 * sg.node], lv.tfs[sg.pad], &lv.sp[s]);
+    }
+    __syncthreads();
+    kd_tile_map(lv.segs, lv.sp, S, lv.tile_seg, lv.tile_cap, lv.st);
+}
+
+// ---------------------------------------------------------------------------
+// Whole subtrees in shared memory, one block per segment.  The block's warps
+// split with the tree: a group of W warps cuts its segment (extents, cut,
+// ranks by ballot, Hoare's swaps, all in shared memory), then each half of the
+// group takes one child; a single warp goes on depth first, the smaller child
+// at once and the larger one stacked.  A point is read and written once; the
+// inverse permutation goes out with it.
+struct KdFrame16 {
+    double lo[3], hi[3];
+    int32_t node;
+    uint16_t b, e;
+};
+
+struct KdBlockShared {
+    int32_t c[3][KD_BLOCK_MAX];
+    uint32_t id[KD_BLOCK_MAX];
+    uint16_t ml[KD_BLOCK_MAX], mr[KD_BLOCK_MAX];
+    KdFrame16 stk[KD_BWARPS][KD_BSTACK];
+    int32_t ext[KD_BWARPS][6];
+    uint32_t cnt[KD_BWARPS][2];
+    uint32_t m[KD_BWARPS];
+    uint32_t cid[KD_BWARPS];
+};
+
+// Barrier of a group of W warps starting at warp w0 (barrier 0 is the block's).
+__device__ __forceinline__ void kd_group_sync(int W, int w0) {
+    if (W == 1) __syncwarp();
+    else asm volatile("bar.sync %0, %1;" ::"r"(1 + (w0 >> 1)), "r"(W * 32) : "memory");
+}
+
+// One Hoare pass of a group over [b, e) (values less than `tp` above `org`
+// satisfy the predicate; L of them).
+__device__ __forceinline__ void kd_group_pass(KdBlockShared& sh, const int32_t* v, uint32_t b, uint32_t e,
+                                              int32_t org, uint32_t tp, uint32_t L, uint32_t before, uint32_t r0, uint32_t r1,
+                                              int W, int w0) {
+    const int lane = threadIdx.x & 31, t = threadIdx.x - w0 * 32;
+    const unsigned lt = (1u << lane) - 1u;
+    for (uint32_t r = r0; r < r1; r += 32) {
+        const uint32_t i = r + lane;
+        const bool in = i < e, p = in && (uint32_t)(v[in ? i : b] - org) < tp;
+        const unsigned bal = __ballot_sync(0xffffffffu, p);
+        if (in) {
+            const uint32_t prank = before + __popc(bal & lt), li = i - b;
+            if (li < L) {
+                if (!p) sh.ml[b + (li - prank)] = (uint16_t)i;
+            } else {
+                if (p) sh.mr[b + (L - 1 - prank)] = (uint16_t)i;
+                if (li == L) sh.m[w0] = L - prank;
+            }
+        }
+        before += __popc(bal);
+    }
+    kd_group_sync(W, w0);
+    const uint32_t m = L < e - b ? sh.m[w0] : 0u;
+    for (uint32_t k = t; k < m; k += W * 32) {
+        const uint32_t a = sh.ml[b + k], z = sh.mr[b + k];
+#pragma unroll
+        for (int d = 0; d < 3; ++d) {
+            const int32_t x = sh.c[d][a];
+            sh.c[d][a] = sh.c[d][z];
+            sh.c[d][z] = x;
+        }
+        const uint32_t x = sh.id[a];
+        sh.id[a] = sh.id[z];
+        sh.id[z] = x;
+    }
+    kd_group_sync(W, w0);
+}
+
+__global__ void __launch_bounds__(KD_BTHREADS, 2) kd_block_build_kernel(
+    const KdSeg* __restrict__ small, int32_t* rx, int32_t* ry, int32_t* rz, uint32_t* rid,
+    uint32_t* kpos, const uint64_t* __restrict__ tree_base, KdNodes N, KdState* st, const Transform* tfs) {
+    extern __shared__ __align__(16) unsigned char kd_smem[];
+    KdBlockShared& sh = *reinterpret_cast<KdBlockShared*>(kd_smem);
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    {
+        const KdSeg root = small[blockIdx.x];
+        const uint32_t base = root.begin, total = root.end - root.begin;
+        const Transform tf = tfs[root.pad];
+        for (uint32_t i = threadIdx.x; i < total; i += KD_BTHREADS) {
+            sh.c[0][i] = rx[base + i];
+            sh.c[1][i] = ry[base + i];
+            sh.c[2][i] = rz[base + i];
+            sh.id[i] = rid[base + i];
+        }
+        __syncthreads();
+        double lo[3], hi[3];
+#pragma unroll
+        for (int d = 0; d < 3; ++d) {
+            lo[d] = root.lo[d];
+            hi[d] = root.hi[d];
+        }
+        uint32_t b = 0, e = total;
+        int32_t node = root.node;
+        int W = KD_BWARPS, w0 = 0, top = 0;
+        while (true) {
+            const uint32_t count = e - b;
+            const int t = threadIdx.x - w0 * 32;
+            int32_t mn[3] = {INT32_MAX, INT32_MAX, INT32_MAX}, mx[3] = {INT32_MIN, INT32_MIN, INT32_MIN};
+            for (uint32_t i = b + t; i < e; i += W * 32) {
+#pragma unroll
+                for (int d = 0; d < 3; ++d) {
+                    const int32_t x = sh.c[d][i];
+                    mn[d] = min(mn[d], x);
+                    mx[d] = max(mx[d], x);
+                }
+            }
+#pragma unroll
+            for (int d = 0; d < 3; ++d) {
+                mn[d] = __reduce_min_sync(0xffffffffu, mn[d]);
+                mx[d] = __reduce_max_sync(0xffffffffu, mx[d]);
+            }
+            if (W > 1) {
+                if (lane == 0) {
+#pragma unroll
+                    for (int d = 0; d < 3; ++d) {
+                        sh.ext[warp][d] = mn[d];
+                        sh.ext[warp][3 + d] = mx[d];
+                    }
+                }
+                kd_group_sync(W, w0);
+#pragma unroll
+                for (int d = 0; d < 3; ++d) {
+                    mn[d] = __reduce_min_sync(0xffffffffu, sh.ext[w0 + (lane & (W - 1))][d]);
+                    mx[d] = __reduce_max_sync(0xffffffffu, sh.ext[w0 + (lane & (W - 1))][3 + d]);
+                }
+            }
+            if (t < 3) {
+                N.bmin[3 * node + t] = t == 0 ? mn[0] : (t == 1 ? mn[1] : mn[2]);
+                N.bmax[3 * node + t] = t == 0 ? mx[0] : (t == 1 ? mx[1] : mx[2]);
+            }
+            bool split = count > (uint32_t)KD_LEAF;
+            if (split) {
+                int f;
+                double cut;
+                kd_choose_cut(lo, hi, mn, mx, tf, f, cut);
+                uint32_t t1, t2;
+                const int32_t org = f == 0 ? mn[0] : (f == 1 ? mn[1] : mn[2]);
+                kd_thresholds(cut, tf.scale[f], tf.offset[f], org, f == 0 ? mx[0] : (f == 1 ? mx[1] : mx[2]),
+                              t1, t2);
+                const int32_t* v = sh.c[f];
+                // each warp of the group takes a run of rows
+                const uint32_t rows = (count + 31) / 32, per = (rows + W - 1) / W;
+                const uint32_t r0 = min(b + (warp - w0) * per * 32, e), r1 = min(r0 + per * 32, e);
+                uint32_t nlt = 0, neq = 0;
+                for (uint32_t r = r0; r < r1; r += 32) {
+                    const uint32_t i = r + lane;
+                    const uint32_t x = i < e ? (uint32_t)(v[i] - org) : 0xFFFFFFFFu;
+                    nlt += x < t1;
+                    neq += x >= t1 && x < t2;
+                }
+                nlt = __reduce_add_sync(0xffffffffu, nlt);
+                neq = __reduce_add_sync(0xffffffffu, neq);
+                uint32_t L = nlt, eq = neq, before = 0;
+                if (W > 1) {
+                    if (lane == 0) {
+                        sh.cnt[warp][0] = nlt;
+                        sh.cnt[warp][1] = neq;
+                    }
+                    kd_group_sync(W, w0);
+                    const uint32_t x = lane < W ? sh.cnt[w0 + lane][0] : 0u;
+                    L = __reduce_add_sync(0xffffffffu, x);
+                    eq = __reduce_add_sync(0xffffffffu, lane < W ? sh.cnt[w0 + lane][1] : 0u);
+                    before = __reduce_add_sync(0xffffffffu, lane < warp - w0 ? x : 0u);
+                }
+                kd_group_pass(sh, v, b, e, org, t1, L, before, r0, r1, W, w0);
+                if (eq) {
+                    // pass 2 moves only points at the cut
+                    const uint32_t b2 = b + L, rows2 = (count - L + 31) / 32, per2 = (rows2 + W - 1) / W;
+                    const uint32_t q0 = min(b2 + (warp - w0) * per2 * 32, e), q1 = min(q0 + per2 * 32, e);
+                    uint32_t before2 = 0;
+                    if (W > 1) {
+                        uint32_t k = 0;
+                        for (uint32_t r = q0; r < q1; r += 32) {
+                            const uint32_t i = r + lane;
+                            k += i < e && (uint32_t)(v[min(i, e - 1)] - org) < t2;
+                        }
+                        k = __reduce_add_sync(0xffffffffu, k);
+                        if (lane == 0) sh.cnt[warp][0] = k;
+                        kd_group_sync(W, w0);
+                        before2 = __reduce_add_sync(0xffffffffu, lane < warp - w0 ? sh.cnt[w0 + lane][0] : 0u);
+                    }
+                    kd_group_pass(sh, v, b2, e, org, t2, eq, before2, q0, q1, W, w0);
+                }
+                const uint32_t mid = b + kd_split_index(count, L, eq);
+                uint32_t cid = 0;
+                if (t == 0) {
+                    cid = atomicAdd(&st->nodes, 2u);
+                    if (cid + 2 <= N.cap)
+                        kd_write_children(N, node, cid, f, base + b, base + mid, base + e, root.pad);
+                    else atomicAdd(&st->errors, 1u);
+                    sh.cid[w0] = cid;
+                }
+                if (W > 1) {
+                    kd_group_sync(W, w0);
+                    cid = sh.cid[w0];
+                    kd_group_sync(W, w0);  // (read by all before a half's leader writes it again)
+                } else {
+                    cid = __shfl_sync(0xffffffffu, cid, 0);
+                }
+                if (cid + 2 > N.cap) {
+                    split = false;  // (the host builds again with more room)
+                } else if (W > 1) {
+                    // each half of the group takes a child
+                    W >>= 1;
+                    const int side = warp >= w0 + W ? 1 : 0;
+                    w0 += side * W;
+                    node = (int32_t)cid + side;
+                    if (side) b = mid;
+                    else e = mid;
+#pragma unroll
+                    for (int d = 0; d < 3; ++d)
+                        if (d == f) {
+                            if (side) lo[d] = cut;
+                            else hi[d] = cut;
+                        }
+                } else {
+                    // the larger child waits, the smaller one is next
+                    const int big = e - mid > mid - b ? 1 : 0;
+                    if (lane == 0) {
+                        KdFrame16& fr = sh.stk[warp][top];
+#pragma unroll
+                        for (int d = 0; d < 3; ++d) {
+                            fr.lo[d] = d == f && big ? cut : lo[d];
+                            fr.hi[d] = d == f && !big ? cut : hi[d];
+                        }
+                        fr.node = (int32_t)cid + big;
+                        fr.b = (uint16_t)(big ? mid : b);
+                        fr.e = (uint16_t)(big ? e : mid);
+                    }
+                    ++top;
+                    __syncwarp();
+                    node = (int32_t)cid + 1 - big;
+                    if (big) e = mid;
+                    else b = mid;
+#pragma unroll
+                    for (int d = 0; d < 3; ++d)
+                        if (d == f) {
+                            if (big) hi[d] = cut;
+                            else lo[d] = cut;
+                        }
+                }
+            }
+            if (!split) {
+                if (W > 1 || top == 0) break;  // a leaf of the whole group, or the warp's last one
+                --top;
+                __syncwarp();
+                const KdFrame16 fr = sh.stk[warp][top];
+#pragma unroll
+                for (int d = 0; d < 3; ++d) {
+                    lo[d] = fr.lo[d];
+                    hi[d] = fr.hi[d];
+                }
+                node = fr.node;
+                b = fr.b;
+                e = fr.e;
+                __syncwarp();
+            }
+        }
+        __syncthreads();
+        const uint64_t tb = tree_base[root.pad];
+        for (uint32_t i = threadIdx.x; i < total; i += KD_BTHREADS) {
+            rx[base + i] = sh.c[0][i];
+            ry[base + i] = sh.c[1][i];
+            rz[base + i] = sh.c[2][i];
+            const uint32_t id = sh.id[i];
+            rid[base + i] = id;
+            kpos[tb + id] = base + i;
         }
     }
 }
 
-__global__ void kd_div_kernel(uint32_t nodes, const int32_t* c1, const int32_t* c2,
-                              const int32_t* feat, const int32_t* bmin, const int32_t* bmax,
-                              const Transform* tfs, const int32_t* ntree, double* dlo, double* dhi) {
-    uint32_t node = blockIdx.x * blockDim.x + threadIdx.x;
-    if (node >= nodes || c1[node] < 0) return;
-    const int f = feat[node];
-    const Transform& tf = tfs[ntree[node]];
-    dlo[node] = ref_coord(bmax[3 * c1[node] + f], tf.scale[f], tf.offset[f]);
-    dhi[node] = ref_coord(bmin[3 * c2[node] + f], tf.scale[f], tf.offset[f]);
-}
-
-// kpos[base + id] = position of point id of the tree starting at base.
-__global__ void kd_inverse_kernel(const uint32_t* rid, uint64_t base, uint64_t n, uint32_t* kpos) {
-    for (uint64_t i = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x; i < n;
-         i += (uint64_t)gridDim.x * blockDim.x)
-        kpos[base + rid[base + i]] = (uint32_t)(base + i);
+__global__ void kd_div_kernel(const KdState* st, const int32_t* c1, const int32_t* c2, const int32_t* feat,
+                              const int32_t* bmin, const int32_t* bmax, const Transform* tfs,
+                              const int32_t* ntree, double* dlo, double* dhi, uint32_t cap) {
+    const uint32_t nodes = min(st->nodes, cap);
+    for (uint32_t node = blockIdx.x * blockDim.x + threadIdx.x; node < nodes; node += gridDim.x * blockDim.x) {
+        if (c1[node] < 0) continue;
+        const int f = feat[node];
+        const Transform& tf = tfs[ntree[node]];
+        dlo[node] = ref_coord(bmax[3 * c1[node] + f], tf.scale[f], tf.offset[f]);
+        dhi[node] = ref_coord(bmin[3 * c2[node] + f], tf.scale[f], tf.offset[f]);
+    }
 }
 
 // ---------------------------------------------------------------------------
@@ -1078,20 +1319,6 @@ static void kd_release(Context* ctx, KdForest* kd, void* p) {
         }
 }
 
-template <class T>
-static int kd_grow(Context* ctx, T** p, size_t old_n, size_t new_n, KdForest* kd, cudaStream_t st) {
-    T* q = nullptr;
-    int rc = kd_alloc(ctx, (void**)&q, new_n * sizeof(T), kd);
-    if (rc) return rc;
-    if (*p) {
-        cudaMemcpyAsync(q, *p, old_n * sizeof(T), cudaMemcpyDeviceToDevice, st);
-        cudaStreamSynchronize(st);
-        kd_release(ctx, kd, *p);
-    }
-    *p = q;
-    return NBG_OK;
-}
-
 uint64_t kd_bytes(uint64_t n) { return n * 28 + (n / 16 + 1024) * 68; }
 
 static void kd_forest_free(Context* ctx, KdForest* f) {
@@ -1108,103 +1335,34 @@ void kd_free(Context* ctx, Tile* t) {
     if (f && --f->refs <= 0) kd_forest_free(ctx, f);
 }
 
-// Builds the tile list of `S` segments; returns the number of tiles.
-static int kd_tiles(Context* ctx, KdForest* kd, const KdSeg* segs, uint32_t S, uint32_t* ntiles,
-                    cudaStream_t st) {
-    kd_seg_tiles_kernel<<<(S + 1 + 255) / 256, 256, 0, st>>>(segs, S, kd->nt);
-    size_t tb = kd->scan_bytes;
-    cub::DeviceScan::ExclusiveSum(kd->scan_tmp, tb, kd->nt, kd->nt, (int)(S + 1), st);
-    uint32_t total = 0;
-    cudaMemcpyAsync(&total, kd->nt + S, 4, cudaMemcpyDeviceToHost, st);
-    if (cudaStreamSynchronize(st) != cudaSuccess) {
-        set_err(ctx, "KD tile scan failed");
-        return NBG_ERR_CUDA;
-    }
-    if (total + 1 > kd->tile_cap) {
-        uint32_t cap = std::max<uint32_t>(total + 1, kd->tile_cap * 2);
-        if (kd->tile_seg) kd_release(ctx, kd, kd->tile_seg);
-        if (kd->tile_cnt) kd_release(ctx, kd, kd->tile_cnt);
-        kd->tile_seg = nullptr;
-        kd->tile_cnt = nullptr;
-        int rc = kd_alloc(ctx, (void**)&kd->tile_seg, (size_t)cap * 4, kd);
-        if (!rc) rc = kd_alloc(ctx, (void**)&kd->tile_cnt, (size_t)(cap + 1) * 8, kd);
-        if (rc) return rc;
-        kd->tile_cap = cap;
-    }
-    if (total) kd_fill_tiles_kernel<<<(total + 255) / 256, 256, 0, st>>>(kd->nt, S, total, kd->tile_seg);
-    NBG_LAUNCHED(3 + (total ? 1 : 0));
-    *ntiles = total;
-    return NBG_OK;
-}
-
-// Blocks of a level-pass launch over `ntiles` tiles: one per tile, or at most
-// the forest's cap when the build shares the SMs with a query.
-static unsigned kd_grid(const KdForest* kd, uint32_t ntiles) {
-    return kd->grid_cap ? std::min(ntiles, kd->grid_cap) : ntiles;
-}
-
-// known_tiles: the tile count when the tile map of `segs` is already built
-// (~0u: build it).
-template <int PASS>
-static int kd_pass(Context* ctx, KdForest* kd, const KdSeg* segs, uint32_t S, KdSplit* sp,
-                   cudaStream_t st, uint32_t known_tiles = ~0u) {
-    uint32_t ntiles = known_tiles;
-    if (known_tiles == ~0u) {
-        int rc = kd_tiles(ctx, kd, segs, S, &ntiles, st);
-        if (rc) return rc;
-    }
-    if (ntiles) {
-        kd_count_kernel<PASS><<<kd_grid(kd, ntiles), KD_THREADS, 0, st>>>(
-            segs, kd->nt, kd->tile_seg, sp, kd->rx, kd->ry, kd->rz, kd->tfs, kd->tile_cnt, ntiles);
-    }
-    cudaMemsetAsync(kd->tile_cnt + ntiles, 0, 8, st);
-    size_t tb = kd->scan_bytes;
-    cub::DeviceScan::ExclusiveSum(kd->scan_tmp, tb, kd->tile_cnt, kd->tile_cnt, (int)(ntiles + 1), st);
-    kd_seg_count_kernel<PASS><<<(S * 32 + 255) / 256, 256, 0, st>>>(segs, S, kd->nt, kd->tile_cnt,
-                                                                    sp, kd->rx, kd->ry, kd->rz,
-                                                                    kd->tfs);
-    if (ntiles) {
-        kd_classify_kernel<PASS><<<kd_grid(kd, ntiles), KD_THREADS, 0, st>>>(
-            segs, kd->nt, kd->tile_seg, kd->tile_cnt, sp, kd->rx, kd->ry, kd->rz, kd->tfs, kd->mlpos,
-            kd->mrpos, ntiles);
-        kd_swap_kernel<PASS><<<kd_grid(kd, ntiles), KD_THREADS, 0, st>>>(
-            segs, kd->nt, kd->tile_seg, sp, kd->mlpos, kd->mrpos, kd->rx, kd->ry, kd->rz, kd->rid, ntiles);
-    }
-    NBG_LAUNCHED(3 + (ntiles ? 3 : 0));
-    return cudaGetLastError() == cudaSuccess ? NBG_OK : NBG_ERR_CUDA;
-}
-
-static int kd_grow_nodes(Context* ctx, KdForest* kd, uint32_t nc, cudaStream_t st) {
-    const uint32_t old = kd->node_cap;
-    if (nc <= old) return NBG_OK;
-    int rc = kd_grow(ctx, &kd->c1, old, nc, kd, st);
-    if (!rc) rc = kd_grow(ctx, &kd->c2, old, nc, kd, st);
-    if (!rc) rc = kd_grow(ctx, &kd->feat, old, nc, kd, st);
-    if (!rc) rc = kd_grow(ctx, &kd->nb, old, nc, kd, st);
-    if (!rc) rc = kd_grow(ctx, &kd->ne, old, nc, kd, st);
-    if (!rc) rc = kd_grow(ctx, &kd->ntree, old, nc, kd, st);
-    if (!rc) rc = kd_grow(ctx, &kd->bmin, (size_t)old * 3, (size_t)nc * 3, kd, st);
-    if (!rc) rc = kd_grow(ctx, &kd->bmax, (size_t)old * 3, (size_t)nc * 3, kd, st);
-    if (rc) return rc;
-    kd->node_cap = nc;
-    return NBG_OK;
-}
-
 static unsigned grid_for(const Context* ctx, uint64_t n) {
     return (unsigned)std::max<uint64_t>(1, std::min<uint64_t>((n + 255) / 256, ctx->sm_count * 8));
 }
 
-// One build of the forest over `tiles`; `small_max` = 0 keeps every level on
-// the level passes (the fallback when a warp subtree overflows its stack or
-// the node arrays).
-static int kd_build(Context* ctx, KdForest* kd, Tile* const* tiles, uint32_t small_max,
-                    cudaStream_t st) {
+// Node arrays for `nc` nodes (nothing in them is kept).
+static int kd_alloc_nodes(Context* ctx, KdForest* kd, uint32_t nc) {
+    void** arrays[] = {(void**)&kd->c1, (void**)&kd->c2, (void**)&kd->feat, (void**)&kd->nb, (void**)&kd->ne,
+                       (void**)&kd->ntree, (void**)&kd->bmin, (void**)&kd->bmax, (void**)&kd->dlo, (void**)&kd->dhi};
+    static const size_t width[] = {4, 4, 4, 4, 4, 4, 12, 12, 8, 8};
+    for (int i = 0; i < 10; ++i) {
+        if (*arrays[i]) kd_release(ctx, kd, *arrays[i]);
+        *arrays[i] = nullptr;
+        const int rc = kd_alloc(ctx, arrays[i], (size_t)nc * width[i], kd);
+        if (rc) return rc;
+    }
+    kd->node_cap = nc;
+    return NBG_OK;
+}
+
+// One build of the forest over `tiles`.  Levels are queued without reading
+// anything back: the kernels take the segment and tile counts from the device,
+// and a level with nothing left exits at once.
+static int kd_build(Context* ctx, KdForest* kd, Tile* const* tiles, cudaStream_t st) {
     const int T = kd->ntrees;
-    int rc = NBG_OK;
     std::vector<KdSeg> level0, small0;
-    std::vector<uint32_t> leaves0;
-    std::vector<int32_t> c_init(T, -1), f_init(T, 0), tree_init(T);
-    std::vector<uint32_t> nb_init(T), ne_init(T);
+    std::vector<int32_t> box(6 * (size_t)T);
+    std::vector<int32_t> init(6 * (size_t)T);  // c1, c2, feat, nb, ne, ntree of the roots
+    uint64_t largest = 0;
     for (int k = 0; k < T; ++k) {
         const Tile* t = tiles[k];
         const uint64_t b = kd->base[k], n = kd->npts[k];
@@ -1223,153 +1381,137 @@ static int kd_build(Context* ctx, KdForest* kd, Tile* const* tiles, uint32_t sma
             root.hi[d] = (double)mx[d] * t->tf.scale[d] + t->tf.offset[d];
             kd->rootbox[6 * k + d] = root.lo[d];
             kd->rootbox[6 * k + 3 + d] = root.hi[d];
+            box[3 * k + d] = mn[d];
+            box[3 * (T + k) + d] = mx[d];
         }
-        tree_init[k] = k;
-        nb_init[k] = root.begin;
-        ne_init[k] = root.end;
-        if (n > (uint64_t)KD_LEAF && n > small_max) level0.push_back(root);
-        else if (n > (uint64_t)KD_LEAF) small0.push_back(root);
-        else leaves0.push_back((uint32_t)k);
+        init[k] = init[T + k] = -1;
+        init[2 * T + k] = 0;
+        init[3 * T + k] = (int32_t)root.begin;
+        init[4 * T + k] = (int32_t)root.end;
+        init[5 * T + k] = k;
+        if (n > KD_BLOCK_MAX) level0.push_back(root);
+        else small0.push_back(root);
+        largest = std::max(largest, n);
     }
     NBG_LAUNCHED(T);
-    if (level0.size() > kd->seg_cap || small0.size() > kd->seg_cap || leaves0.size() > kd->leaf_cap) {
+    if (level0.size() > kd->seg_cap || small0.size() > kd->small_cap) {
         set_err(ctx, "KD replica: too many trees for the segment lists");
         return NBG_ERR_UNSUPPORTED;
     }
-    // root nodes 0..T-1 (host arrays outlive the copies: the stream is synchronised below)
-    cudaMemcpyAsync(kd->c1, c_init.data(), T * 4, cudaMemcpyHostToDevice, st);
-    cudaMemcpyAsync(kd->c2, c_init.data(), T * 4, cudaMemcpyHostToDevice, st);
-    cudaMemcpyAsync(kd->feat, f_init.data(), T * 4, cudaMemcpyHostToDevice, st);
-    cudaMemcpyAsync(kd->nb, nb_init.data(), T * 4, cudaMemcpyHostToDevice, st);
-    cudaMemcpyAsync(kd->ne, ne_init.data(), T * 4, cudaMemcpyHostToDevice, st);
-    cudaMemcpyAsync(kd->ntree, tree_init.data(), T * 4, cudaMemcpyHostToDevice, st);
-    cudaMemcpyAsync(kd->tfs, kd->tfh.data(), T * sizeof(Transform), cudaMemcpyHostToDevice, st);
-    if (!level0.empty())
-        cudaMemcpyAsync(kd->seg[0], level0.data(), level0.size() * sizeof(KdSeg), cudaMemcpyHostToDevice, st);
-    if (!small0.empty())
-        cudaMemcpyAsync(kd->small, small0.data(), small0.size() * sizeof(KdSeg), cudaMemcpyHostToDevice, st);
-    if (!leaves0.empty())
-        cudaMemcpyAsync(kd->leaves, leaves0.data(), leaves0.size() * 4, cudaMemcpyHostToDevice, st);
-    uint32_t cnt[5] = {0, (uint32_t)T, 0, (uint32_t)small0.size(), (uint32_t)leaves0.size()};
-    cudaMemcpyAsync(kd->counters, cnt, sizeof(cnt), cudaMemcpyHostToDevice, st);
-    if (cudaStreamSynchronize(st) != cudaSuccess) {
-        set_err(ctx, "KD replica init failed");
+    // root nodes 0..T-1 (the host arrays outlive the copies: pageable sources are
+    // taken before the calls return)
+    void* const roots[] = {kd->c1, kd->c2, kd->feat, kd->nb, kd->ne, kd->ntree};
+    cudaError_t e = cudaSuccess;
+    for (int i = 0; i < 6 && !e; ++i)
+        e = cudaMemcpyAsync(roots[i], &init[(size_t)i * T], T * 4, cudaMemcpyHostToDevice, st);
+    if (!e) e = cudaMemcpyAsync(kd->bmin, &box[0], T * 12, cudaMemcpyHostToDevice, st);
+    if (!e) e = cudaMemcpyAsync(kd->bmax, &box[3 * (size_t)T], T * 12, cudaMemcpyHostToDevice, st);
+    if (!e) e = cudaMemcpyAsync(kd->tfs, kd->tfh.data(), T * sizeof(Transform), cudaMemcpyHostToDevice, st);
+    if (!e) e = cudaMemcpyAsync(kd->bases, kd->base.data(), T * 8, cudaMemcpyHostToDevice, st);
+    if (!e && !level0.empty())
+        e = cudaMemcpyAsync(kd->seg[0], level0.data(), level0.size() * sizeof(KdSeg), cudaMemcpyHostToDevice, st);
+    if (!e && !small0.empty())
+        e = cudaMemcpyAsync(kd->small, small0.data(), small0.size() * sizeof(KdSeg), cudaMemcpyHostToDevice, st);
+    KdState state{};
+    state.nodes = (uint32_t)T;
+    state.small = (uint32_t)small0.size();
+    if (!e) e = cudaMemcpyAsync(kd->state, &state, sizeof(state), cudaMemcpyHostToDevice, st);
+    if (e) {
+        set_err(ctx, std::string("KD replica init failed: ") + cudaGetErrorString(e));
         return NBG_ERR_CUDA;
     }
-    uint32_t node_count = (uint32_t)T;
-    uint32_t S = (uint32_t)level0.size();
+    const KdNodes N{kd->c1, kd->c2, kd->feat, kd->nb, kd->ne, kd->bmin, kd->bmax, kd->ntree, kd->node_cap};
+    uint32_t built = 0;  // small segments whose subtrees are queued
+    auto subtrees = [&](uint32_t upto) -> int {
+        if (upto <= built) return NBG_OK;
+        if (cudaFuncSetAttribute(kd_block_build_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                 (int)sizeof(KdBlockShared)))
+            return NBG_ERR_CUDA;
+        if (kd->beside && cudaStreamWaitEvent(st, ctx->fev[0], 0)) return NBG_ERR_CUDA;
+        const uint32_t ns = upto - built;
+        kd_block_build_kernel<<<ns, KD_BTHREADS, sizeof(KdBlockShared), st>>>(
+            kd->small + built, kd->rx, kd->ry, kd->rz, kd->rid, kd->kpos, kd->bases, N, kd->state, kd->tfs);
+        NBG_LAUNCHED(1);
+        built = upto;
+        return NBG_OK;
+    };
     int cur = 0;
-    while (S > 0) {
-        // room for this level's children
-        if (node_count + 2 * S > kd->node_cap) {
-            rc = kd_grow_nodes(ctx, kd, std::max<uint32_t>(kd->node_cap * 2, node_count + 2 * S + 64), st);
-            if (rc) return rc;
-        }
-        const KdSeg* segs = kd->seg[cur];
-        uint32_t ntiles = 0;
-        kd_minmax_init_kernel<<<(S + 127) / 128, 128, 0, st>>>(kd->split, S);
-        rc = kd_tiles(ctx, kd, segs, S, &ntiles, st);
-        if (rc) return rc;
-        if (ntiles)
-            kd_minmax_kernel<<<kd_grid(kd, ntiles), KD_THREADS, 0, st>>>(segs, kd->nt, kd->tile_seg, kd->rx,
-                                                                         kd->ry, kd->rz, kd->split, ntiles);
-        kd_split_kernel<<<(S + 127) / 128, 128, 0, st>>>(segs, S, kd->split, kd->tfs, kd->bmin, kd->bmax);
-        NBG_LAUNCHED(2 + (ntiles ? 1 : 0));
-        // pass 1 runs on the same segments: their tile map is already built
-        rc = kd_pass<1>(ctx, kd, segs, S, kd->split, st, ntiles);
-        if (rc) return rc;
-        // pass 2 only where points equal the cut value
-        cudaMemsetAsync(kd->counters + 5, 0, 4, st);
-        kd_pass2_plan_kernel<<<(S + 127) / 128, 128, 0, st>>>(segs, S, kd->split, kd->seg2,
-                                                              kd->split2, kd->seg2_from,
-                                                              kd->counters + 5);
-        uint32_t S2 = 0;
-        cudaMemcpyAsync(&S2, kd->counters + 5, 4, cudaMemcpyDeviceToHost, st);
-        if (cudaStreamSynchronize(st) != cudaSuccess) {
-            set_err(ctx, "KD replica pass-2 plan failed");
-            return NBG_ERR_CUDA;
-        }
+    auto level = [&](int c) {
+        KdLevel lv;
+        lv.segs = kd->seg[c];
+        lv.sp = kd->split[c];
+        lv.next = kd->seg[c ^ 1];
+        lv.next_sp = kd->split[c ^ 1];
+        lv.small = kd->small;
+        lv.tile_seg = kd->tile_seg;
+        lv.tile_cnt = kd->tile_cnt;
+        lv.st = kd->state;
+        lv.rx = kd->rx;
+        lv.ry = kd->ry;
+        lv.rz = kd->rz;
+        lv.rid = kd->rid;
+        lv.mlpos = kd->mlpos;
+        lv.mrpos = kd->mrpos;
+        lv.tfs = kd->tfs;
+        lv.N = N;
+        lv.seg_cap = kd->seg_cap;
+        lv.small_cap = kd->small_cap;
+        lv.tile_cap = kd->tile_cap;
+        return lv;
+    };
+    if (!level0.empty()) {
+        kd_roots_kernel<<<1, KD_THREADS, 0, st>>>(level(0), (uint32_t)level0.size());
         NBG_LAUNCHED(1);
-        if (S2) {
-            rc = kd_pass<2>(ctx, kd, kd->seg2, S2, kd->split2, st);
+        const uint32_t most = std::min<uint32_t>(kd->tile_cap, (uint32_t)ctx->sm_count * 8);
+        const unsigned blocks = kd->grid_cap ? std::min(most, kd->grid_cap) : most;
+        // halving gets the largest tree to KD_BLOCK_MAX in `depth` levels;
+        // midpoint cuts are uneven, so a few more are queued before looking
+        int depth = 1;
+        while ((largest >> depth) > KD_BLOCK_MAX) ++depth;
+        int queued = depth + 2;
+        while (true) {
+            for (int l = 0; l < queued; ++l) {
+                const KdLevel lv = level(cur);
+                kd_count_kernel<1><<<blocks, KD_THREADS, 0, st>>>(lv);
+                kd_classify_kernel<1><<<blocks, KD_THREADS, 0, st>>>(lv);
+                kd_swap_kernel<1><<<blocks, KD_THREADS, 0, st>>>(lv);
+                kd_count_kernel<2><<<blocks, KD_THREADS, 0, st>>>(lv);
+                kd_classify_kernel<2><<<blocks, KD_THREADS, 0, st>>>(lv);
+                kd_swap_kernel<2><<<blocks, KD_THREADS, 0, st>>>(lv);
+                cur ^= 1;
+            }
+            NBG_LAUNCHED(6 * queued);
+            e = cudaGetLastError();
+            if (!e) e = cudaMemcpyAsync(&state, kd->state, sizeof(state), cudaMemcpyDeviceToHost, st);
+            if (!e) e = cudaStreamSynchronize(st);
+            if (e) {
+                set_err(ctx, std::string("KD replica build failed: ") + cudaGetErrorString(e));
+                return NBG_ERR_CUDA;
+            }
+            if (state.errors) return KD_RETRY;
+            const int rc = subtrees(state.small);
             if (rc) return rc;
-            kd_pass2_done_kernel<<<(S2 + 127) / 128, 128, 0, st>>>(S2, kd->split2, kd->seg2_from,
-                                                                   kd->split);
-            NBG_LAUNCHED(1);
+            if (!state.segs) break;
+            queued = 3;
         }
-        cudaMemsetAsync(kd->counters, 0, 4, st);
-        NBG_LAUNCHED(2);
-        kd_children_kernel<<<(S + 127) / 128, 128, 0, st>>>(segs, S, kd->split, kd->seg[cur ^ 1],
-                                                            kd->counters, kd->c1, kd->c2, kd->feat,
-                                                            kd->nb, kd->ne, kd->node_cap,
-                                                            kd->seg_cap, kd->small, small_max,
-                                                            kd->leaves, kd->leaf_cap, kd->ntree);
-        cudaMemcpyAsync(cnt, kd->counters, sizeof(cnt), cudaMemcpyDeviceToHost, st);
-        cudaError_t be = cudaGetLastError();
-        if (be == cudaSuccess) be = cudaStreamSynchronize(st);
-        if (be != cudaSuccess) {
-            set_err(ctx, std::string("KD replica build failed: ") + cudaGetErrorString(be));
-            return NBG_ERR_CUDA;
-        }
-        if (cnt[2]) {
-            set_err(ctx, "KD replica build ran out of node or segment capacity");
-            return NBG_ERR_UNSUPPORTED;
-        }
-        node_count = cnt[1];
-        S = cnt[0];
-        cur ^= 1;
-    }
-    // subtrees of the small segments, one warp each
-    const uint32_t nsmall = cnt[3], nleaves = cnt[4];
-    const uint64_t n = kd->n;
-    if (nsmall) {
-        rc = kd_grow_nodes(ctx, kd, std::max<uint32_t>(kd->node_cap, node_count + (uint32_t)(n / 8) + 1024), st);
+    } else {
+        const int rc = subtrees(state.small);
         if (rc) return rc;
-        const uint32_t wblocks = (nsmall + KD_WARPS - 1) / KD_WARPS;
-        kd_warp_build_kernel<<<kd->wgrid_cap ? std::min(wblocks, kd->wgrid_cap) : wblocks, 32 * KD_WARPS, 0, st>>>(
-            kd->small, nsmall, kd->rx, kd->ry, kd->rz, kd->rid, kd->mlpos, kd->mrpos, kd->c1, kd->c2,
-            kd->feat, kd->nb, kd->ne, kd->bmin, kd->bmax, kd->counters, kd->node_cap, kd->tfs,
-            kd->ntree);
-        NBG_LAUNCHED(1);
     }
-    if (nleaves)
-        kd_leaf_bbox_kernel<<<(nleaves * 32 + 127) / 128, 128, 0, st>>>(
-            kd->leaves, nleaves, kd->nb, kd->ne, kd->rx, kd->ry, kd->rz, kd->bmin, kd->bmax);
-    cudaMemcpyAsync(cnt, kd->counters, sizeof(cnt), cudaMemcpyDeviceToHost, st);
-    cudaError_t we = cudaGetLastError();
-    if (we == cudaSuccess) we = cudaStreamSynchronize(st);
-    if (we != cudaSuccess) {
-        set_err(ctx, std::string("KD replica subtree build failed: ") + cudaGetErrorString(we));
-        return NBG_ERR_CUDA;
-    }
-    if (cnt[2]) return KD_RETRY;
-    node_count = cnt[1];
-    kd->node_count = node_count;
     // divlow / divhigh from the children's extents
-    const uint32_t nn = node_count;
-    if (!kd->dlo || kd->dl_cap < nn) {
-        if (kd->dlo) kd_release(ctx, kd, kd->dlo);
-        if (kd->dhi) kd_release(ctx, kd, kd->dhi);
-        kd->dlo = kd->dhi = nullptr;
-        rc = kd_alloc(ctx, (void**)&kd->dlo, (size_t)nn * 8, kd);
-        if (!rc) rc = kd_alloc(ctx, (void**)&kd->dhi, (size_t)nn * 8, kd);
-        if (rc) return rc;
-        kd->dl_cap = nn;
-    }
-    kd_div_kernel<<<(nn + 127) / 128, 128, 0, st>>>(nn, kd->c1, kd->c2, kd->feat, kd->bmin,
-                                                    kd->bmax, kd->tfs, kd->ntree, kd->dlo, kd->dhi);
-    if (!kd->kpos) {
-        rc = kd_alloc(ctx, (void**)&kd->kpos, n * 4, kd);
-        if (rc) return rc;
-    }
-    for (int k = 0; k < T; ++k)
-        kd_inverse_kernel<<<grid_for(ctx, kd->npts[k]), 256, 0, st>>>(kd->rid, kd->base[k],
-                                                                      kd->npts[k], kd->kpos);
-    NBG_LAUNCHED(1 + T + (nleaves ? 1 : 0));
-    if (cudaStreamSynchronize(st) != cudaSuccess) {
-        set_err(ctx, "KD replica extents failed");
+    kd_div_kernel<<<grid_for(ctx, kd->node_cap / 8), 256, 0, st>>>(kd->state, kd->c1, kd->c2, kd->feat, kd->bmin,
+                                                                   kd->bmax, kd->tfs, kd->ntree, kd->dlo, kd->dhi,
+                                                                   kd->node_cap);
+    NBG_LAUNCHED(1);
+    e = cudaGetLastError();
+    if (!e) e = cudaMemcpyAsync(&state, kd->state, sizeof(state), cudaMemcpyDeviceToHost, st);
+    if (!e) e = cudaStreamSynchronize(st);
+    if (e) {
+        set_err(ctx, std::string("KD replica subtree build failed: ") + cudaGetErrorString(e));
         return NBG_ERR_CUDA;
     }
+    if (state.errors) return KD_RETRY;
+    kd->node_count = state.nodes;
     return NBG_OK;
 }
 
@@ -1398,7 +1540,7 @@ int kd_ensure_many(Context* ctx, Tile* const* tiles, int count, cudaStream_t st,
     kd->n = n;
     if (beside_query && n >= kKdBesideMinPoints) {
         kd->grid_cap = (uint32_t)(kKdBesideBlocksPerSm * ctx->sm_count);
-        kd->wgrid_cap = (uint32_t)(kKdBesideWarpBlocksPerSm * ctx->sm_count);
+        kd->beside = true;
     }
     kd->rootbox.assign(6 * (size_t)kd->ntrees, 0.0);
     const int T = kd->ntrees;
@@ -1408,35 +1550,34 @@ int kd_ensure_many(Context* ctx, Tile* const* tiles, int count, cudaStream_t st,
     if (!rc) rc = kd_alloc(ctx, (void**)&kd->rid, n * 4, kd);
     if (!rc) rc = kd_alloc(ctx, (void**)&kd->mlpos, n * 4, kd);
     if (!rc) rc = kd_alloc(ctx, (void**)&kd->mrpos, n * 4, kd);
-    kd->seg_cap = (uint32_t)(n / 50 + 64 + T);
-    if (!rc) rc = kd_alloc(ctx, (void**)&kd->seg[0], kd->seg_cap * sizeof(KdSeg), kd);
-    if (!rc) rc = kd_alloc(ctx, (void**)&kd->seg[1], kd->seg_cap * sizeof(KdSeg), kd);
-    if (!rc) rc = kd_alloc(ctx, (void**)&kd->seg2, kd->seg_cap * sizeof(KdSeg), kd);
-    if (!rc) rc = kd_alloc(ctx, (void**)&kd->small, kd->seg_cap * sizeof(KdSeg), kd);
-    if (!rc) rc = kd_alloc(ctx, (void**)&kd->split, kd->seg_cap * sizeof(KdSplit), kd);
-    if (!rc) rc = kd_alloc(ctx, (void**)&kd->split2, kd->seg_cap * sizeof(KdSplit), kd);
-    if (!rc) rc = kd_alloc(ctx, (void**)&kd->seg2_from, kd->seg_cap * 4, kd);
-    if (!rc) rc = kd_alloc(ctx, (void**)&kd->nt, (kd->seg_cap + 1) * 4, kd);
-    kd->leaf_cap = (uint32_t)(n / 16 + 1024 + T);
-    if (!rc) rc = kd_alloc(ctx, (void**)&kd->leaves, (size_t)kd->leaf_cap * 4, kd);
+    if (!rc) rc = kd_alloc(ctx, (void**)&kd->kpos, n * 4, kd);
+    // a level's segments hold more than KD_BLOCK_MAX points each
+    kd->seg_cap = (uint32_t)(n / KD_BLOCK_MAX + 1);
+    for (int i = 0; i < 2; ++i) {
+        if (!rc) rc = kd_alloc(ctx, (void**)&kd->seg[i], kd->seg_cap * sizeof(KdSeg), kd);
+        if (!rc) rc = kd_alloc(ctx, (void**)&kd->split[i], kd->seg_cap * sizeof(KdSplit), kd);
+    }
+    kd->small_cap = (uint32_t)(n / 64 + 1024 + T);
+    if (!rc) rc = kd_alloc(ctx, (void**)&kd->small, (size_t)kd->small_cap * sizeof(KdSeg), kd);
+    kd->tile_cap = (uint32_t)(n / KD_TILE + kd->seg_cap + 1);
+    if (!rc) rc = kd_alloc(ctx, (void**)&kd->tile_seg, (size_t)kd->tile_cap * 4, kd);
+    if (!rc) rc = kd_alloc(ctx, (void**)&kd->tile_cnt, ((size_t)kd->tile_cap + 1) * 8, kd);
+    if (!rc) rc = kd_alloc(ctx, (void**)&kd->state, sizeof(KdState), kd);
     if (!rc) rc = kd_alloc(ctx, (void**)&kd->counters, 64, kd);
     if (!rc) rc = kd_alloc(ctx, (void**)&kd->tfs, (size_t)T * sizeof(Transform), kd);
-    size_t b1 = 0, b2 = 0;
-    cub::DeviceScan::ExclusiveSum(nullptr, b1, (uint32_t*)nullptr, (uint32_t*)nullptr,
-                                  (int)(n / KD_TILE + kd->seg_cap + 2));
-    cub::DeviceScan::ExclusiveSum(nullptr, b2, (unsigned long long*)nullptr,
-                                  (unsigned long long*)nullptr, (int)(n / KD_TILE + kd->seg_cap + 2));
-    b1 = std::max(b1, b2);
-    kd->scan_bytes = b1;
-    if (!rc) rc = kd_alloc(ctx, (void**)&kd->scan_tmp, b1, kd);
-    if (!rc) rc = kd_grow_nodes(ctx, kd, (uint32_t)(n / 25 + 64 + 2 * (uint64_t)T), st);
+    if (!rc) rc = kd_alloc(ctx, (void**)&kd->bases, (size_t)T * 8, kd);
+    if (!rc) rc = kd_alloc_nodes(ctx, kd, (uint32_t)(n / 16 + 1024 + 2 * (uint64_t)T));
     if (!rc) {
-        rc = kd_build(ctx, kd, todo.data(), KD_WARP_MAX, st);
+        rc = kd_build(ctx, kd, todo.data(), st);
         if (rc == KD_RETRY) {
-            // a warp subtree overflowed its stack or the node arrays: redo the
-            // whole build with the level passes only
-            rc = kd_grow_nodes(ctx, kd, (uint32_t)std::min<uint64_t>(2 * n + 64 + 2 * (uint64_t)T, UINT32_MAX), st);
-            if (!rc) rc = kd_build(ctx, kd, todo.data(), 0, st);
+            // a very uneven tree outgrew the node or subtree lists: build it again
+            // with room for every node it can have
+            kd_release(ctx, kd, kd->small);
+            kd->small_cap = (uint32_t)(n + T);
+            rc = kd_alloc(ctx, (void**)&kd->small, (size_t)kd->small_cap * sizeof(KdSeg), kd);
+            if (!rc)
+                rc = kd_alloc_nodes(ctx, kd, (uint32_t)std::min<uint64_t>(2 * n + 64 + 2 * (uint64_t)T, UINT32_MAX));
+            if (!rc) rc = kd_build(ctx, kd, todo.data(), st);
             if (rc == KD_RETRY) {
                 set_err(ctx, "KD replica build ran out of node capacity");
                 rc = NBG_ERR_UNSUPPORTED;

@@ -1136,7 +1136,7 @@ struct LaunchArgs {
     QueryArgs q;
     cudaStream_t stream;
     cudaStream_t fork = nullptr;   // second stream for the handed-back rows (null: `stream`)
-    cudaEvent_t fev[3] = {};       // fork, handed-back rows done, finish done
+    cudaEvent_t fev[3] = {};       // select done (fork), handed-back rows done, finish done
     cudaEvent_t done = nullptr;    // QueryLaunch::done
     bool ids;
     int group = 0;        // select kernel (nbg_tile_set_select; 0: two-pass per-thread)
@@ -1204,6 +1204,7 @@ struct KnnLauncher {
         if (la.group == 1 && la.q.sums && !la.ids) {
             const uint64_t b256 = (rows + 255) / 256;
             knn_select_morton_kernel<KS><<<(unsigned)b256, 256, 0, la.stream>>>(la.q);
+            if (la.fork && cudaEventRecord(la.fev[0], la.stream)) return NBG_ERR_CUDA;
             knn_finish_kernel<<<(unsigned)blocks, threads, 0, la.stream>>>(la.q);
             NBG_LAUNCHED(2);
             return cudaGetLastError() == cudaSuccess ? NBG_OK : NBG_ERR_CUDA;
@@ -1222,6 +1223,7 @@ struct KnnLauncher {
                                    0, la.stream>>>(r);
             NBG_LAUNCHED(1);
             if (!la.ids) {
+                if (la.fork && cudaEventRecord(la.fev[0], la.stream)) return NBG_ERR_CUDA;
                 knn_finish_kernel<<<(unsigned)blocks, threads, 0, la.stream>>>(la.q);
                 NBG_LAUNCHED(1);
             }
@@ -1232,6 +1234,7 @@ struct KnnLauncher {
             NBG_LAUNCHED(1);
         } else if (la.q.sums) {
             knn_select_kernel<KS><<<(unsigned)blocks, threads, 0, la.stream>>>(la.q);
+            if (la.fork && cudaEventRecord(la.fev[0], la.stream)) return NBG_ERR_CUDA;
             knn_finish_kernel<<<(unsigned)blocks, threads, 0, la.stream>>>(la.q);
             NBG_LAUNCHED(2);
         } else {
