@@ -273,6 +273,11 @@ int ensure_scratch(Context* ctx, uint64_t n, uint64_t ex_cap) {
     return NBG_OK;
 }
 
+// the point keys, later the box tree of the clump order
+static size_t keys_bytes(uint64_t n) {
+    return std::max<size_t>(n * 4, ClumpTree(n).off[ClumpTree::kLevels] * sizeof(float));
+}
+
 static void tile_release(Context* ctx, Tile* t) {
     kd_free(ctx, t);
     const uint64_t n = t->n;
@@ -284,7 +289,7 @@ static void tile_release(Context* ctx, Tile* t) {
     dev_free(ctx, t->colinfo, t->cols_cap * 16);
     dev_free(ctx, t->ext, (t->cols_cap + 1) * 4);
     dev_free(ctx, t->table_dev, 16);
-    dev_free(ctx, t->keys, n * 4);
+    dev_free(ctx, t->keys, keys_bytes(n));
     dev_free(ctx, t->cstart, t->table_cap * 4);
     dev_free(ctx, t->cursor, t->table_cap * 4);
     dev_free(ctx, t->sorted, n * 16);
@@ -512,7 +517,8 @@ int tile_alloc(Context* ctx, uint64_t n, const double scale[3], const double off
     ALLOC(t->colinfo, t->cols_cap * 16);
     ALLOC(t->ext, (t->cols_cap + 1) * 4);
     ALLOC(t->table_dev, 16);
-    ALLOC(t->keys, n * 4);
+    ALLOC(t->keys, keys_bytes(n));
+    t->clumps = true;
     ALLOC(t->cstart, t->table_cap * 4);
     ALLOC(t->cursor, t->table_cap * 4);
     ALLOC(t->sorted, n * 16);
@@ -743,7 +749,7 @@ struct PipeStats {
     uint64_t tie_rows = 0, deferred_rows = 0, replay_rows = 0, retry_rows = 0;
 };
 
-static int run_pipelined(Context* ctx, Tile* t, int K, const StageGroup& g, const ExceptionSink& sink,
+static int run_pipelined(Context* ctx, Tile* t, int K, int select, const StageGroup& g, const ExceptionSink& sink,
                          const char* dev_records, char* host_records, size_t record_bytes, int C,
                          cudaStream_t stream, PipeStats& ps) {
     NBG_RANGE("nbg pipelined query");
@@ -771,7 +777,7 @@ static int run_pipelined(Context* ctx, Tile* t, int K, const StageGroup& g, cons
     }
     if (!e) e = cudaEventCreateWithFlags(&done, cudaEventDisableTiming);
     if (e) rc = fail(ctx, NBG_ERR_CUDA, std::string("pipeline setup: ") + cudaGetErrorString(e));
-    if (!rc) rc = build_id_chunks(ctx, t, b, C, rows, ctx->counters + 48, stream);
+    if (!rc) rc = build_id_chunks(ctx, t, b, C, rows, ctx->counters + 48, select >= 8, stream);
     const bool speculative = !(t->kd && kd_built(t));
     auto finish_chunk = [&](int c) -> int {
         const uint32_t rows_c = (uint32_t)(b[c + 1] - b[c]);
@@ -836,7 +842,7 @@ static int run_pipelined(Context* ctx, Tile* t, int K, const StageGroup& g, cons
         ql.rows = rows + b[c];
         ql.nrows = b[c + 1] - b[c];
         ql.retry_rows = ctx->retry_rows + b[c];
-        ql.group = t->group;
+        ql.group = select;
         ql.margin0 = t->margin0;
         // sel[c] marks the chunk's rows answered; the next chunk's select may
         // start while this chunk's handed-back rows still run
@@ -1169,6 +1175,11 @@ extern "C" int nbg_run(nbg_context* h, nbg_tile* th, const nbg_stage_opts* stage
             }
             continue;
         }
+        const int select = select_kernel(t, K);
+        if (!radius_group && select >= 8) {
+            rc = ensure_clumps(ctx, t, stream);
+            if (rc) { cleanup(); return fail(ctx, rc, "clump order"); }
+        }
         if (radius_group) {
             RadiusLaunch rl;
             rl.tile = t;
@@ -1190,7 +1201,7 @@ extern "C" int nbg_run(nbg_context* h, nbg_tile* th, const nbg_stage_opts* stage
         }
         if (pipelined) {
             PipeStats ps;
-            rc = run_pipelined(ctx, t, K, g, sink, packed_dev, (char*)outputs[0].base,
+            rc = run_pipelined(ctx, t, K, select, g, sink, packed_dev, (char*)outputs[0].base,
                                (size_t)outputs[0].point_stride, pipe_chunks, stream, ps);
             if (rc) { cleanup(); return rc; }
             float ms = 0;
@@ -1219,7 +1230,7 @@ extern "C" int nbg_run(nbg_context* h, nbg_tile* th, const nbg_stage_opts* stage
         ql.sums = ctx->sums;
         ql.row_k = row_k;
         ql.retry_rows = ctx->retry_rows;
-        ql.group = t->group;
+        ql.group = select;
         ql.margin0 = t->margin0;
         // the KD replica does not depend on the query: build it on the side
         // stream while the query kernel runs (tie rows almost always need it)
@@ -1406,6 +1417,17 @@ static std::pair<int, int> tuning_class(const Tile* t, int K) {
     return std::make_pair(lg, slots_for_k(K));
 }
 
+// The library's choice for a tile nobody tuned.  Long lists go to the group
+// select: an insertion into a sorted list of K + 1 registers costs 2 (K + 1)
+// min/max whenever any lane inserts, the group select's batch merge a tenth of
+// that (1.5M points, knn = 64: select 11.9 ms per thread, 5.5 ms grouped; at
+// knn = 32 the two are even, 1.0 and 1.1 ms on 300k points, and below it the
+// per-thread search reads fewer candidates).
+int select_kernel(const Tile* t, int K) {
+    if (t->group >= 0) return t->group;
+    return t->clumps && slots_for_k(K) >= 50 ? 32 : 0;
+}
+
 // A tile the caller did not tune takes the context's cached choice for its
 // class (from nbg_tile_autotune or a loaded tuning file), if there is one.
 // The batched form tunes its tiles through the autotuner's cache itself.
@@ -1487,6 +1509,10 @@ int tile_autotune(Context* ctx, Tile* t, int32_t knn, const float* candidates, i
         rc = ensure_grid(ctx, t, K, stream);
         if (rc) break;
         cudaEventRecord(ctx->ev[1], stream);
+        if (!per_thread_only) {
+            rc = ensure_clumps(ctx, t, stream);
+            if (rc) break;
+        }
         for (int gi = 0; gi < ngroups; ++gi) {
             const int G = kGroups[gi];
             QueryLaunch ql;
@@ -1623,9 +1649,12 @@ extern "C" int nbg_neighbor_sets(nbg_context* h, nbg_tile* th, int32_t knn, uint
         if (rc) return rc;
     }
     cudaMemsetAsync(ctx->counters, 0, 64 * sizeof(uint32_t), stream);
-    rc = launch_neighbor_sets(ctx, t, K, 8, dev_ids, ctx->exact_rows, ctx->counters, ctx->ties,
-                              (uint32_t)std::min<uint64_t>(ctx->tie_cap, UINT32_MAX), stream,
-                              ctx->retry_rows);
+    const int select = select_kernel(t, K);
+    if (select >= 8) rc = ensure_clumps(ctx, t, stream);
+    if (!rc)
+        rc = launch_neighbor_sets(ctx, t, K, 8, dev_ids, ctx->exact_rows, ctx->counters, ctx->ties,
+                                  (uint32_t)std::min<uint64_t>(ctx->tie_cap, UINT32_MAX), stream,
+                                  ctx->retry_rows, select);
     uint32_t cnt[5] = {0, 0, 0, 0, 0};
     cudaError_t e = cudaSuccess;
     if (!rc) {

@@ -267,6 +267,7 @@ extern "C" int nbg_run_batch(nbg_context* h, const nbg_batch_item* items, int32_
         const Tile* t = &items[i].tile->t;
         QueryArgs q{};
         q.gv = grid_view(t);
+        q.qpts = t->sorted;
         q.gp = t->gp;
         q.n = t->n;
         q.K = Ks[i];

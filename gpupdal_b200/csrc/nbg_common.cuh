@@ -23,7 +23,32 @@ struct GridParams {
     int32_t gx, gy, gz;
     uint32_t ncols;    // gx*gy
     uint32_t cap_hit;  // cell size had to grow to fit the column directory
+    int32_t tgx;       // columns are laid out in 64 x 64 tiles, tgx tiles a row (0: row by row)
+    uint32_t nslots;   // column slots of that layout (tiles at the edge are padded)
+    float r1;          // radius holding one point at the tile's planar density
 };
+
+// Slot of column (cx, cy) in the layout of the columns' runs of cells: Morton
+// order inside 64 x 64 tiles, so that consecutive cells (and the points in
+// cell order) stay near in both directions.
+__host__ __device__ __forceinline__ uint32_t column_slot(const GridParams& g, uint32_t cx, uint32_t cy) {
+    if (!g.tgx) return cy * (uint32_t)g.gx + cx;
+    uint32_t m = (cx & 63u) | (cy & 63u) << 16;
+    m = (m | m << 4) & 0x0F0F0F0Fu;
+    m = (m | m << 2) & 0x33333333u;
+    m = (m | m << 1) & 0x55555555u;
+    return ((cy >> 6) * (uint32_t)g.tgx + (cx >> 6)) * 4096u + ((m & 0xFFFFu) | (m >> 16) << 1);
+}
+
+// 10-bit Morton interleave of three coordinates.
+__device__ __forceinline__ uint32_t spread3(uint32_t v) {
+    v &= 0x3FFu;
+    v = (v | (v << 16)) & 0x030000FFu;
+    v = (v | (v << 8)) & 0x0300F00Fu;
+    v = (v | (v << 4)) & 0x030C30C3u;
+    v = (v | (v << 2)) & 0x09249249u;
+    return v;
+}
 
 // Device pointers of a tile's grid.
 struct GridView {
@@ -119,6 +144,34 @@ struct QueryArgs {
     uint64_t nq = 0;                 // entries of `rows`
     const uint32_t* nq_dev = nullptr;  // entries of `rows` read on the device (retry launches)
     uint32_t* retry_rows = nullptr;    // group select: rows it hands to the per-thread select
+    // the points the rows index: gv.sorted, or the clump order of the group
+    // select (rows, sums and retry_rows then hold its slots), with the boxes
+    // of the clumps (ClumpTree)
+    const float4* qpts = nullptr;
+    const float* boxes = nullptr;
+};
+
+// Bounding boxes over the clump order: clumps of 32 consecutive slots, then
+// 32-ary parents up to a level of at most 32 nodes.  Level l's boxes are six
+// arrays (lo x, y, z, hi x, y, z) of count[l] floats from off[l].
+struct ClumpTree {
+    static constexpr int kLevels = 7;  // 32^7 slots
+    uint32_t count[kLevels];
+    uint64_t off[kLevels + 1];
+    int top;  // first level of at most 32 nodes
+    __host__ __device__ explicit ClumpTree(uint64_t n) {
+        uint64_t c = (n + 31) / 32, o = 0;
+        top = -1;
+#pragma unroll
+        for (int l = 0; l < kLevels; ++l) {
+            count[l] = (uint32_t)c;
+            off[l] = o;
+            o += 6 * c;
+            if (top < 0 && c <= 32) top = l;
+            c = (c + 31) / 32;
+        }
+        off[kLevels] = o;
+    }
 };
 
 // Neighbour count of a row: K, or the point's OptimalKNN rounded half away

@@ -102,14 +102,21 @@ __global__ void grid_config_kernel(const int32_t* bb, uint64_t n, int k1, float 
         g.cap_hit = 1;
     }
     g.cell = (int32_t)c;
+    g.r1 = (float)sqrt(ex * ey / (3.14159265358979 * (double)n));
     g.ncols = (uint32_t)g.gx * (uint32_t)g.gy;
+    // tiled layout of the columns' runs where its padded slots fit the directory
+    const uint64_t tx = ((uint64_t)g.gx + 63) / 64, ty = ((uint64_t)g.gy + 63) / 64;
+    g.tgx = tx * ty * 4096 <= cols_cap ? (int32_t)tx : 0;
+    g.nslots = g.tgx ? (uint32_t)(tx * ty * 4096) : g.ncols;
     *gp = g;
 }
 
-__global__ void col_init_kernel(uint32_t ncols_cap, int4* __restrict__ colinfo) {
-    for (uint32_t c = blockIdx.x * blockDim.x + threadIdx.x; c < ncols_cap;
-         c += gridDim.x * blockDim.x)
-        colinfo[c] = make_int4(0, INT32_MAX, -1, 0);
+__global__ void col_init_kernel(uint32_t ncols_cap, int4* __restrict__ colinfo, uint32_t* __restrict__ ext) {
+    for (uint32_t c = blockIdx.x * blockDim.x + threadIdx.x; c <= ncols_cap;
+         c += gridDim.x * blockDim.x) {
+        if (c < ncols_cap) colinfo[c] = make_int4(0, INT32_MAX, -1, 0);
+        ext[c] = 0;
+    }
 }
 
 __global__ void col_zrange_kernel(const int32_t* __restrict__ x, const int32_t* __restrict__ y,
@@ -127,27 +134,25 @@ __global__ void col_zrange_kernel(const int32_t* __restrict__ x, const int32_t* 
     }
 }
 
+// Extents in layout order (column_slot), one past the last slot included;
+// the padded slots of edge tiles are cleared before.
 __global__ void col_extent_kernel(const GridParams* __restrict__ gpp,
                                   const int4* __restrict__ colinfo, uint32_t* __restrict__ ext) {
-    const uint32_t ncols = gpp->ncols;
-    for (uint32_t c = blockIdx.x * blockDim.x + threadIdx.x; c <= ncols;
-         c += gridDim.x * blockDim.x) {
-        uint32_t e = 0;
-        if (c < ncols) {
-            const int4 ci = colinfo[c];
-            e = ci.z >= ci.y ? (uint32_t)(ci.z - ci.y + 1) : 0u;
-        }
-        ext[c] = e;
+    const GridParams g = *gpp;
+    for (uint32_t c = blockIdx.x * blockDim.x + threadIdx.x; c < g.ncols; c += gridDim.x * blockDim.x) {
+        const int4 ci = colinfo[c];
+        ext[column_slot(g, c % (uint32_t)g.gx, c / (uint32_t)g.gx)] =
+            ci.z >= ci.y ? (uint32_t)(ci.z - ci.y + 1) : 0u;
     }
 }
 
 __global__ void col_base_kernel(const GridParams* __restrict__ gpp, const uint32_t* __restrict__ ext,
                                 int4* __restrict__ colinfo, uint32_t* __restrict__ table_size) {
-    const uint32_t ncols = gpp->ncols;
-    for (uint32_t c = blockIdx.x * blockDim.x + threadIdx.x; c <= ncols;
+    const GridParams g = *gpp;
+    for (uint32_t c = blockIdx.x * blockDim.x + threadIdx.x; c <= g.ncols;
          c += gridDim.x * blockDim.x) {
-        if (c < ncols) colinfo[c].x = (int)ext[c];
-        else *table_size = ext[c];
+        if (c < g.ncols) colinfo[c].x = (int)ext[column_slot(g, c % (uint32_t)g.gx, c / (uint32_t)g.gx)];
+        else *table_size = ext[g.nslots];
     }
 }
 
@@ -196,6 +201,177 @@ __global__ void cell_scatter_kernel(const int32_t* __restrict__ x, const int32_t
     }
 }
 
+// Clump order of the group select: every block of kClumpRows consecutive rows
+// (a patch of neighbouring columns) is halved at the median of its longest
+// side until 32 points are left, so a clump's box is small and square: ground,
+// wall and canopy points of a column come apart.  Against 32-point runs of a
+// Hilbert curve through the same blocks, a clump's search examines 166 instead
+// of 268 candidates (terrain, K = 17; 251 instead of 333 on the mixture).
+// Writes the points in that order, the clumps' boxes and the blocks' boxes.
+static constexpr int kClumpRows = 1024;
+
+// Ascending bitonic sort of each segment of SEG threads' keys (one each):
+// shuffles inside a warp, shared memory across.
+template <int SEG>
+__device__ __forceinline__ uint32_t sort_segment(uint32_t key, uint32_t* sh) {
+    const int tid = threadIdx.x;
+#pragma unroll
+    for (int k = 2; k <= SEG; k <<= 1) {
+        // (descending runs are sorted as ascending runs of the complement)
+        const uint32_t flip = k < SEG && (tid & k) ? 0xFFFFFFFFu : 0u;
+        key ^= flip;
+#pragma unroll
+        for (int j = k >> 1; j > 0; j >>= 1) {
+            uint32_t other;
+            if (j >= 32) {
+                __syncthreads();
+                sh[tid] = key;
+                __syncthreads();
+                other = sh[tid ^ j];
+            } else {
+                other = __shfl_xor_sync(0xffffffffu, key, j);
+            }
+            key = (tid & j) ? max(key, other) : min(key, other);
+        }
+        key ^= flip;
+    }
+    return key;
+}
+
+__global__ void __launch_bounds__(kClumpRows) clump_kernel(const float4* __restrict__ sorted, uint64_t n,
+                                                           float4* __restrict__ pts, float* __restrict__ boxes) {
+    __shared__ uint32_t sh[kClumpRows];
+    __shared__ int sc[3][kClumpRows];
+    __shared__ uint32_t sid[kClumpRows];
+    __shared__ int wbox[32][6];
+    const int tid = threadIdx.x, lane = tid & 31, wid = tid >> 5;
+    const uint64_t base = (uint64_t)blockIdx.x * kClumpRows;
+    const int rows = (int)min((uint64_t)kClumpRows, n - base);
+    if (tid < rows) {
+        const float4 q = __ldg(&sorted[base + tid]);
+        sc[0][tid] = __float2int_rz(q.x);
+        sc[1][tid] = __float2int_rz(q.y);
+        sc[2][tid] = __float2int_rz(q.z);
+        sid[tid] = __float_as_uint(q.w);
+    }
+    __syncthreads();
+    uint32_t idx = (uint32_t)tid;  // the row in this thread's place
+    // box of the warp's rows
+    auto warp_box = [&](int (&v)[6]) {
+        const bool in = idx < (uint32_t)rows;
+#pragma unroll
+        for (int d = 0; d < 3; ++d) {
+            v[d] = __reduce_min_sync(0xffffffffu, in ? sc[d][idx] : INT32_MAX);
+            v[3 + d] = __reduce_max_sync(0xffffffffu, in ? sc[d][idx] : INT32_MIN);
+        }
+    };
+#pragma unroll 1
+    for (int seg = kClumpRows; seg > 32; seg >>= 1) {
+        int v[6];
+        warp_box(v);
+        if (lane == 0)
+#pragma unroll
+            for (int d = 0; d < 6; ++d) wbox[wid][d] = v[d];
+        __syncthreads();
+        const int sw = seg >> 5, w0 = wid & ~(sw - 1);  // the segment's warps
+        int best = -1, axis = 0, lo = 0;
+#pragma unroll
+        for (int d = 0; d < 3; ++d) {
+            const int l = __reduce_min_sync(0xffffffffu, wbox[w0 + (lane & (sw - 1))][d]);
+            const int h = __reduce_max_sync(0xffffffffu, wbox[w0 + (lane & (sw - 1))][3 + d]);
+            const int e = h >= l ? h - l : 0;
+            if (e > best) {
+                best = e;
+                axis = d;
+                lo = l;
+            }
+        }
+        const int s = max(0, 32 - __clz(max(best, 1)) - 21);  // (extent >> s) < 2^21
+        uint32_t key = 0x80000000u | idx;  // threads past the rows sort last
+        if (idx < (uint32_t)rows) key = (uint32_t)(sc[axis][idx] - lo) >> s << 10 | idx;
+        switch (seg) {
+            case 1024: key = sort_segment<1024>(key, sh); break;
+            case 512: key = sort_segment<512>(key, sh); break;
+            case 256: key = sort_segment<256>(key, sh); break;
+            case 128: key = sort_segment<128>(key, sh); break;
+            default: key = sort_segment<64>(key, sh); break;
+        }
+        idx = key & (kClumpRows - 1u);
+        __syncthreads();
+    }
+    // (rows past the end keep the last places of the last block)
+    if (base + tid < n)
+        pts[base + tid] = make_float4((float)sc[0][idx], (float)sc[1][idx], (float)sc[2][idx],
+                                      __uint_as_float(sid[idx]));
+    const ClumpTree tr(n);
+    int v[6];
+    warp_box(v);
+    const uint64_t clump = (base >> 5) + wid;
+    if (lane < 6 && clump < tr.count[0]) {
+        int r = v[0];
+#pragma unroll
+        for (int d = 1; d < 6; ++d)
+            if (lane == d) r = v[d];
+        boxes[tr.off[0] + (uint64_t)lane * tr.count[0] + clump] = (float)r;
+    }
+    if (lane == 0)
+#pragma unroll
+        for (int d = 0; d < 6; ++d) wbox[wid][d] = v[d];
+    __syncthreads();
+    if (wid < 6) {
+        const int x = wbox[lane][wid];
+        const int r = wid < 3 ? __reduce_min_sync(0xffffffffu, x) : __reduce_max_sync(0xffffffffu, x);
+        if (lane == 0) boxes[tr.off[1] + (uint64_t)wid * tr.count[1] + blockIdx.x] = (float)r;
+    }
+}
+
+// Boxes of a level's nodes from their 32 children's, one warp per node.
+__global__ void clump_parents_kernel(float* __restrict__ boxes, uint64_t n, int level) {
+    const ClumpTree tr(n);
+    uint32_t nc = 0, np = 0;
+    uint64_t oc = 0, op = 0;
+#pragma unroll
+    for (int l = 1; l < ClumpTree::kLevels; ++l)
+        if (l == level) {
+            nc = tr.count[l - 1];
+            oc = tr.off[l - 1];
+            np = tr.count[l];
+            op = tr.off[l];
+        }
+    const uint32_t node = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
+    const int lane = threadIdx.x & 31;
+    if (node >= np) return;
+    const uint32_t ch = node * 32u + lane;
+#pragma unroll
+    for (int d = 0; d < 6; ++d) {
+        const int none = d < 3 ? INT32_MAX : INT32_MIN;
+        const int x = ch < nc ? (int)boxes[oc + (uint64_t)d * nc + ch] : none;
+        const int r = d < 3 ? __reduce_min_sync(0xffffffffu, x) : __reduce_max_sync(0xffffffffu, x);
+        if (lane == 0) boxes[op + (uint64_t)d * np + node] = (float)r;
+    }
+}
+
+int ensure_clumps(Context* ctx, Tile* t, cudaStream_t stream) {
+    (void)ctx;
+    if (t->pts || !t->n) return NBG_OK;
+    if (!t->clumps || !t->grid_valid) return NBG_ERR_INVALID;
+    NBG_RANGE("nbg clump order");
+    float4* pts = (float4*)t->cursor;
+    float* boxes = (float*)t->keys;
+    const ClumpTree tr(t->n);
+    clump_kernel<<<(unsigned)((t->n + kClumpRows - 1) / kClumpRows), kClumpRows, 0, stream>>>(t->sorted, t->n, pts,
+                                                                                              boxes);
+    NBG_LAUNCHED(1);
+    for (int l = 2; l <= tr.top; ++l) {
+        clump_parents_kernel<<<(tr.count[l] + 3) / 4, 128, 0, stream>>>(boxes, t->n, l);
+        NBG_LAUNCHED(1);
+    }
+    if (cudaGetLastError() != cudaSuccess) return NBG_ERR_CUDA;
+    t->pts = pts;
+    t->boxes = boxes;
+    return NBG_OK;
+}
+
 static int grid_blocks(uint64_t n, int threads, int sms, int per_sm = 8) {
     uint64_t b = (n + threads - 1) / threads;
     uint64_t cap = (uint64_t)sms * per_sm;
@@ -215,6 +391,7 @@ size_t grid_temp_bytes(uint64_t items) {
 // Builds the grid of `t` on `stream`.  One host synchronisation reads the
 // table size T (sum of the column extents); the table grows when needed.
 int build_grid(Context* ctx, Tile* t, int k1, cudaStream_t stream) {
+    t->pts = nullptr;  // (their arrays are the build's)
     const uint64_t n = t->n;
     const int sms = ctx->sm_count;
     const int nb = grid_blocks(n, 256, sms);
@@ -226,7 +403,7 @@ int build_grid(Context* ctx, Tile* t, int k1, cudaStream_t stream) {
     grid_config_kernel<<<1, 1, 0, stream>>>(t->bbox, n, k1, t->cell_factor, t->cols_cap,
                                             t->fixed_cell, t->gp);
     const int cb = grid_blocks(t->cols_cap + 1, 256, sms);
-    col_init_kernel<<<cb, 256, 0, stream>>>((uint32_t)t->cols_cap, t->colinfo);
+    col_init_kernel<<<cb, 256, 0, stream>>>((uint32_t)t->cols_cap, t->colinfo, t->ext);
     col_zrange_kernel<<<nb, 256, 0, stream>>>(t->x, t->y, t->z, n, t->gp, t->colinfo);
     col_extent_kernel<<<cb, 256, 0, stream>>>(t->gp, t->colinfo, t->ext);
     size_t tmp = t->grid_tmp_bytes;
@@ -266,6 +443,7 @@ int build_grid(Context* ctx, Tile* t, int k1, cudaStream_t stream) {
 // its scan cover the whole table capacity.  A grid whose table would not fit
 // sets bit 2 of cap_hit; the caller rebuilds it with build_grid.
 int build_grid_async(Context* ctx, Tile* t, int k1, cudaStream_t stream) {
+    t->pts = nullptr;  // (their arrays are the build's)
     const uint64_t n = t->n;
     const int sms = ctx->sm_count;
     const int nb = grid_blocks(n, 256, sms);
@@ -278,7 +456,7 @@ int build_grid_async(Context* ctx, Tile* t, int k1, cudaStream_t stream) {
     grid_config_kernel<<<1, 1, 0, stream>>>(t->bbox, n, k1, t->cell_factor, t->cols_cap,
                                             t->fixed_cell, t->gp);
     const int cb = grid_blocks(t->cols_cap + 1, 256, sms);
-    col_init_kernel<<<cb, 256, 0, stream>>>((uint32_t)t->cols_cap, t->colinfo);
+    col_init_kernel<<<cb, 256, 0, stream>>>((uint32_t)t->cols_cap, t->colinfo, t->ext);
     col_zrange_kernel<<<nb, 256, 0, stream>>>(t->x, t->y, t->z, n, t->gp, t->colinfo);
     col_extent_kernel<<<cb, 256, 0, stream>>>(t->gp, t->colinfo, t->ext);
     size_t tmp = t->grid_tmp_bytes;

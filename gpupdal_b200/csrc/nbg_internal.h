@@ -113,6 +113,12 @@ struct Tile {
     uint32_t* ext = nullptr;     // cols_cap + 1: column extents, then bases
     uint32_t* table_dev = nullptr;
     uint32_t* keys = nullptr;    // n: table entry of each point
+    // the group select's clump order, built when that select first wants it, in
+    // the arrays the grid's build is done with (16 bytes a point of `cursor`,
+    // the box tree in `keys`)
+    bool clumps = false;         // may be built (false: fixed storage)
+    float4* pts = nullptr;       // n: points in clump order; null: not built for this grid
+    float* boxes = nullptr;      // boxes of the clumps and their parents (ClumpTree)
     uint32_t* cstart = nullptr;  // table_cap: first point of each entry
     uint32_t* cursor = nullptr;  // table_cap: scatter cursor
     float4* sorted = nullptr;    // n
@@ -124,11 +130,11 @@ struct Tile {
     bool fixed_storage = false;  // storage provided by the caller: never grow
     float cell_factor = 4.0f;
     int32_t fixed_cell = 0;
-    // select kernel: 0 the two-pass per-thread ring search (default), 1 the
-    // same in block-local Morton order, 2 the single-pass ring search, 8 / 16
-    // / 32 queries sharing one candidate list; the group select's first box
-    // margin in cell edges
-    int group = 0;
+    // select kernel: -1 the library's choice (select_kernel), 0 the two-pass
+    // per-thread ring search, 1 the same in block-local Morton order, 2 the
+    // single-pass ring search, 8 / 16 / 32 a warp's queries sharing one
+    // candidate list; the group select's first margin (nbg_tile_set_select)
+    int group = -1;
     float margin0 = 0.5f;
     // the caller chose the cell factor or select kernel (nbg_tile_tune,
     // nbg_tile_set_select, nbg_tile_autotune): the context's cached tuning of
@@ -189,8 +195,9 @@ int launch_query(Context* ctx, const QueryLaunch& q, cudaStream_t stream);
 // point id lies in [bounds[c], bounds[c+1]), for c < nchunks (bounds[nchunks]
 // = n); `dnum` is one device word the selection writes its count to.
 // Returns after the selection completed.
+// (With `clumps` slots of the clump order instead.)
 int build_id_chunks(Context* ctx, const Tile* t, const uint64_t* bounds, int nchunks,
-                    uint32_t* rows, uint32_t* dnum, cudaStream_t st);
+                    uint32_t* rows, uint32_t* dnum, bool clumps, cudaStream_t st);
 // Select pass over a sample of `blocks` blocks of 128 rows, in runs of `run`
 // consecutive blocks whose starts are `stride` rows apart.
 int launch_select_sample(Context* ctx, const QueryLaunch& q, uint64_t stride, unsigned blocks,
@@ -215,6 +222,11 @@ int launch_ties(Context* ctx, const TieLaunch& tl, cudaStream_t stream);
 // (tl.nties: the list's capacity), so the launch can be queued before the
 // query that fills the list has finished.
 int launch_ties_counted(Context* ctx, const TieLaunch& tl, const uint32_t* count, cudaStream_t stream);
+// The select kernel a launch over `t` with K neighbours takes: the tile's own
+// setting, else the library's choice.
+int select_kernel(const Tile* t, int K);
+// The clump order of the tile's current grid (group select).
+int ensure_clumps(Context* ctx, Tile* t, cudaStream_t stream);
 // True when launch_query answers `q`'s handed-back rows on the context's fork
 // stream (the single-pass select): work queued there after the launch runs
 // once the tie list is complete, beside the finish pass.
@@ -268,7 +280,7 @@ int kd_export(Context* ctx, Tile* t, uint32_t* vind, uint32_t* nnodes, int32_t* 
 // neighbour-set export of the grid path
 int launch_neighbor_sets(Context* ctx, const Tile* t, int K, int rmax, uint32_t* ids_out,
                          uint32_t* exact_rows, uint32_t* counters, uint2* ties, uint32_t tie_cap,
-                         cudaStream_t stream, uint32_t* retry_rows = nullptr);
+                         cudaStream_t stream, uint32_t* retry_rows, int group);
 
 // A tile the caller did not tune (cell factor, select kernel) takes the
 // context's cached autotuner choice for its (size, neighbour slots) class.

@@ -146,7 +146,7 @@ __global__ void __launch_bounds__(128) knn_fused_kernel(const QueryArgs a) {
     const uint64_t i = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x;
     if (i >= a.n) return;
     const GridParams g = *a.gp;
-    const float4 q = __ldg(&a.gv.sorted[i]);
+    const float4 q = __ldg(&a.qpts[i]);
     const uint32_t id = __float_as_uint(q.w);
     const int K = a.K;
     QueryCell qc;
@@ -187,7 +187,7 @@ __global__ void __launch_bounds__(128) knn_fused_kernel(const QueryArgs a) {
 template <int KS>
 __device__ __forceinline__ void select_row(const QueryArgs& a, const uint64_t i) {
     const GridParams g = *a.gp;
-    const float4 q = __ldg(&a.gv.sorted[i]);
+    const float4 q = __ldg(&a.qpts[i]);
     const uint32_t id = __float_as_uint(q.w);
     const int K = row_neighbours(a.row_k, a.K, a.n, id);
     if (K <= 0) {
@@ -342,7 +342,7 @@ __device__ __forceinline__ void loc_shell(const GridView& gv, const GridParams& 
 template <int KS>
 __device__ __forceinline__ void select_row_loc(const QueryArgs& a, const uint64_t i, uint32_t ob) {
     const GridParams g = *a.gp;
-    const float4 q = __ldg(&a.gv.sorted[i]);
+    const float4 q = __ldg(&a.qpts[i]);
     const uint32_t id = __float_as_uint(q.w);
     const int K = row_neighbours(a.row_k, a.K, a.n, id);
     auto retry = [&]() {
@@ -473,7 +473,7 @@ __device__ __forceinline__ void finish_row(const QueryArgs& a, const uint64_t i)
     const RowSums r = a.sums[i];
     if (r.cnt == 0) return;
     const GridParams* gp = a.gp;
-    const float4 q = __ldg(&a.gv.sorted[i]);
+    const float4 q = __ldg(&a.qpts[i]);
     const uint32_t id = __float_as_uint(q.w);
     const long long n = r.cnt;
     long long M[6];
@@ -590,7 +590,7 @@ struct QueueLauncher {
 template <int KS>
 __device__ __forceinline__ void ids_row(const QueryArgs& a, const uint64_t i) {
     const GridParams g = *a.gp;
-    const float4 q = __ldg(&a.gv.sorted[i]);
+    const float4 q = __ldg(&a.qpts[i]);
     const uint32_t id = __float_as_uint(q.w);
     const int K = a.K;
     QueryCell qc;
@@ -628,15 +628,13 @@ __global__ void __launch_bounds__(128) knn_ids_kernel(const QueryArgs a) {
     if (i < a.n) ids_row<KS>(a, i);
 }
 
-// Rows the group select handed back (a.rows, a.nq_dev entries), answered by
-// the per-thread ring search: neighbour sums, or the neighbour-set export.
+// Neighbour-set export: rows the group select handed back (a.rows, a.nq_dev
+// entries), answered by the per-thread ring search.
 template <int KS>
 __global__ void __launch_bounds__(128) knn_retry_kernel(const QueryArgs a) {
     const uint32_t nr = *a.nq_dev;
     for (uint32_t r = blockIdx.x * blockDim.x + threadIdx.x; r < nr; r += gridDim.x * blockDim.x) {
-        const uint32_t i = __ldg(&a.rows[r]);
-        if (a.ids_out) ids_row<KS>(a, i);
-        else select_row<KS>(a, i);
+        ids_row<KS>(a, __ldg(&a.rows[r]));
     }
 }
 
@@ -859,7 +857,7 @@ __global__ void __launch_bounds__(128) knn_stride_kernel(const StrideArgs sa) {
     const uint64_t i = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x;
     if (i >= a.n) return;
     const GridParams g = *a.gp;
-    const float4 q = __ldg(&a.gv.sorted[i]);
+    const float4 q = __ldg(&a.qpts[i]);
     const uint32_t rid = __float_as_uint(q.w);
     const int K = a.K;
     QueryCell qc;
@@ -1145,8 +1143,7 @@ struct LaunchArgs {
     uint32_t ob = 11;     // single-pass select: offset bits of a key
 };
 
-int launch_group_select(const QueryArgs& q, int slots, int group, float margin0,
-                        cudaStream_t stream);
+int launch_group_select(const QueryArgs& q, int slots, float margin0, cudaStream_t stream);
 
 // Handed-back rows are the sparse-region and hard rows: long ring searches
 // that need many resident warps to hide their latency.  The row count is read
@@ -1162,12 +1159,19 @@ struct KnnLauncher {
         const uint64_t rows = la.q.rows ? la.q.nq : la.q.n;
         const uint64_t blocks = (rows + threads - 1) / threads;
         if (blocks == 0) return NBG_OK;
-        if (la.group == 2 && la.q.sums && !la.ids) {
-            // single pass with located keys; rows it hands back through the
-            // two-pass kernel (count read on the device); then the finish pass
+        if ((la.group == 2 || la.group >= 8) && la.q.sums && !la.ids) {
+            // shared candidate lists, or single pass with located keys; rows
+            // either hands back go to warps of their own (count read on the
+            // device), beside the finish pass
             if (cudaMemsetAsync(la.q.counters + 6, 0, sizeof(uint32_t), la.stream))
                 return NBG_ERR_CUDA;
-            knn_select_loc_kernel<KS><<<(unsigned)blocks, threads, 0, la.stream>>>(la.q, la.ob);
+            if (la.group >= 8) {
+                const int rc = launch_group_select(la.q, KS, la.margin0, la.stream);
+                if (rc) return rc;
+            } else {
+                knn_select_loc_kernel<KS><<<(unsigned)blocks, threads, 0, la.stream>>>(la.q, la.ob);
+                NBG_LAUNCHED(1);
+            }
             QueryArgs r = la.q;
             r.rows = la.q.retry_rows;
             r.nq_dev = la.q.counters + 6;
@@ -1176,7 +1180,7 @@ struct KnnLauncher {
                 const int rc = launch_retry_finish(r, KS, la.sms, la.stream);
                 if (rc) return rc;
                 knn_finish_kernel<<<(unsigned)blocks, threads, 0, la.stream>>>(la.q);
-                NBG_LAUNCHED(2);
+                NBG_LAUNCHED(1);
                 return cudaGetLastError() == cudaSuccess ? NBG_OK : NBG_ERR_CUDA;
             }
             // the handed-back rows on the fork stream, queued first so their
@@ -1188,7 +1192,7 @@ struct KnnLauncher {
             const int rc = launch_retry_finish(r, KS, la.sms, la.fork);
             if (rc) return rc;
             knn_finish_kernel<<<(unsigned)blocks, threads, 0, la.stream>>>(la.q);
-            NBG_LAUNCHED(2);
+            NBG_LAUNCHED(1);
             if (la.done) {
                 // join on the fork stream: `stream` may go on to the next launch
                 e = cudaEventRecord(la.fev[2], la.stream);
@@ -1209,12 +1213,12 @@ struct KnnLauncher {
             NBG_LAUNCHED(2);
             return cudaGetLastError() == cudaSuccess ? NBG_OK : NBG_ERR_CUDA;
         }
-        if (la.group >= 8 && (la.ids || la.q.sums)) {
+        if (la.group >= 8 && la.ids) {
             // group select, then the rows it handed back through the per-thread
-            // select (count read on the device), then the finish pass
+            // select (count read on the device)
             if (cudaMemsetAsync(la.q.counters + 6, 0, sizeof(uint32_t), la.stream))
                 return NBG_ERR_CUDA;
-            int rc = launch_group_select(la.q, KS, la.group, la.margin0, la.stream);
+            const int rc = launch_group_select(la.q, KS, la.margin0, la.stream);
             if (rc) return rc;
             QueryArgs r = la.q;
             r.rows = la.q.retry_rows;
@@ -1222,11 +1226,6 @@ struct KnnLauncher {
             knn_retry_kernel<KS><<<(unsigned)std::min<uint64_t>(blocks, (uint64_t)la.sms * kRetryBlocksPerSm), threads,
                                    0, la.stream>>>(r);
             NBG_LAUNCHED(1);
-            if (!la.ids) {
-                if (la.fork && cudaEventRecord(la.fev[0], la.stream)) return NBG_ERR_CUDA;
-                knn_finish_kernel<<<(unsigned)blocks, threads, 0, la.stream>>>(la.q);
-                NBG_LAUNCHED(1);
-            }
             return cudaGetLastError() == cudaSuccess ? NBG_OK : NBG_ERR_CUDA;
         }
         if (la.ids) {
@@ -1282,6 +1281,8 @@ int launch_query(Context* ctx, const QueryLaunch& ql, cudaStream_t stream) {
     la.done = ql.done;
     la.ids = false;
     la.group = ql.retry_rows ? ql.group : 0;
+    la.q.qpts = la.group >= 8 ? ql.tile->pts : ql.tile->sorted;
+    la.q.boxes = ql.tile->boxes;
     la.margin0 = ql.margin0;
     la.sms = ctx ? ctx->sm_count : 148;
     la.ob = loc_offset_bits(ql.tile->host_gp.cell);
@@ -1294,14 +1295,16 @@ int launch_query(Context* ctx, const QueryLaunch& ql, cudaStream_t stream) {
 
 bool query_forks(const Context* ctx, const QueryLaunch& ql) {
     const uint64_t rows = ql.rows ? ql.nrows : ql.tile->n;
-    return ctx && ctx->fork && ql.retry_rows && ql.group == 2 && ql.sums && rows > 0;
+    return ctx && ctx->fork && ql.retry_rows && (ql.group == 2 || ql.group >= 8) && ql.sums && rows > 0;
 }
 
 int launch_neighbor_sets(Context* ctx, const Tile* t, int K, int rmax, uint32_t* ids_out,
                          uint32_t* exact_rows, uint32_t* counters, uint2* ties, uint32_t tie_cap,
-                         cudaStream_t stream, uint32_t* retry_rows) {
+                         cudaStream_t stream, uint32_t* retry_rows, int group) {
     LaunchArgs la{};
-    la.group = retry_rows ? t->group : 0;
+    la.group = retry_rows ? group : 0;
+    la.q.qpts = la.group >= 8 ? t->pts : t->sorted;
+    la.q.boxes = t->boxes;
     la.margin0 = t->margin0;
     la.sms = ctx ? ctx->sm_count : 148;
     la.q.retry_rows = retry_rows;
@@ -1336,19 +1339,20 @@ struct InIdRange {
 };
 
 int build_id_chunks(Context* ctx, const Tile* t, const uint64_t* bounds, int nchunks,
-                    uint32_t* rows, uint32_t* dnum, cudaStream_t st) {
+                    uint32_t* rows, uint32_t* dnum, bool clumps, cudaStream_t st) {
     const uint64_t n = t->n;
+    const float4* pts = clumps ? t->pts : t->sorted;
     cub::CountingInputIterator<uint32_t> first(0);
     size_t tmp_bytes = 0;
     cudaError_t e = cub::DeviceSelect::If(nullptr, tmp_bytes, first, rows, dnum, (int64_t)n,
-                                          InIdRange{t->sorted, 0, 0}, st);
+                                          InIdRange{pts, 0, 0}, st);
     if (e) return fail(ctx, NBG_ERR_CUDA, std::string("row chunks: ") + cudaGetErrorString(e));
     void* tmp = nullptr;
     int rc = ctx_alloc(ctx, &tmp, std::max<size_t>(tmp_bytes, 16));
     if (rc) return rc;
     for (int c = 0; c < nchunks && !e; ++c) {
         e = cub::DeviceSelect::If(tmp, tmp_bytes, first, rows + bounds[c], dnum, (int64_t)n,
-                                  InIdRange{t->sorted, (uint32_t)bounds[c], (uint32_t)bounds[c + 1]},
+                                  InIdRange{pts, (uint32_t)bounds[c], (uint32_t)bounds[c + 1]},
                                   st);
         NBG_LAUNCHED(1);
     }
@@ -1382,6 +1386,7 @@ int launch_select_sample(Context* ctx, const QueryLaunch& ql, uint64_t stride, u
     (void)ctx;
     SampleArgs s{};
     s.q.gv = grid_view(ql.tile);
+    s.q.qpts = ql.tile->sorted;
     s.q.gp = ql.tile->gp;
     s.q.n = ql.tile->n;
     s.q.K = ql.K;
@@ -1447,6 +1452,7 @@ int launch_stride(Context* ctx, const QueryLaunch& ql, int stride, int kpick, co
     }
     QueryArgs& q = l.s.q;
     q.gv = grid_view(ql.tile);
+    q.qpts = ql.tile->sorted;
     q.gp = ql.tile->gp;
     q.n = ql.tile->n;
     q.K = ql.K;

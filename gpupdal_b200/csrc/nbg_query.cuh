@@ -142,16 +142,6 @@ __device__ __forceinline__ void defer_row(const QueryArgs& a, uint32_t id, bool 
     a.exact_rows[slot] = id;
 }
 
-// 10-bit Morton interleave of three coordinates.
-__device__ __forceinline__ uint32_t spread3(uint32_t v) {
-    v &= 0x3FFu;
-    v = (v | (v << 16)) & 0x030000FFu;
-    v = (v | (v << 8)) & 0x0300F00Fu;
-    v = (v | (v << 4)) & 0x030C30C3u;
-    v = (v | (v << 2)) & 0x09249249u;
-    return v;
-}
-
 // Sort keys of a block's rows r0 .. r0 + nvalid - 1 (threads past nvalid get
 // a key above every row's): a Morton key of the row's coordinates relative to
 // the block's bounding box, at the resolution that fits the box in 10 bits

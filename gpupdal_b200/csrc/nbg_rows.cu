@@ -283,7 +283,7 @@ __global__ void __launch_bounds__(kRowThreads) knn_retry_finish_kernel(const Que
         float4 mq = make_float4(0.f, 0.f, 0.f, 0.f);  // this lane's row
         int mk = -1;                                   // its neighbours (-1: nothing to finish)
         int ms[9] = {0, 0, 0, 0, 0, 0, 0, 0, 0};
-        if ((uint32_t)lane < m) mq = __ldg(&a.gv.sorted[__ldg(&a.rows[r0 + lane])]);
+        if ((uint32_t)lane < m) mq = __ldg(&a.qpts[__ldg(&a.rows[r0 + lane])]);
         for (uint32_t j = 0; j < m; ++j) {
             const float4 q = make_float4(__shfl_sync(kAll, mq.x, j), __shfl_sync(kAll, mq.y, j),
                                          __shfl_sync(kAll, mq.z, j), __shfl_sync(kAll, mq.w, j));

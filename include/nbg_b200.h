@@ -237,14 +237,16 @@ int nbg_tile_free(nbg_context* ctx, nbg_tile* tile);
  * reference (whose KD tree has no tunable). */
 int nbg_tile_tune(nbg_context* ctx, nbg_tile* tile, float cell_factor, int32_t fixed_cell);
 /* Select kernel of a tile (the k-nearest search of nbg_run; results are
- * identical for every setting):
- *   0  two-pass ring search, one query per thread (default)
+ * identical for every setting; a tile left alone takes the library's choice,
+ * 32 for long lists and 0 otherwise):
+ *   0  two-pass ring search, one query per thread
  *   1  the same with the queries of each 256-row block in Morton order
  *   2  single-pass ring search: top-list keys carry the candidate's column and
  *      position, so the K nearest are read back without a second scan
- *   8, 16, 32  that many neighbouring queries (Morton-compact) share one
- *      candidate list, gathered box ring by box ring from a first margin of
- *      first_margin cell edges
+ *   8, 16, 32  a warp's 32 neighbouring queries share one candidate list,
+ *      gathered from a tree of boxes over compact 32-point clumps; the first
+ *      margin is at most 8 first_margin times the radius that holds K points at
+ *      the tile's planar density
  * Rows the faster forms cannot answer exactly go to the two-pass search.
  * Used by the autotuner; no counterpart in the reference. */
 int nbg_tile_set_select(nbg_context* ctx, nbg_tile* tile, int32_t select_kernel,
