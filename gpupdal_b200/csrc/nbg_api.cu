@@ -1175,7 +1175,7 @@ extern "C" int nbg_run(nbg_context* h, nbg_tile* th, const nbg_stage_opts* stage
             }
             continue;
         }
-        const int select = select_kernel(t, K);
+        const int select = select_kernel(t, K, pipelined);
         if (!radius_group && select >= 8) {
             rc = ensure_clumps(ctx, t, stream);
             if (rc) { cleanup(); return fail(ctx, rc, "clump order"); }
@@ -1417,15 +1417,24 @@ static std::pair<int, int> tuning_class(const Tile* t, int K) {
     return std::make_pair(lg, slots_for_k(K));
 }
 
-// The library's choice for a tile nobody tuned.  Long lists go to the group
-// select: an insertion into a sorted list of K + 1 registers costs 2 (K + 1)
-// min/max whenever any lane inserts, the group select's batch merge a tenth of
-// that (1.5M points, knn = 64: select 11.9 ms per thread, 5.5 ms grouped; at
-// knn = 32 the two are even, 1.0 and 1.1 ms on 300k points, and below it the
-// per-thread search reads fewer candidates).
-int select_kernel(const Tile* t, int K) {
+// The library's choice for a tile nobody tuned.  Whole calls on fresh tiles, ms,
+// per-thread two-pass (0) / single pass (2) / group (32):
+//   K = 9    2M mixture 3.02 / 2.41 / 2.90     16M stress 25.2 / 19.3 / 25.6
+//   K = 17   2M mixture 3.55 / 3.39 / 3.04     32M stress 56.0 / 50.4 / 53.3
+//   K = 25   2M mixture 4.73 / 5.25 / 3.69     2M stress  5.58 / 5.18 / 4.46
+//   K = 33   2M mixture 6.76 / 15.6 / 4.50     300k terrain 1.47 / 3.5 / 0.93
+// The single pass pays one min/max per list slot and candidate and wins while the
+// list is short (from 16M points also at 18 slots: the replica built beside it
+// gets more of the SMs than beside the group select's shared memory), as long as
+// its keys hold a column; the group select sorts batches and wins above.  A chunk
+// holds a fraction of each clump, so the group select's bounds are loose there
+// (6M stress records, K = 17: 18.8 ms against 17.4 with the two-pass search).
+int select_kernel(const Tile* t, int K, bool chunks) {
     if (t->group >= 0) return t->group;
-    return t->clumps && slots_for_k(K) >= 50 ? 32 : 0;
+    if (!t->clumps) return 0;
+    const int slots = slots_for_k(K);
+    if ((slots <= 14 || (slots <= 18 && (chunks || t->n >= 16000000))) && located_keys_fit(t)) return 2;
+    return chunks && slots < 50 ? 0 : 32;
 }
 
 // A tile the caller did not tune takes the context's cached choice for its
@@ -1649,7 +1658,7 @@ extern "C" int nbg_neighbor_sets(nbg_context* h, nbg_tile* th, int32_t knn, uint
         if (rc) return rc;
     }
     cudaMemsetAsync(ctx->counters, 0, 64 * sizeof(uint32_t), stream);
-    const int select = select_kernel(t, K);
+    const int select = select_kernel(t, K, false);
     if (select >= 8) rc = ensure_clumps(ctx, t, stream);
     if (!rc)
         rc = launch_neighbor_sets(ctx, t, K, 8, dev_ids, ctx->exact_rows, ctx->counters, ctx->ties,

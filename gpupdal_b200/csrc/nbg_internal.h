@@ -222,9 +222,11 @@ int launch_ties(Context* ctx, const TieLaunch& tl, cudaStream_t stream);
 // (tl.nties: the list's capacity), so the launch can be queued before the
 // query that fills the list has finished.
 int launch_ties_counted(Context* ctx, const TieLaunch& tl, const uint32_t* count, cudaStream_t stream);
-// The select kernel a launch over `t` with K neighbours takes: the tile's own
-// setting, else the library's choice.
-int select_kernel(const Tile* t, int K);
+// The select kernel a launch over `t` (its grid built) with K neighbours takes:
+// the tile's own setting, else the library's choice.  `chunks`: the launches
+// answer the rows of id-range chunks.
+int select_kernel(const Tile* t, int K, bool chunks);
+bool located_keys_fit(const Tile* t);
 // The clump order of the tile's current grid (group select).
 int ensure_clumps(Context* ctx, Tile* t, cudaStream_t stream);
 // True when launch_query answers `q`'s handed-back rows on the context's fork

@@ -1130,6 +1130,15 @@ static uint32_t loc_offset_bits(int32_t c) {
     return (uint32_t)std::min(16, std::max(6, 27 - bits));
 }
 
+// The single-pass select's offset field holds a column of four times the
+// tile's mean population: fuller columns are rare then, and their rows few
+// enough to hand back.
+bool located_keys_fit(const Tile* t) {
+    const GridParams& g = t->host_gp;
+    const double mean = (double)t->n / ((double)g.gx * (double)g.gy);
+    return (double)(1u << loc_offset_bits(g.cell)) >= 4.0 * mean;
+}
+
 struct LaunchArgs {
     QueryArgs q;
     cudaStream_t stream;

@@ -237,8 +237,8 @@ int nbg_tile_free(nbg_context* ctx, nbg_tile* tile);
  * reference (whose KD tree has no tunable). */
 int nbg_tile_tune(nbg_context* ctx, nbg_tile* tile, float cell_factor, int32_t fixed_cell);
 /* Select kernel of a tile (the k-nearest search of nbg_run; results are
- * identical for every setting; a tile left alone takes the library's choice,
- * 32 for long lists and 0 otherwise):
+ * identical for every setting; a tile left alone takes the library's choice of
+ * 0, 2 and 32 by neighbour count and size):
  *   0  two-pass ring search, one query per thread
  *   1  the same with the queries of each 256-row block in Morton order
  *   2  single-pass ring search: top-list keys carry the candidate's column and
