@@ -38,12 +38,14 @@
 namespace nbg {
 
 static constexpr int KD_LEAF = 100;
-// Level passes: tiles of KD_TILE elements, KD_THREADS threads; each warp takes
-// KD_ROWS rows of 32 consecutive elements.  A tile this long keeps the tile
-// list of a 32M-point tree at 8k entries, which one block can scan.
-static constexpr int KD_TILE = 4096;
+// Level passes: tiles of KD_THREADS * ROWS elements, each warp taking ROWS rows
+// of 32 consecutive elements.  Long tiles keep the tile list of a 32M-point tree
+// at 8k entries, which one block can scan; up to KD_SHORT_MAX points a tile of
+// that length would leave most SMs without one (245 tiles at 1M points: 13.7 us
+// a classify pass), so the tiles are a quarter as long.
 static constexpr int KD_THREADS = 256;
-static constexpr int KD_ROWS = KD_TILE / KD_THREADS;
+static constexpr int KD_ROWS_LONG = 16, KD_ROWS_SHORT = 4;
+static constexpr uint64_t KD_SHORT_MAX = 2500000;
 // Segments of at most this many points are finished, subtree and all, in the
 // shared memory of one block (kd_block_build_kernel).
 static constexpr uint32_t KD_BLOCK_MAX = 4096;
@@ -157,6 +159,7 @@ struct KdForest {
     uint32_t* tile_seg = nullptr;
     unsigned long long* tile_cnt = nullptr;  // per tile counts (below | at << 32), then prefix
     uint32_t tile_cap = 0;
+    uint32_t tile = 0;  // elements a tile
     KdState* state = nullptr;
     uint32_t* counters = nullptr;  // [2] errors of the search replay
     uint64_t* bases = nullptr;     // device, first position per tree
@@ -210,7 +213,7 @@ __device__ __forceinline__ void kd_choose_cut(const double lo[3], const double h
             }
         }
     }
-    double split_val = __ddiv_rn(__dadd_rn(lo[cutfeat], hi[cutfeat]), 2.0);
+    double split_val = __dmul_rn(__dadd_rn(lo[cutfeat], hi[cutfeat]), 0.5);  // (halving is exact either way)
     double mn = ref_coord(mn_[cutfeat], tf.scale[cutfeat], tf.offset[cutfeat]);
     double mx = ref_coord(mx_[cutfeat], tf.scale[cutfeat], tf.offset[cutfeat]);
     if (split_val < mn) cutval = mn;
@@ -252,6 +255,26 @@ __device__ __forceinline__ void kd_thresholds(double cut, double sc, double of, 
     }
     t1 = bound[0];
     t2 = bound[1];
+}
+
+// The same by a whole warp: its lanes try 32 raw values around the estimate
+// (inv = 1 / sc) at once.
+__device__ __forceinline__ void kd_warp_thresholds(double cut, double sc, double inv, double of, int32_t mn,
+                                                   int32_t mx, uint32_t& t1, uint32_t& t2) {
+    const uint32_t range = (uint32_t)((long long)mx - mn) + 1u;
+    const double est = (cut - of) * inv - (double)mn - 15.0;
+    const uint32_t base = est <= 0.0 ? 0u : est >= (double)range ? range - 1u : (uint32_t)est;
+    const uint32_t u = base + (threadIdx.x & 31u);
+    const double v = ref_coord((int32_t)((long long)mn + min(u, range - 1u)), sc, of);
+    const unsigned in = __ballot_sync(0xffffffffu, u < range);
+    const unsigned below = __ballot_sync(0xffffffffu, u < range && v < cut);
+    const unsigned upto = __ballot_sync(0xffffffffu, u < range && v <= cut);
+    if ((base && !(below & 1u)) || (upto == in && base + __popc(in) < range)) {
+        kd_thresholds(cut, sc, of, mn, mx, t1, t2);  // beyond the lanes' reach
+        return;
+    }
+    t1 = base + __popc(below);
+    t2 = base + __popc(upto);
 }
 
 // Hoare's pass swaps the t-th element from the left that fails the predicate
@@ -303,6 +326,7 @@ struct KdLevel {
     const Transform* tfs;
     KdNodes N;
     uint32_t seg_cap, small_cap, tile_cap;
+    uint32_t tile;  // elements a tile
 };
 
 // True in every thread of the block that finishes a pass last; what the other
@@ -348,14 +372,15 @@ __device__ __forceinline__ void kd_block_prefix(unsigned long long* v, uint32_t 
 }
 
 // Rows of a tile: warp w's element of row k.
+template <int ROWS>
 __device__ __forceinline__ uint32_t kd_row(uint32_t begin, uint32_t tile, int k) {
-    return begin + tile * KD_TILE + ((threadIdx.x >> 5) * KD_ROWS + k) * 32 + (threadIdx.x & 31u);
+    return begin + tile * (KD_THREADS * ROWS) + ((threadIdx.x >> 5) * ROWS + k) * 32 + (threadIdx.x & 31u);
 }
 
 // Per tile, pass 1: points below the cut in the low 32 bits, at it in the high
 // ones; pass 2: points at the cut at or after position L (segments that have
 // any).  The last block turns the counts into their prefix.
-template <int PASS>
+template <int PASS, int ROWS>
 __global__ void __launch_bounds__(KD_THREADS) kd_count_kernel(const KdLevel lv) {
     __shared__ unsigned long long red[KD_THREADS / 32];
     const uint32_t ntiles = lv.st->tiles;
@@ -370,14 +395,14 @@ __global__ void __launch_bounds__(KD_THREADS) kd_count_kernel(const KdLevel lv) 
         const int32_t* rc = f == 0 ? lv.rx : (f == 1 ? lv.ry : lv.rz);
         uint32_t nlt = 0, neq = 0;
         if (PASS == 1 || sp->eq) {
-            int32_t v[KD_ROWS];
+            int32_t v[ROWS];
 #pragma unroll
-            for (int k = 0; k < KD_ROWS; ++k) {
-                const uint32_t i = kd_row(b, t - sp->first, k);
+            for (int k = 0; k < ROWS; ++k) {
+                const uint32_t i = kd_row<ROWS>(b, t - sp->first, k);
                 v[k] = i >= from && i < e ? rc[i] - org : -1;
             }
 #pragma unroll
-            for (int k = 0; k < KD_ROWS; ++k) {
+            for (int k = 0; k < ROWS; ++k) {
                 const uint32_t x = (uint32_t)v[k];  // (outside the range: above every bound)
                 if (PASS == 1) nlt += x < t1;
                 neq += x >= t1 && x < t2;
@@ -420,7 +445,7 @@ __global__ void __launch_bounds__(KD_THREADS) kd_count_kernel(const KdLevel lv) 
 // The positions of the misplaced elements (mlpos, mrpos: see kd_split_index's
 // note); pass 1 also takes the extents of the points below, at and above the
 // cut, the children's boxes.
-template <int PASS>
+template <int PASS, int ROWS>
 __global__ void __launch_bounds__(KD_THREADS) kd_classify_kernel(const KdLevel lv) {
     __shared__ uint32_t s_cnt[KD_THREADS / 32];
     __shared__ int32_t s_ext[18];
@@ -440,7 +465,7 @@ __global__ void __launch_bounds__(KD_THREADS) kd_classify_kernel(const KdLevel l
         const uint32_t t1 = sp->t1, t2 = sp->t2;
         const int dims = sp->dims;
         const int32_t* rc = f == 0 ? lv.rx : (f == 1 ? lv.ry : lv.rz);
-        unsigned bal[KD_ROWS];
+        unsigned bal[ROWS];
         uint32_t n = 0;
         if (PASS == 1) {
             if (threadIdx.x < 18) s_ext[threadIdx.x] = threadIdx.x < 9 ? INT32_MAX : INT32_MIN;
@@ -454,8 +479,8 @@ __global__ void __launch_bounds__(KD_THREADS) kd_classify_kernel(const KdLevel l
                 }
             __syncthreads();
 #pragma unroll
-            for (int k = 0; k < KD_ROWS; ++k) {
-                const uint32_t i = kd_row(sb, t - sp->first, k);
+            for (int k = 0; k < ROWS; ++k) {
+                const uint32_t i = kd_row<ROWS>(sb, t - sp->first, k);
                 const bool in = i < e;
                 const int32_t c[3] = {in && dims & 1 ? lv.rx[i] : 0, in && dims & 2 ? lv.ry[i] : 0,
                                       in && dims & 4 ? lv.rz[i] : 0};
@@ -490,8 +515,8 @@ __global__ void __launch_bounds__(KD_THREADS) kd_classify_kernel(const KdLevel l
                 }
         } else {
 #pragma unroll
-            for (int k = 0; k < KD_ROWS; ++k) {
-                const uint32_t i = kd_row(sb, t - sp->first, k);
+            for (int k = 0; k < ROWS; ++k) {
+                const uint32_t i = kd_row<ROWS>(sb, t - sp->first, k);
                 const bool in = i >= b && i < e;
                 bal[k] = __ballot_sync(0xffffffffu, in && (uint32_t)(rc[in ? i : b] - org) < t2);
                 n += __popc(bal[k]);
@@ -503,8 +528,8 @@ __global__ void __launch_bounds__(KD_THREADS) kd_classify_kernel(const KdLevel l
         uint32_t before = PASS == 1 ? (uint32_t)pre : (uint32_t)(pre >> 32);
         for (int w = 0; w < warp; ++w) before += s_cnt[w];
 #pragma unroll
-        for (int k = 0; k < KD_ROWS; ++k) {
-            const uint32_t i = kd_row(sb, t - sp->first, k);
+        for (int k = 0; k < ROWS; ++k) {
+            const uint32_t i = kd_row<ROWS>(sb, t - sp->first, k);
             if (i >= b && i < e) {
                 const uint32_t prank = before + __popc(bal[k] & lt), li = i - b;
                 const bool p = bal[k] >> lane & 1u;
@@ -569,13 +594,13 @@ __device__ __forceinline__ void kd_plan_segment(const KdSeg& sg, const int32_t m
 
 // One block: the tile list of the S segments in segs / sp.
 __device__ __forceinline__ void kd_tile_map(const KdSeg* segs, KdSplit* sp, uint32_t S, uint32_t* tile_seg,
-                                            uint32_t tile_cap, KdState* st) {
+                                            uint32_t tile_cap, uint32_t tile, KdState* st) {
     typedef cub::BlockScan<uint32_t, KD_THREADS> Scan;
     __shared__ typename Scan::TempStorage tmp;
     uint32_t carry = 0;
     for (uint32_t base = 0; base < S; base += KD_THREADS) {
         const uint32_t s = base + threadIdx.x;
-        const uint32_t nt = s < S ? (segs[s].end - segs[s].begin + KD_TILE - 1) / KD_TILE : 0u;
+        const uint32_t nt = s < S ? (segs[s].end - segs[s].begin + tile - 1) / tile : 0u;
         uint32_t first, total;
         Scan(tmp).ExclusiveSum(nt, first, total);
         if (s < S) sp[s].first = carry + first;
@@ -621,8 +646,8 @@ __global__ void __launch_bounds__(KD_THREADS) kd_swap_kernel(const KdLevel lv) {
             const KdSplit* sp = &lv.sp[s];
             const uint32_t m = PASS == 1 ? sp->m : sp->m2;
             const uint32_t b = lv.segs[s].begin + (PASS == 1 ? 0u : sp->L);
-            const uint32_t end = min(m, (t - sp->first + 1) * KD_TILE);
-            for (uint32_t l0 = (t - sp->first) * KD_TILE + threadIdx.x; l0 < end; l0 += KD_THREADS * ITEMS) {
+            const uint32_t end = min(m, (t - sp->first + 1) * lv.tile);
+            for (uint32_t l0 = (t - sp->first) * lv.tile + threadIdx.x; l0 < end; l0 += KD_THREADS * ITEMS) {
                 uint32_t a[ITEMS], z[ITEMS], ai[ITEMS], zi[ITEMS];
                 int32_t ax[ITEMS], ay[ITEMS], az[ITEMS], zx[ITEMS], zy[ITEMS], zz[ITEMS];
 #pragma unroll
@@ -732,7 +757,7 @@ __global__ void __launch_bounds__(KD_THREADS) kd_swap_kernel(const KdLevel lv) {
     }
     __syncthreads();
     if (threadIdx.x == 0) lv.st->ticket = 0;
-    kd_tile_map(lv.next, lv.next_sp, min(s_next, lv.seg_cap), lv.tile_seg, lv.tile_cap, lv.st);
+    kd_tile_map(lv.next, lv.next_sp, min(s_next, lv.seg_cap), lv.tile_seg, lv.tile_cap, lv.tile, lv.st);
 }
 
 // The roots: extents, cuts and tile list of the first level (one block).
@@ -742,7 +767,7 @@ __global__ void __launch_bounds__(KD_THREADS) kd_roots_kernel(const KdLevel lv, 
         kd_plan_segment(sg, &lv.N.bmin[3 * sg.node], &lv.N.bmax[3 * sg.node], lv.tfs[sg.pad], &lv.sp[s]);
     }
     __syncthreads();
-    kd_tile_map(lv.segs, lv.sp, S, lv.tile_seg, lv.tile_cap, lv.st);
+    kd_tile_map(lv.segs, lv.sp, S, lv.tile_seg, lv.tile_cap, lv.tile, lv.st);
 }
 
 // ---------------------------------------------------------------------------
@@ -824,6 +849,7 @@ __global__ void __launch_bounds__(KD_BTHREADS, 2) kd_block_build_kernel(
         const KdSeg root = small[blockIdx.x];
         const uint32_t base = root.begin, total = root.end - root.begin;
         const Transform tf = tfs[root.pad];
+        const double inv[3] = {1.0 / tf.scale[0], 1.0 / tf.scale[1], 1.0 / tf.scale[2]};
         for (uint32_t i = threadIdx.x; i < total; i += KD_BTHREADS) {
             sh.c[0][i] = rx[base + i];
             sh.c[1][i] = ry[base + i];
@@ -878,13 +904,16 @@ __global__ void __launch_bounds__(KD_BTHREADS, 2) kd_block_build_kernel(
             }
             bool split = count > (uint32_t)KD_LEAF;
             if (split) {
+                // the children's numbers, asked for now and used after the passes
+                uint32_t cid = 0;
+                if (t == 0) cid = atomicAdd(&st->nodes, 2u);
                 int f;
                 double cut;
                 kd_choose_cut(lo, hi, mn, mx, tf, f, cut);
                 uint32_t t1, t2;
                 const int32_t org = f == 0 ? mn[0] : (f == 1 ? mn[1] : mn[2]);
-                kd_thresholds(cut, tf.scale[f], tf.offset[f], org, f == 0 ? mx[0] : (f == 1 ? mx[1] : mx[2]),
-                              t1, t2);
+                kd_warp_thresholds(cut, tf.scale[f], f == 0 ? inv[0] : (f == 1 ? inv[1] : inv[2]), tf.offset[f],
+                                   org, f == 0 ? mx[0] : (f == 1 ? mx[1] : mx[2]), t1, t2);
                 const int32_t* v = sh.c[f];
                 // each warp of the group takes a run of rows
                 const uint32_t rows = (count + 31) / 32, per = (rows + W - 1) / W;
@@ -930,9 +959,7 @@ __global__ void __launch_bounds__(KD_BTHREADS, 2) kd_block_build_kernel(
                     kd_group_pass(sh, v, b2, e, org, t2, eq, before2, q0, q1, W, w0);
                 }
                 const uint32_t mid = b + kd_split_index(count, L, eq);
-                uint32_t cid = 0;
                 if (t == 0) {
-                    cid = atomicAdd(&st->nodes, 2u);
                     if (cid + 2 <= N.cap)
                         kd_write_children(N, node, cid, f, base + b, base + mid, base + e, root.pad);
                     else atomicAdd(&st->errors, 1u);
@@ -1354,6 +1381,52 @@ static int kd_alloc_nodes(Context* ctx, KdForest* kd, uint32_t nc) {
     return NBG_OK;
 }
 
+// A single tree's points, root and build state in one launch (ten small copies
+// from the host cost as much as a level).
+struct KdRoot {
+    KdSeg seg;
+    int32_t mn[3], mx[3];
+    Transform tf;
+};
+
+__global__ void kd_init_one_kernel(const int32_t* __restrict__ x, const int32_t* __restrict__ y,
+                                   const int32_t* __restrict__ z, uint32_t n, int32_t* rx, int32_t* ry,
+                                   int32_t* rz, uint32_t* rid, const KdRoot root, KdNodes N, KdSeg* dst,
+                                   Transform* tfs, uint64_t* bases, KdState* st, const KdState state) {
+    for (uint64_t i = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x; i < n;
+         i += (uint64_t)gridDim.x * blockDim.x) {
+        rx[i] = x[i];
+        ry[i] = y[i];
+        rz[i] = z[i];
+        rid[i] = (uint32_t)i;
+    }
+    if (blockIdx.x || threadIdx.x) return;
+    N.c1[0] = N.c2[0] = -1;
+    N.feat[0] = 0;
+    N.nb[0] = 0;
+    N.ne[0] = n;
+    N.ntree[0] = 0;
+    for (int d = 0; d < 3; ++d) {
+        N.bmin[d] = root.mn[d];
+        N.bmax[d] = root.mx[d];
+    }
+    *dst = root.seg;
+    *tfs = root.tf;
+    *bases = 0;
+    *st = state;
+}
+
+// The passes of one level.
+template <int ROWS>
+static void kd_level(const KdLevel& lv, unsigned blocks, cudaStream_t st) {
+    kd_count_kernel<1, ROWS><<<blocks, KD_THREADS, 0, st>>>(lv);
+    kd_classify_kernel<1, ROWS><<<blocks, KD_THREADS, 0, st>>>(lv);
+    kd_swap_kernel<1><<<blocks, KD_THREADS, 0, st>>>(lv);
+    kd_count_kernel<2, ROWS><<<blocks, KD_THREADS, 0, st>>>(lv);
+    kd_classify_kernel<2, ROWS><<<blocks, KD_THREADS, 0, st>>>(lv);
+    kd_swap_kernel<2><<<blocks, KD_THREADS, 0, st>>>(lv);
+}
+
 // One build of the forest over `tiles`.  Levels are queued without reading
 // anything back: the kernels take the segment and tile counts from the device,
 // and a level with nothing left exits at once.
@@ -1366,8 +1439,9 @@ static int kd_build(Context* ctx, KdForest* kd, Tile* const* tiles, cudaStream_t
     for (int k = 0; k < T; ++k) {
         const Tile* t = tiles[k];
         const uint64_t b = kd->base[k], n = kd->npts[k];
-        kd_init_kernel<<<grid_for(ctx, n), 256, 0, st>>>(t->x, t->y, t->z, n, kd->rx + b, kd->ry + b,
-                                                         kd->rz + b, kd->rid + b);
+        if (T > 1)
+            kd_init_kernel<<<grid_for(ctx, n), 256, 0, st>>>(t->x, t->y, t->z, n, kd->rx + b, kd->ry + b,
+                                                             kd->rz + b, kd->rid + b);
         // root: the tile's actual bounding box, as calculateBounds
         const GridParams& g = t->host_gp;
         const int32_t mn[3] = {g.minx, g.miny, g.minz}, mx[3] = {g.maxx, g.maxy, g.maxz};
@@ -1398,41 +1472,52 @@ static int kd_build(Context* ctx, KdForest* kd, Tile* const* tiles, cudaStream_t
         set_err(ctx, "KD replica: too many trees for the segment lists");
         return NBG_ERR_UNSUPPORTED;
     }
-    // root nodes 0..T-1 (the host arrays outlive the copies: pageable sources are
-    // taken before the calls return)
-    void* const roots[] = {kd->c1, kd->c2, kd->feat, kd->nb, kd->ne, kd->ntree};
-    cudaError_t e = cudaSuccess;
-    for (int i = 0; i < 6 && !e; ++i)
-        e = cudaMemcpyAsync(roots[i], &init[(size_t)i * T], T * 4, cudaMemcpyHostToDevice, st);
-    if (!e) e = cudaMemcpyAsync(kd->bmin, &box[0], T * 12, cudaMemcpyHostToDevice, st);
-    if (!e) e = cudaMemcpyAsync(kd->bmax, &box[3 * (size_t)T], T * 12, cudaMemcpyHostToDevice, st);
-    if (!e) e = cudaMemcpyAsync(kd->tfs, kd->tfh.data(), T * sizeof(Transform), cudaMemcpyHostToDevice, st);
-    if (!e) e = cudaMemcpyAsync(kd->bases, kd->base.data(), T * 8, cudaMemcpyHostToDevice, st);
-    if (!e && !level0.empty())
-        e = cudaMemcpyAsync(kd->seg[0], level0.data(), level0.size() * sizeof(KdSeg), cudaMemcpyHostToDevice, st);
-    if (!e && !small0.empty())
-        e = cudaMemcpyAsync(kd->small, small0.data(), small0.size() * sizeof(KdSeg), cudaMemcpyHostToDevice, st);
+    const KdNodes N{kd->c1, kd->c2, kd->feat, kd->nb, kd->ne, kd->bmin, kd->bmax, kd->ntree, kd->node_cap};
     KdState state{};
     state.nodes = (uint32_t)T;
     state.small = (uint32_t)small0.size();
-    if (!e) e = cudaMemcpyAsync(kd->state, &state, sizeof(state), cudaMemcpyHostToDevice, st);
+    cudaError_t e = cudaSuccess;
+    if (T == 1) {
+        KdRoot root;
+        root.seg = level0.empty() ? small0[0] : level0[0];
+        for (int d = 0; d < 3; ++d) {
+            root.mn[d] = box[d];
+            root.mx[d] = box[3 + d];
+        }
+        root.tf = kd->tfh[0];
+        kd_init_one_kernel<<<grid_for(ctx, kd->n), 256, 0, st>>>(
+            tiles[0]->x, tiles[0]->y, tiles[0]->z, (uint32_t)kd->n, kd->rx, kd->ry, kd->rz, kd->rid, root, N,
+            level0.empty() ? kd->small : kd->seg[0], kd->tfs, kd->bases, kd->state, state);
+        e = cudaGetLastError();
+    } else {
+        // root nodes 0..T-1 (the host arrays outlive the copies: pageable sources are
+        // taken before the calls return)
+        void* const roots[] = {kd->c1, kd->c2, kd->feat, kd->nb, kd->ne, kd->ntree};
+        for (int i = 0; i < 6 && !e; ++i)
+            e = cudaMemcpyAsync(roots[i], &init[(size_t)i * T], T * 4, cudaMemcpyHostToDevice, st);
+        if (!e) e = cudaMemcpyAsync(kd->bmin, &box[0], T * 12, cudaMemcpyHostToDevice, st);
+        if (!e) e = cudaMemcpyAsync(kd->bmax, &box[3 * (size_t)T], T * 12, cudaMemcpyHostToDevice, st);
+        if (!e) e = cudaMemcpyAsync(kd->tfs, kd->tfh.data(), T * sizeof(Transform), cudaMemcpyHostToDevice, st);
+        if (!e) e = cudaMemcpyAsync(kd->bases, kd->base.data(), T * 8, cudaMemcpyHostToDevice, st);
+        if (!e && !level0.empty())
+            e = cudaMemcpyAsync(kd->seg[0], level0.data(), level0.size() * sizeof(KdSeg), cudaMemcpyHostToDevice, st);
+        if (!e && !small0.empty())
+            e = cudaMemcpyAsync(kd->small, small0.data(), small0.size() * sizeof(KdSeg), cudaMemcpyHostToDevice, st);
+        if (!e) e = cudaMemcpyAsync(kd->state, &state, sizeof(state), cudaMemcpyHostToDevice, st);
+    }
     if (e) {
         set_err(ctx, std::string("KD replica init failed: ") + cudaGetErrorString(e));
         return NBG_ERR_CUDA;
     }
-    const KdNodes N{kd->c1, kd->c2, kd->feat, kd->nb, kd->ne, kd->bmin, kd->bmax, kd->ntree, kd->node_cap};
-    uint32_t built = 0;  // small segments whose subtrees are queued
-    auto subtrees = [&](uint32_t upto) -> int {
-        if (upto <= built) return NBG_OK;
+    auto subtrees = [&](uint32_t ns) -> int {
+        if (!ns) return NBG_OK;
         if (cudaFuncSetAttribute(kd_block_build_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                  (int)sizeof(KdBlockShared)))
             return NBG_ERR_CUDA;
         if (kd->beside && cudaStreamWaitEvent(st, ctx->fev[0], 0)) return NBG_ERR_CUDA;
-        const uint32_t ns = upto - built;
         kd_block_build_kernel<<<ns, KD_BTHREADS, sizeof(KdBlockShared), st>>>(
-            kd->small + built, kd->rx, kd->ry, kd->rz, kd->rid, kd->kpos, kd->bases, N, kd->state, kd->tfs);
+            kd->small, kd->rx, kd->ry, kd->rz, kd->rid, kd->kpos, kd->bases, N, kd->state, kd->tfs);
         NBG_LAUNCHED(1);
-        built = upto;
         return NBG_OK;
     };
     int cur = 0;
@@ -1457,6 +1542,7 @@ static int kd_build(Context* ctx, KdForest* kd, Tile* const* tiles, cudaStream_t
         lv.seg_cap = kd->seg_cap;
         lv.small_cap = kd->small_cap;
         lv.tile_cap = kd->tile_cap;
+        lv.tile = kd->tile;
         return lv;
     };
     if (!level0.empty()) {
@@ -1472,12 +1558,8 @@ static int kd_build(Context* ctx, KdForest* kd, Tile* const* tiles, cudaStream_t
         while (true) {
             for (int l = 0; l < queued; ++l) {
                 const KdLevel lv = level(cur);
-                kd_count_kernel<1><<<blocks, KD_THREADS, 0, st>>>(lv);
-                kd_classify_kernel<1><<<blocks, KD_THREADS, 0, st>>>(lv);
-                kd_swap_kernel<1><<<blocks, KD_THREADS, 0, st>>>(lv);
-                kd_count_kernel<2><<<blocks, KD_THREADS, 0, st>>>(lv);
-                kd_classify_kernel<2><<<blocks, KD_THREADS, 0, st>>>(lv);
-                kd_swap_kernel<2><<<blocks, KD_THREADS, 0, st>>>(lv);
+                if (lv.tile == KD_THREADS * KD_ROWS_SHORT) kd_level<KD_ROWS_SHORT>(lv, blocks, st);
+                else kd_level<KD_ROWS_LONG>(lv, blocks, st);
                 cur ^= 1;
             }
             NBG_LAUNCHED(6 * queued);
@@ -1489,11 +1571,11 @@ static int kd_build(Context* ctx, KdForest* kd, Tile* const* tiles, cudaStream_t
                 return NBG_ERR_CUDA;
             }
             if (state.errors) return KD_RETRY;
-            const int rc = subtrees(state.small);
-            if (rc) return rc;
             if (!state.segs) break;
             queued = 3;
         }
+        const int rc = subtrees(state.small);  // (one launch: a block's latency is most of a small build)
+        if (rc) return rc;
     } else {
         const int rc = subtrees(state.small);
         if (rc) return rc;
@@ -1559,7 +1641,8 @@ int kd_ensure_many(Context* ctx, Tile* const* tiles, int count, cudaStream_t st,
     }
     kd->small_cap = (uint32_t)(n / 64 + 1024 + T);
     if (!rc) rc = kd_alloc(ctx, (void**)&kd->small, (size_t)kd->small_cap * sizeof(KdSeg), kd);
-    kd->tile_cap = (uint32_t)(n / KD_TILE + kd->seg_cap + 1);
+    kd->tile = KD_THREADS * (n <= KD_SHORT_MAX ? KD_ROWS_SHORT : KD_ROWS_LONG);
+    kd->tile_cap = (uint32_t)(n / kd->tile + kd->seg_cap + 1);
     if (!rc) rc = kd_alloc(ctx, (void**)&kd->tile_seg, (size_t)kd->tile_cap * 4, kd);
     if (!rc) rc = kd_alloc(ctx, (void**)&kd->tile_cnt, ((size_t)kd->tile_cap + 1) * 8, kd);
     if (!rc) rc = kd_alloc(ctx, (void**)&kd->state, sizeof(KdState), kd);
