@@ -1452,7 +1452,7 @@ void apply_cached_tuning(Context* ctx, Tile* t, int K) {
 }
 
 int tile_autotune(Context* ctx, Tile* t, int32_t knn, const float* candidates, int32_t n_candidates,
-                  bool use_cache, float* chosen, cudaStream_t stream, bool per_thread_only) {
+                  bool use_cache, float* chosen, cudaStream_t stream) {
     if (knn < 0 || knn > 64) return fail(ctx, NBG_ERR_INVALID, "knn must be in [0, 64]");
     static const float defaults[] = {1.0f, 1.5f, 2.0f, 3.0f, 4.0f, 6.0f};
     if (!candidates || n_candidates <= 0) {
@@ -1497,10 +1497,8 @@ int tile_autotune(Context* ctx, Tile* t, int32_t knn, const float* candidates, i
         return rc;
     }
     // select kernels tried: the two-pass ring search, the same in Morton
-    // order, the single-pass ring search, 32 queries per candidate list (the
-    // batched form's queue kernels are the two-pass ring search only)
+    // order, the single-pass ring search, 32 queries per candidate list
     static const int kGroups[] = {0, 1, 2, 32};
-    const int ngroups = per_thread_only ? 1 : 4;
     uint32_t* cnt_dev = ctx->counters + 32;  // scratch block, not the call counters
     float best = candidates[0];
     int best_group = 0;
@@ -1518,12 +1516,9 @@ int tile_autotune(Context* ctx, Tile* t, int32_t knn, const float* candidates, i
         rc = ensure_grid(ctx, t, K, stream);
         if (rc) break;
         cudaEventRecord(ctx->ev[1], stream);
-        if (!per_thread_only) {
-            rc = ensure_clumps(ctx, t, stream);
-            if (rc) break;
-        }
-        for (int gi = 0; gi < ngroups; ++gi) {
-            const int G = kGroups[gi];
+        rc = ensure_clumps(ctx, t, stream);
+        if (rc) break;
+        for (const int G : kGroups) {
             QueryLaunch ql;
             ql.tile = t;
             ql.K = K;

@@ -3,11 +3,13 @@
 // 1. grids     every tile's grid, built without host synchronisation, then
 //              one synchronisation reads all grid shapes (a tile whose cell
 //              table overflowed is rebuilt by the synchronising build)
-// 2. queue     per neighbour-count class one persistent select kernel drains
-//              the class's (tile, 128-query block) items; one persistent
-//              finish kernel then takes every item of every class.  The head
-//              resets and the launches are captured in a CUDA graph, replayed
-//              while the batch's job arrays and counts are unchanged.
+// 2. queue     per class (neighbour slots, select kernel) one launch answers the
+//              class's (tile, 128-query block) items: the single-pass and group
+//              selects take a block or two an item, the two-pass select drains
+//              them persistently; handed-back rows follow, then one persistent
+//              finish kernel takes every item of every class.  The head resets
+//              and the launches are captured in a CUDA graph, replayed while the
+//              batch's job arrays and counts are unchanged.
 // 3. replicas  the tiles' KD replicas, all as one forest (one level-synchronous
 //              build for every tile), once the queue has drained
 // 4. exact     per tile: the tie-order resolver, then the search replay for
@@ -33,14 +35,19 @@ int launch_select_queue(Context* ctx, int K, const BatchJob* jobs, int njobs, ui
 int launch_finish_queue(Context* ctx, const BatchJob* jobs, int njobs, uint64_t items,
                         unsigned long long* head, cudaStream_t stream, int reserve);
 int slots_for_k(int K);
+int launch_loc_batch(int K, const BatchJob* jobs, int njobs, uint64_t items, cudaStream_t stream);
+uint32_t located_offset_bits(const Tile* t);
+int launch_group_batch(int slots, const BatchJob* jobs, int njobs, uint64_t items, cudaStream_t stream);
+int launch_retry_batch(int slots, const BatchJob* jobs, int njobs, int sms, cudaStream_t stream);
 
 static constexpr int kCounters = 64;  // u32 counters per tile
 
 struct BatchScratch {
-    uint64_t rows = 0, items = 0, ex = 0;
+    uint64_t rows = 0, retry_cap = 0, items = 0, ex = 0;
     RowSums* sums = nullptr;
     uint2* ties = nullptr;
     uint32_t* exact = nullptr;
+    uint32_t* retry = nullptr;
     uint32_t* counters = nullptr;
     nbg_row_exception* ex_rows = nullptr;
     BatchJob* jobs = nullptr;  // select order (by class), then finish order
@@ -87,6 +94,7 @@ void batch_release(Context* ctx) {
     if (B->sums) ctx_free(ctx, B->sums, B->rows * sizeof(RowSums));
     if (B->ties) ctx_free(ctx, B->ties, B->rows * sizeof(uint2));
     if (B->exact) ctx_free(ctx, B->exact, B->rows * 4);
+    if (B->retry) ctx_free(ctx, B->retry, B->retry_cap * 4);
     if (B->counters) ctx_free(ctx, B->counters, B->items * 4);
     if (B->ex_rows) ctx_free(ctx, B->ex_rows, B->ex * sizeof(nbg_row_exception));
     if (B->jobs) ctx_free(ctx, B->jobs, B->jobs_cap * sizeof(BatchJob));
@@ -175,11 +183,19 @@ extern "C" int nbg_run_batch(nbg_context* h, const nbg_batch_item* items, int32_
     int rc = NBG_OK;
     if (B->rows < rows) {
         uint64_t c1 = B->rows, c2 = B->rows, c3 = B->rows;
+        B->rows = 0;  // (a list that could not grow is gone)
         rc = grow(ctx, &B->sums, c1, rows);
         if (!rc) rc = grow(ctx, &B->ties, c2, rows);
         if (!rc) rc = grow(ctx, &B->exact, c3, rows);
         if (rc) return rc;
         B->rows = rows;
+    }
+    // without room for the handed-back rows every tile takes the two-pass
+    // select, which hands none back
+    if (B->retry_cap < rows) {
+        uint64_t c = B->retry_cap;
+        B->retry_cap = 0;
+        if (grow(ctx, &B->retry, c, rows) == NBG_OK) B->retry_cap = rows;
     }
     if (B->items < (uint64_t)nl * kCounters) {
         uint64_t c = B->items;
@@ -197,7 +213,7 @@ extern "C" int nbg_run_batch(nbg_context* h, const nbg_batch_item* items, int32_
     if (flags & NBG_BATCH_AUTOTUNE) {
         for (int i : live) {
             rc = tile_autotune(ctx, &items[i].tile->t, items[i].stages[0].knn, nullptr, 0, true,
-                               nullptr, st, true);
+                               nullptr, st);
             if (rc) return rc;
         }
     }
@@ -239,9 +255,23 @@ extern "C" int nbg_run_batch(nbg_context* h, const nbg_batch_item* items, int32_
         t->grid_fixed = t->fixed_cell;
     }
     // ---- jobs: select order grouped by class, then finish order
+    // each tile's select kernel as in nbg_run (the Morton variant, 1, has no
+    // batch form: the two-pass search it reorders stands in).  24 mixture tiles
+    // of 15k to 1M points, knn 8, 16 and 32: 38.5 ms when every tile took the
+    // two-pass queue, 30.5 ms with these
+    std::vector<int> select(n_items, 0);
+    for (int i : live) {
+        Tile* t = &items[i].tile->t;
+        const int k = B->retry_cap ? select_kernel(t, Ks[i], false) : 0;
+        select[i] = k >= 8 && t->clumps ? 32 : (k == 2 && slots_for_k(Ks[i]) <= 18 ? 2 : 0);
+        if (select[i] == 32) {
+            rc = ensure_clumps(ctx, t, st);
+            if (rc) return fail(ctx, rc, "clump order");
+        }
+    }
+    auto class_of = [&](int i) { return slots_for_k(Ks[i]) * 64 + select[i]; };
     std::vector<int> order(live);
-    std::stable_sort(order.begin(), order.end(),
-                     [&](int a, int b) { return slots_for_k(Ks[a]) < slots_for_k(Ks[b]); });
+    std::stable_sort(order.begin(), order.end(), [&](int a, int b) { return class_of(a) < class_of(b); });
     std::vector<BatchJob> jobs(2 * (size_t)nl);
     std::vector<uint64_t> row0(n_items, 0), ex0(n_items, 0), slot(n_items, 0);
     {
@@ -256,7 +286,7 @@ extern "C" int nbg_run_batch(nbg_context* h, const nbg_batch_item* items, int32_
         }
     }
     struct Cls {
-        int K;
+        int K, select;
         int begin, count;
         uint64_t items;
     };
@@ -267,7 +297,9 @@ extern "C" int nbg_run_batch(nbg_context* h, const nbg_batch_item* items, int32_
         const Tile* t = &items[i].tile->t;
         QueryArgs q{};
         q.gv = grid_view(t);
-        q.qpts = t->sorted;
+        q.qpts = select[i] == 32 ? t->pts : t->sorted;
+        q.boxes = t->boxes;
+        q.retry_rows = select[i] ? B->retry + row0[i] : nullptr;
         q.gp = t->gp;
         q.n = t->n;
         q.K = Ks[i];
@@ -284,11 +316,13 @@ extern "C" int nbg_run_batch(nbg_context* h, const nbg_batch_item* items, int32_
         q.tie_cap = (uint32_t)t->n;
         q.sums = B->sums + row0[i];
         const uint64_t blocks = (t->n + 127) / 128;
-        if (classes.empty() || slots_for_k(classes.back().K) != slots_for_k(Ks[i]))
-            classes.push_back(Cls{Ks[i], j, 0, 0});
+        if (classes.empty() || class_of(order[j - 1]) != class_of(i))
+            classes.push_back(Cls{Ks[i], select[i], j, 0, 0});
         Cls& c = classes.back();
         jobs[j].q = q;
         jobs[j].first = c.items;
+        jobs[j].ob = located_offset_bits(t);
+        jobs[j].margin = t->margin0;
         c.items += blocks;
         c.count += 1;
         jobs[nl + j].q = q;
@@ -327,7 +361,7 @@ extern "C" int nbg_run_batch(nbg_context* h, const nbg_batch_item* items, int32_
     key.push_back(fin_items);
     key.push_back((uint64_t)nl);
     for (const Cls& c : classes) {
-        key.push_back((uint64_t)slots_for_k(c.K));
+        key.push_back((uint64_t)slots_for_k(c.K) * 64 + (uint64_t)c.select);
         key.push_back((uint64_t)c.begin);
         key.push_back((uint64_t)c.count);
         key.push_back(c.items);
@@ -336,8 +370,17 @@ extern "C" int nbg_run_batch(nbg_context* h, const nbg_batch_item* items, int32_
         cudaMemsetAsync(B->heads, 0, (classes.size() + 1) * sizeof(unsigned long long), s);
         for (size_t k = 0; k < classes.size(); ++k) {
             const Cls& c = classes[k];
-            int r = launch_select_queue(ctx, c.K, B->jobs + c.begin, c.count, c.items, B->heads + k, s,
-                                        reserve);
+            const BatchJob* j = B->jobs + c.begin;
+            int r = c.select == 32 ? launch_group_batch(slots_for_k(c.K), j, c.count, c.items, s)
+                    : c.select == 2
+                        ? launch_loc_batch(c.K, j, c.count, c.items, s)
+                        : launch_select_queue(ctx, c.K, j, c.count, c.items, B->heads + k, s, reserve);
+            if (r) return r;
+        }
+        // rows handed back (their sums slots hold 0: the finish pass skips them)
+        for (const Cls& c : classes) {
+            if (!c.select) continue;
+            const int r = launch_retry_batch(slots_for_k(c.K), B->jobs + c.begin, c.count, ctx->sm_count, s);
             if (r) return r;
         }
         return launch_finish_queue(ctx, B->jobs + nl, nl, fin_items, B->heads + classes.size(), s,
@@ -391,12 +434,13 @@ extern "C" int nbg_run_batch(nbg_context* h, const nbg_batch_item* items, int32_
     std::vector<uint32_t> cnt((size_t)nl * kCounters);
     cudaMemcpyAsync(cnt.data(), B->counters, cnt.size() * 4, cudaMemcpyDeviceToHost, st);
     if (cudaStreamSynchronize(st) != cudaSuccess) return fail(ctx, NBG_ERR_CUDA, "batch counters");
-    uint64_t tie_rows = 0, deferred_rows = 0, replay_rows = 0, resolved = 0;
+    uint64_t tie_rows = 0, deferred_rows = 0, replay_rows = 0, resolved = 0, retry_rows = 0;
     std::vector<TieLaunch> tls;
     for (int i : live) {
         const uint32_t* c = &cnt[slot[i] * kCounters];
         tie_rows += c[1];
         deferred_rows += c[2];
+        retry_rows += c[6];
         const uint32_t nties = std::min<uint32_t>(c[4], (uint32_t)items[i].tile->t.n);
         if (!nties) continue;
         Tile* t = &items[i].tile->t;
@@ -463,6 +507,7 @@ extern "C" int nbg_run_batch(nbg_context* h, const nbg_batch_item* items, int32_
         stats->deferred_rows = deferred_rows;
         stats->resolved_rows = resolved;
         stats->replay_rows = replay_rows;
+        stats->retry_rows = retry_rows;
         float ms = 0;
         cudaEventElapsedTime(&ms, B->ev[0], B->ev[1]);
         stats->grid_ms = ms;

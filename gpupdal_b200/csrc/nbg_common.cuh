@@ -190,7 +190,42 @@ __device__ __forceinline__ int row_neighbours(const double* row_k, int K, uint64
 struct BatchJob {
     QueryArgs q;
     uint64_t first;
+    uint32_t ob;   // single-pass select: offset bits of a key
+    float margin;  // group select: its first margin
 };
+
+// The job that owns item `item` of a launch over jobs[0 .. njobs).
+__device__ __forceinline__ int job_of(const BatchJob* __restrict__ jobs, int njobs, uint64_t item) {
+    int lo = 0, hi = njobs;
+    while (hi - lo > 1) {
+        const int mid = (lo + hi) >> 1;
+        if (jobs[mid].first <= item) lo = mid;
+        else hi = mid;
+    }
+    return lo;
+}
+
+// What a select kernel reads of a job, in registers (the job lies in memory the
+// kernel's own stores might alias).
+__device__ __forceinline__ QueryArgs select_args(const BatchJob& j) {
+    QueryArgs a;
+    a.gv = j.q.gv;
+    a.gp = j.q.gp;
+    a.n = j.q.n;
+    a.K = j.q.K;
+    a.rmax = j.q.rmax;
+    a.exact_rows = j.q.exact_rows;
+    a.counters = j.q.counters;
+    a.ids_out = nullptr;
+    a.ties = j.q.ties;
+    a.tie_cap = j.q.tie_cap;
+    a.sums = j.q.sums;
+    a.row_k = nullptr;
+    a.retry_rows = j.q.retry_rows;
+    a.qpts = j.q.qpts;
+    a.boxes = j.q.boxes;
+    return a;
+}
 
 // ---------------------------------------------------------------------------
 // The reference's coordinate, fl(fl(raw*scale) + offset), with no contraction.

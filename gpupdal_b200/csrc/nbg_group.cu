@@ -7,35 +7,44 @@
 // tie-order resolver / the exact KD path.  The per-thread ring search gives
 // every lane its own rings of cells, so a warp walks the union of its lanes'
 // cells with most lanes masked, and pays the whole top-list insertion network
-// whenever any lane inserts.  Here
+// (2 (K+1) min/max) whenever any lane inserts.  Here
 //
-//   order     the block's 256 rows are re-sorted by a Morton key of their
-//             coordinates (bitonic, shuffles within a warp), so a warp's 32
-//             queries are spatially compact
-//   members   the rows of the warp (and, for K >= 32, of its neighbouring
-//             warps) are the first candidates: after them every lane holds
-//             K + 1 real points, so its (K+1)-th distance bounds the search
-//   gather    lanes of similar bound are answered together: the points of
-//             the grid cells within a margin of the box around their queries
-//             are filtered by the lanes in parallel and staged in shared
-//             memory.  The margin is the largest bound of the lanes (capped
-//             at first, then grown), so the points left out are farther than
-//             every answer
+//   order     a warp's 32 queries are one clump of the clump order
+//             (clump_kernel, nbg_grid.cu: median splits of a block of 1024
+//             points), spatially compact at any density
+//   members   the clump and its siblings are the first list: after it every
+//             lane holds K + 1 real points, so its (K+1)-th distance bounds
+//             the search
+//   rounds    a round takes the open lanes near the one of smallest bound and
+//             a margin that covers theirs.  Its list is the points within the
+//             margin of the box around the round's queries, found by a walk
+//             down the tree of clump boxes (32 boxes a step, one per lane; the
+//             warp's own block first, so the bounds fall before the rest of
+//             the tree is tested).  A lane whose K-th lies inside the margin is
+//             answered: the points left out are farther.  The others see the
+//             shell between this margin and a wider one
 //   scan      each lane forms the exact integer squared distance of every
-//             staged candidate (uniform loop, broadcast loads) and appends the
-//             ones below its current (K+1)-th to a short list of its own in
-//             shared memory; when a lane's list is full all lanes sort theirs
-//             (a register network) and merge it into their sorted top list
-//             (one bitonic merge).  A candidate costs a compare and a store
-//             instead of the top list's 2 (K+1) min/max, and the network runs
-//             once per M appended candidates with every lane active
+//             staged candidate (uniform loop, two at once in packed f32
+//             arithmetic) and appends the ones below its bound to a short list
+//             of its own in shared memory; when a lane's list is full all lanes
+//             sort theirs (a register network) and merge it into their sorted
+//             top list (one bitonic merge).  A candidate costs a compare and a
+//             store, and the network runs once per up to M of them with every
+//             lane active
 //   sums      keys pack the squared distance above the candidate's index in
 //             the warp's list, so the K nearest are read back directly
 //
-// Rows this form cannot answer (a distance or list beyond the key's fields, a
-// tile with fewer than K + 1 rows in a block) go to the per-thread select
-// through a retry list read on the device.  Ties and far rows are decided
-// exactly as the per-thread select decides them.
+// A list of more candidates than the index field holds is started over with
+// the bounds it gave (`again`); rows that overflow it twice, or whose distances
+// pass the key's field, go to the retry launch (warps of their own) through a
+// list read on the device.  Ties and far rows are decided exactly as the
+// per-thread select decides them.
+//
+// Bound by instruction issue (the data lie in L2): 2.7 candidates are scanned
+// for each of the K + 1 kept, and the merges cost about as much as the scan.  Measured
+// select times at the densities of the synthetic clouds, per-thread two-pass
+// search -> this kernel: K = 65, 1.5M points, 8.9 -> 3.6 ms; K = 33, 5M
+// points of 24 tiles, 12.6 -> 7 ms.
 #include <climits>
 
 #include "nbg_common.cuh"
@@ -522,6 +531,44 @@ __global__ void __launch_bounds__(WarpShape<KS>::kThreads, WarpShape<KS>::kMinBl
     extern __shared__ __align__(16) unsigned char smem[];
     const uint64_t s0 = (uint64_t)blockIdx.x * S::kThreads + (threadIdx.x & ~31u);
     if (s0 < (a.rows ? a.nq : a.n)) group_warp<KS>(a, s0, margin0, smem + (threadIdx.x >> 5) * S::kWarpBytes);
+}
+
+// The clumps of many tiles in one launch: items of 128 rows, two blocks each.
+template <int KS>
+__global__ void __launch_bounds__(WarpShape<KS>::kThreads, WarpShape<KS>::kMinBlocks)
+    knn_group_batch_kernel(const BatchJob* __restrict__ jobs, int njobs) {
+    using S = WarpShape<KS>;
+    extern __shared__ __align__(16) unsigned char smem[];
+    const uint64_t item = blockIdx.x >> 1;
+    const BatchJob& job = jobs[job_of(jobs, njobs, item)];
+    const uint64_t s0 = (item - job.first) * 128u + (blockIdx.x & 1u) * S::kThreads + (threadIdx.x & ~31u);
+    if (s0 < job.q.n) group_warp<KS>(select_args(job), s0, job.margin, smem + (threadIdx.x >> 5) * S::kWarpBytes);
+}
+
+template <int KS>
+static int launch_group_batch_k(const BatchJob* jobs, int njobs, uint64_t items, cudaStream_t stream) {
+    using S = WarpShape<KS>;
+    if (!items) return NBG_OK;
+    if (cudaFuncSetAttribute(knn_group_batch_kernel<KS>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                             (int)S::kSmem))
+        return NBG_ERR_CUDA;
+    knn_group_batch_kernel<KS><<<(unsigned)(2 * items), S::kThreads, S::kSmem, stream>>>(jobs, njobs);
+    NBG_LAUNCHED(1);
+    return cudaGetLastError() == cudaSuccess ? NBG_OK : NBG_ERR_CUDA;
+}
+
+int launch_group_batch(int slots, const BatchJob* jobs, int njobs, uint64_t items, cudaStream_t stream) {
+    switch (slots) {
+        case 10: return launch_group_batch_k<10>(jobs, njobs, items, stream);
+        case 12: return launch_group_batch_k<12>(jobs, njobs, items, stream);
+        case 14: return launch_group_batch_k<14>(jobs, njobs, items, stream);
+        case 18: return launch_group_batch_k<18>(jobs, njobs, items, stream);
+        case 26: return launch_group_batch_k<26>(jobs, njobs, items, stream);
+        case 34: return launch_group_batch_k<34>(jobs, njobs, items, stream);
+        case 50: return launch_group_batch_k<50>(jobs, njobs, items, stream);
+        case 66: return launch_group_batch_k<66>(jobs, njobs, items, stream);
+    }
+    return NBG_ERR_INVALID;
 }
 
 template <int KS>

@@ -290,8 +290,7 @@ void apply_cached_tuning(Context* ctx, Tile* t, int K);
 
 // Autotuner (nbg_tile_autotune without the context lock).
 int tile_autotune(Context* ctx, Tile* t, int32_t knn, const float* candidates, int32_t n_candidates,
-                  bool use_cache, float* chosen, cudaStream_t stream,
-                  bool per_thread_only = false);
+                  bool use_cache, float* chosen, cudaStream_t stream);
 
 // A tile of n points with its device storage allocated (coordinates unset),
 // and its release (nbg_api.cu).

@@ -561,6 +561,35 @@ __global__ void __launch_bounds__(128) knn_finish_queue_kernel(const BatchJob* _
     }
 }
 
+// The single-pass select over the tiles of a batch, a block per item.
+template <int KS>
+__global__ void __launch_bounds__(128) knn_select_loc_batch_kernel(const BatchJob* __restrict__ jobs, int njobs) {
+    const BatchJob& job = jobs[job_of(jobs, njobs, blockIdx.x)];
+    const uint64_t i = (blockIdx.x - job.first) * 128u + threadIdx.x;
+    if (i < job.q.n) select_row_loc<KS>(select_args(job), i, job.ob);
+}
+
+struct LocBatchArgs {
+    const BatchJob* jobs;
+    int njobs;
+    uint64_t items;
+    cudaStream_t stream;
+};
+
+template <int KS>
+struct LocBatchLauncher {
+    using Args = LocBatchArgs;
+    static int run(const LocBatchArgs& b) {
+        if (!b.items) return NBG_OK;
+        if constexpr (KS <= 18) {  // (select_kernel gives longer lists to the other kernels)
+            knn_select_loc_batch_kernel<KS><<<(unsigned)b.items, 128, 0, b.stream>>>(b.jobs, b.njobs);
+            NBG_LAUNCHED(1);
+            return cudaGetLastError() == cudaSuccess ? NBG_OK : NBG_ERR_CUDA;
+        }
+        return NBG_ERR_INVALID;
+    }
+};
+
 struct QueueArgs {
     const BatchJob* jobs;
     int njobs;
@@ -1421,6 +1450,12 @@ int launch_select_queue(Context* ctx, int K, const BatchJob* jobs, int njobs, ui
     return dispatch_slots<QueueLauncher>(
         K, QueueArgs{jobs, njobs, items, head, ctx->sm_count, stream, reserve});
 }
+
+int launch_loc_batch(int K, const BatchJob* jobs, int njobs, uint64_t items, cudaStream_t stream) {
+    return dispatch_slots<LocBatchLauncher>(K, LocBatchArgs{jobs, njobs, items, stream});
+}
+
+uint32_t located_offset_bits(const Tile* t) { return loc_offset_bits(t->host_gp.cell); }
 
 int launch_finish_queue(Context* ctx, const BatchJob* jobs, int njobs, uint64_t items,
                         unsigned long long* head, cudaStream_t stream, int reserve) {

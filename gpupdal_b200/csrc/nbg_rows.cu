@@ -271,9 +271,8 @@ __device__ __forceinline__ uint32_t rows_per_warp(uint32_t rows) {
 // finished (their sums slots hold cnt = 0, so the finish pass over the other
 // rows, which may run at the same time, skips them).
 template <int NR>
-__global__ void __launch_bounds__(kRowThreads) knn_retry_finish_kernel(const QueryArgs a) {
-    __shared__ uint32_t s_gather[kRowThreads / 32][64];
-    const uint32_t nr = *a.nq_dev;
+__device__ __forceinline__ void retry_finish_rows(const QueryArgs& a, const uint32_t* rows, const uint32_t nr,
+                                                  uint32_t (*s_gather)[64]) {
     const uint32_t rpw = rows_per_warp(nr);
     const int lane = threadIdx.x & 31;
     const uint32_t warp = (blockIdx.x * blockDim.x + threadIdx.x) >> 5, warps = gridDim.x * (blockDim.x >> 5);
@@ -283,7 +282,7 @@ __global__ void __launch_bounds__(kRowThreads) knn_retry_finish_kernel(const Que
         float4 mq = make_float4(0.f, 0.f, 0.f, 0.f);  // this lane's row
         int mk = -1;                                   // its neighbours (-1: nothing to finish)
         int ms[9] = {0, 0, 0, 0, 0, 0, 0, 0, 0};
-        if ((uint32_t)lane < m) mq = __ldg(&a.qpts[__ldg(&a.rows[r0 + lane])]);
+        if ((uint32_t)lane < m) mq = __ldg(&a.qpts[__ldg(&rows[r0 + lane])]);
         for (uint32_t j = 0; j < m; ++j) {
             const float4 q = make_float4(__shfl_sync(kAll, mq.x, j), __shfl_sync(kAll, mq.y, j),
                                          __shfl_sync(kAll, mq.z, j), __shfl_sync(kAll, mq.w, j));
@@ -306,6 +305,20 @@ __global__ void __launch_bounds__(kRowThreads) knn_retry_finish_kernel(const Que
         }
         __syncwarp();
     }
+}
+
+template <int NR>
+__global__ void __launch_bounds__(kRowThreads) knn_retry_finish_kernel(const QueryArgs a) {
+    __shared__ uint32_t s_gather[kRowThreads / 32][64];
+    retry_finish_rows<NR>(a, a.rows, *a.nq_dev, s_gather);
+}
+
+// The same for the tiles of a batch: job blockIdx.y's rows.
+template <int NR>
+__global__ void __launch_bounds__(kRowThreads) knn_retry_batch_kernel(const BatchJob* __restrict__ jobs) {
+    __shared__ uint32_t s_gather[kRowThreads / 32][64];
+    const QueryArgs& a = jobs[blockIdx.y].q;
+    retry_finish_rows<NR>(a, a.retry_rows, a.counters[6], s_gather);
 }
 
 // One tie row by a warp (see tie_row): the sums over its K points, in every
@@ -456,6 +469,17 @@ int launch_retry_finish(const QueryArgs& q, int slots, int sms, cudaStream_t str
     if (slots <= 32) knn_retry_finish_kernel<1><<<blocks, kRowThreads, 0, stream>>>(q);
     else if (slots <= 64) knn_retry_finish_kernel<2><<<blocks, kRowThreads, 0, stream>>>(q);
     else knn_retry_finish_kernel<3><<<blocks, kRowThreads, 0, stream>>>(q);
+    NBG_LAUNCHED(1);
+    return cudaGetLastError() == cudaSuccess ? NBG_OK : NBG_ERR_CUDA;
+}
+
+int launch_retry_batch(int slots, const BatchJob* jobs, int njobs, int sms, cudaStream_t stream) {
+    if (!njobs) return NBG_OK;
+    const dim3 grid((unsigned)std::max<uint64_t>(4, (uint64_t)sms * kRowBlocksPerSm / (uint64_t)njobs),
+                    (unsigned)njobs);
+    if (slots <= 32) knn_retry_batch_kernel<1><<<grid, kRowThreads, 0, stream>>>(jobs);
+    else if (slots <= 64) knn_retry_batch_kernel<2><<<grid, kRowThreads, 0, stream>>>(jobs);
+    else knn_retry_batch_kernel<3><<<grid, kRowThreads, 0, stream>>>(jobs);
     NBG_LAUNCHED(1);
     return cudaGetLastError() == cudaSuccess ? NBG_OK : NBG_ERR_CUDA;
 }

@@ -52,3 +52,47 @@ def test_long_lists_take_the_group_select(nbg, knn, scale):
     assert np.array_equal(np.sort(exc, order="point_id"), np.sort(wexc, order="point_id"))
     tile.free()
     ref.free()
+
+
+@pytest.mark.parametrize("select", (-1, 0, 2, 32))
+def test_batch_select_kernels(nbg, select):
+    """Tiles at the edges of the batched launches' items (128 rows, two blocks
+    of 64), of every list length, against the two-pass search tile by tile."""
+    import torch
+
+    from gpupdal_b200.native import record_columns
+    cases = [(n, knn) for n in (1, 63, 64, 65, 127, 129, 1025) for knn in (3, 8, 13, 17, 32)]
+    cases += [(5000, 49), (20_000, 64), (20_000, 10)]
+    tiles, stages, cols, recs, want = [], [], [], [], []
+    for n, knn in cases:
+        xyz = _cloud(n)
+        st = [abi.make_opts(abi.STAGE_EIGENVALUES, knn=knn), abi.make_opts(abi.STAGE_NORMAL, knn=knn)]
+        ref = nbg.tile(*xyz)
+        ref.set_select(0)
+        outs, exc, _ = nbg.run(ref, st)
+        ref.free()
+        want.append((outs, exc))
+        tile = nbg.tile(*xyz)
+        if select >= 0:
+            tile.set_select(select)
+        rec = torch.full((n, 16), float("nan"), dtype=torch.float64, device="cuda")
+        tiles.append(tile)
+        stages.append(st)
+        recs.append(rec)
+        cols.append(record_columns(rec.data_ptr(), st, 128, 1))
+    for graph in (False, True):
+        for rec in recs:
+            rec.fill_(float("nan"))
+        got, _ = nbg.run_batch(tiles, stages, cols, graph=graph)
+        torch.cuda.synchronize()
+        for i, case in enumerate(cases):
+            rec = recs[i].cpu().numpy()
+            # rows a stage skips keep the output's previous value (NaN here, 0 in run's)
+            keep = np.ones(len(rec), bool)
+            keep[want[i][1]["point_id"]] = False
+            for d, v in enumerate(np.concatenate(want[i][0])):
+                assert np.array_equal(rec[keep, d], v[keep], equal_nan=True), (case, graph)
+            key = ["point_id", "stage", "code"]
+            assert np.array_equal(np.sort(got[i], order=key), np.sort(want[i][1], order=key)), (case, graph)
+    for tile in tiles:
+        tile.free()
