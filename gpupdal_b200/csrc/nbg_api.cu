@@ -841,6 +841,7 @@ static int run_pipelined(Context* ctx, Tile* t, int K, int select, const StageGr
         ql.row_k = nullptr;
         ql.rows = rows + b[c];
         ql.nrows = b[c + 1] - b[c];
+        ql.id0 = (int64_t)b[c];
         ql.retry_rows = ctx->retry_rows + b[c];
         ql.group = select;
         ql.margin0 = t->margin0;

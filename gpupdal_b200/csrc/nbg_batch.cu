@@ -257,8 +257,8 @@ extern "C" int nbg_run_batch(nbg_context* h, const nbg_batch_item* items, int32_
     // ---- jobs: select order grouped by class, then finish order
     // each tile's select kernel as in nbg_run (the Morton variant, 1, has no
     // batch form: the two-pass search it reorders stands in).  24 mixture tiles
-    // of 15k to 1M points, knn 8, 16 and 32: 38.5 ms when every tile took the
-    // two-pass queue, 30.5 ms with these
+    // (16.6M points, knn 8, 16 and 32): 38.5 ms when every tile took the two-pass
+    // queue, 30.5 ms with these
     std::vector<int> select(n_items, 0);
     for (int i : live) {
         Tile* t = &items[i].tile->t;
@@ -301,6 +301,9 @@ extern "C" int nbg_run_batch(nbg_context* h, const nbg_batch_item* items, int32_
         q.boxes = t->boxes;
         q.retry_rows = select[i] ? B->retry + row0[i] : nullptr;
         q.gp = t->gp;
+        q.x = t->x;
+        q.y = t->y;
+        q.z = t->z;
         q.n = t->n;
         q.K = Ks[i];
         q.rmax = 8;

@@ -105,7 +105,7 @@ struct KdOrder {
 // Exact integer neighbourhood sums of one row (offsets from the query, raw
 // units): s = {S1x, S1y, S1z, Sxx, Syx, Syy, Szx, Szy, Szz}; cnt = 0 marks a
 // row the grid path did not finish.
-struct RowSums {
+struct alignas(8) RowSums {
     int32_t s[9];
     int32_t cnt;
 };
@@ -138,17 +138,23 @@ struct QueryArgs {
     uint32_t* ids_out;   // neighbour-set export (null in the fused path)
     uint2* ties;         // tie list {id, (D_K - 2^23 bias) | R << 24}; null: ties go to exact_rows
     uint32_t tie_cap;
-    RowSums* sums;       // split form: per sorted position, read by knn_finish_kernel
+    RowSums* sums;       // split form: per point id, read by knn_finish_kernel
     const double* row_k; // covariancefeatures optimized: per-point k = OptimalKNN (null: K)
     const uint32_t* rows = nullptr;  // split form: the sorted positions to answer (null: all n)
     uint64_t nq = 0;                 // entries of `rows`
     const uint32_t* nq_dev = nullptr;  // entries of `rows` read on the device (retry launches)
     uint32_t* retry_rows = nullptr;    // group select: rows it hands to the per-thread select
     // the points the rows index: gv.sorted, or the clump order of the group
-    // select (rows, sums and retry_rows then hold its slots), with the boxes
-    // of the clumps (ClumpTree)
+    // select (rows and retry_rows then hold its slots), with the boxes of the
+    // clumps (ClumpTree)
     const float4* qpts = nullptr;
     const float* boxes = nullptr;
+    // the finish pass: the tile's raw coordinates, and the first of the nq ids
+    // when `rows` holds the positions of consecutive ids (negative: any ids)
+    const int32_t* x = nullptr;
+    const int32_t* y = nullptr;
+    const int32_t* z = nullptr;
+    int64_t id0 = -1;
 };
 
 // Bounding boxes over the clump order: clumps of 32 consecutive slots, then
@@ -270,7 +276,7 @@ __device__ __forceinline__ double nbg_pos_hypot(double x, double y) {
 
 // a: symmetric 3x3 (a00,a10,a11,a20,a21,a22 lower triangle).  Returns 1 on
 // success.  eval ascending; evec[c*3+r].
-__device__ inline int nbg_eigen_chain(const double low[6], double eval[3], double evec[9]) {
+static __device__ __noinline__ int nbg_eigen_chain_call(const double low[6], double eval[3], double evec[9]) {
     double m00 = low[0], m10 = low[1], m11 = low[2], m20 = low[3], m21 = low[4], m22 = low[5];
     double scale = fmax(fmax(fmax(fabs(m00), fabs(m10)), fmax(fabs(m11), fabs(m20))),
                         fmax(fabs(m21), fabs(m22)));
@@ -383,6 +389,21 @@ __device__ inline int nbg_eigen_chain(const double low[6], double eval[3], doubl
     eval[2] = __dmul_rn(diag[2], scale);
 #pragma unroll
     for (int i = 0; i < 9; ++i) evec[i] = Q[i];
+    return ok;
+}
+
+// A call, not inlined: few rows take the chain, and with its four copies in a
+// finish kernel the common path waited for instructions.  The arrays are
+// copied around the call, so that the caller's stay in registers.
+__device__ __forceinline__ int nbg_eigen_chain(const double low[6], double eval[3], double evec[9]) {
+    double c[6], e[3], v[9];
+#pragma unroll
+    for (int i = 0; i < 6; ++i) c[i] = low[i];
+    const int ok = nbg_eigen_chain_call(c, e, v);
+#pragma unroll
+    for (int i = 0; i < 3; ++i) eval[i] = e[i];
+#pragma unroll
+    for (int i = 0; i < 9; ++i) evec[i] = v[i];
     return ok;
 }
 

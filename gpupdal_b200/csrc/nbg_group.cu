@@ -43,8 +43,8 @@
 // Bound by instruction issue (the data lie in L2): 2.7 candidates are scanned
 // for each of the K + 1 kept, and the merges cost about as much as the scan.  Measured
 // select times at the densities of the synthetic clouds, per-thread two-pass
-// search -> this kernel: K = 65, 1.5M points, 8.9 -> 3.6 ms; K = 33, 5M
-// points of 24 tiles, 12.6 -> 7 ms.
+// search -> this kernel: K = 65, 1.5M points, 8.9 -> 3.6 ms; K = 33, 4.7M
+// points of 24 tiles, 12.6 -> 5.8 ms.
 #include <climits>
 
 #include "nbg_common.cuh"
@@ -447,7 +447,7 @@ __device__ __forceinline__ void group_warp(const QueryArgs& a, const uint64_t s0
                 const QueryCell qc{qx, qy, qz, qx / g.cell, qy / g.cell, qz / g.cell};
                 const int R = ring_for(g, qc, kk);
                 defer_row(a, id, R < 256, KEY_BASE + kk, R);
-                if (a.sums) a.sums[pos].cnt = 0;
+                if (a.sums) a.sums[id].cnt = 0;
             } else if (a.ids_out) {
                 uint32_t* row = a.ids_out + (uint64_t)id * a.K;
                 int w = 0;
@@ -486,7 +486,7 @@ __device__ __forceinline__ void group_warp(const QueryArgs& a, const uint64_t s0
                     }
                 }
                 out.cnt = K;
-                a.sums[pos] = out;
+                a.sums[id] = out;
             }
         }
         __syncwarp();
@@ -520,7 +520,7 @@ __device__ __forceinline__ void group_warp(const QueryArgs& a, const uint64_t s0
     if (retry || !done) {
         const uint32_t slot = atomicAdd(&a.counters[6], 1u);
         a.retry_rows[slot] = pos;
-        if (a.sums) a.sums[pos].cnt = 0;  // the finish pass leaves the row to the retry launch
+        if (a.sums) a.sums[id].cnt = 0;  // the finish pass leaves the row to the retry launch
     }
 }
 

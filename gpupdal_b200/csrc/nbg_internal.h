@@ -179,6 +179,7 @@ struct QueryLaunch {
     const double* row_k = nullptr;  // per-row neighbour count (optimized), device
     const uint32_t* rows = nullptr;  // split form only: sorted positions to answer (null: all)
     uint64_t nrows = 0;
+    int64_t id0 = -1;  // when `rows` are the positions of ids [id0, id0 + nrows)
     // group select (split form): rows handed back to the per-thread select
     // (capacity: the rows answered; null: the per-thread select for every row)
     uint32_t* retry_rows = nullptr;
@@ -198,11 +199,6 @@ int launch_query(Context* ctx, const QueryLaunch& q, cudaStream_t stream);
 // (With `clumps` slots of the clump order instead.)
 int build_id_chunks(Context* ctx, const Tile* t, const uint64_t* bounds, int nchunks,
                     uint32_t* rows, uint32_t* dnum, bool clumps, cudaStream_t st);
-// Select pass over a sample of `blocks` blocks of 128 rows, in runs of `run`
-// consecutive blocks whose starts are `stride` rows apart.
-int launch_select_sample(Context* ctx, const QueryLaunch& q, uint64_t stride, unsigned blocks,
-                         unsigned run, cudaStream_t stream);
-
 // Tie rows ordered on the KD replica's tree (no search replay).
 struct TieLaunch {
     const Tile* tile;

@@ -182,8 +182,8 @@ __global__ void __launch_bounds__(128) knn_fused_kernel(const QueryArgs a) {
     nbg_finish_row(a.grp, a.tf, a.ex, id, (int)n, M, qraw);
 }
 
-// Split form, pass 1 + pass 2: the row's exact neighbourhood sums, in sorted
-// order (cnt = 0 marks a row handed to the exact path).
+// Split form, pass 1 + pass 2: the row's exact neighbourhood sums, at its point
+// id (cnt = 0 marks a row handed to the exact path).
 template <int KS>
 __device__ __forceinline__ void select_row(const QueryArgs& a, const uint64_t i) {
     const GridParams g = *a.gp;
@@ -198,7 +198,7 @@ __device__ __forceinline__ void select_row(const QueryArgs& a, const uint64_t i)
         nbg_finish_row(a.grp, a.tf, a.ex, id, 0, M, qraw);
         RowSums z;
         z.cnt = 0;
-        a.sums[i] = z;
+        a.sums[id] = z;
         return;
     }
     QueryCell qc;
@@ -215,14 +215,14 @@ __device__ __forceinline__ void select_row(const QueryArgs& a, const uint64_t i)
     out.cnt = 0;
     if (!select_kth<KS>(a, g, qc, q, K, R, kk, tie)) {
         defer_row(a, id, tie, kk, R);
-        a.sums[i] = out;
+        a.sums[id] = out;
         return;
     }
     Pass2Fn f2{q.x, q.y, q.z, kk, 0, 0, 0, 0, 0, 0, 0, 0, 0, 0};
     for (int r = 0; r <= R; ++r) scan_shell(a.gv, g, qc, r, f2);
     if (f2.cnt != K) {
         defer_row(a, id, false, kk, R);
-        a.sums[i] = out;
+        a.sums[id] = out;
         return;
     }
     out.s[0] = f2.s1x;
@@ -235,7 +235,7 @@ __device__ __forceinline__ void select_row(const QueryArgs& a, const uint64_t i)
     out.s[7] = f2.szy;
     out.s[8] = f2.szz;
     out.cnt = f2.cnt;
-    a.sums[i] = out;
+    a.sums[id] = out;
 }
 
 template <int KS>
@@ -348,7 +348,7 @@ __device__ __forceinline__ void select_row_loc(const QueryArgs& a, const uint64_
     auto retry = [&]() {
         const uint32_t slot = atomicAdd(&a.counters[6], 1u);
         a.retry_rows[slot] = (uint32_t)i;
-        a.sums[i].cnt = 0;  // the finish pass leaves the row to the retry launch
+        a.sums[id].cnt = 0;  // the finish pass leaves the row to the retry launch
     };
     if (K <= 0) {
         retry();
@@ -398,7 +398,7 @@ __device__ __forceinline__ void select_row_loc(const QueryArgs& a, const uint64_
         defer_row(a, id, true, KEY_BASE + kk, R);
         RowSums z;
         z.cnt = 0;
-        a.sums[i] = z;
+        a.sums[id] = z;
         return;
     }
     int s1x = 0, s1y = 0, s1z = 0, sxx = 0, syx = 0, syy = 0, szx = 0, szy = 0, szz = 0;
@@ -435,7 +435,7 @@ __device__ __forceinline__ void select_row_loc(const QueryArgs& a, const uint64_
     out.s[7] = szy;
     out.s[8] = szz;
     out.cnt = K;
-    a.sums[i] = out;
+    a.sums[id] = out;
 }
 
 template <int KS>
@@ -468,13 +468,24 @@ __global__ void __launch_bounds__(256) knn_select_morton_kernel(const QueryArgs 
 }
 
 // Split form, finish: covariance, eigensolve and stage projections of the
-// rows the select kernel completed.  Uniform work per thread.
-__device__ __forceinline__ void finish_row(const QueryArgs& a, const uint64_t i) {
-    const RowSums r = a.sums[i];
+// rows the select kernel completed, a thread per point id.  Uniform work per
+// thread.
+//
+// In id order because the outputs and the optimal columns lie in id order:
+// the select kernels, which leave the memory idle (1 % of the DRAM rate), put
+// a row's sums (40 bytes) at its id, and everything here is read and written
+// in order.  In the select's order instead, every output of a point is a
+// sector of its own in memory, written as a read, a merge and a write back
+// wherever the ids do not follow the points' positions (4M points, 11 feature
+// columns: 1.95 ms, 65 % of it waiting for memory; the call 5.97 -> 4.57 ms).
+//
+// What is left is bound by the latency of its dependent FP32 and FP64 chains:
+// 24 warps an SM at 80 registers (some of the rare paths' values spill) beat
+// 16 at 128.  4M rows, eigenvalues and normals 0.61 -> 0.46 ms, the features
+// 0.80 -> 0.54 ms, with the Eigen chain behind a call.
+__device__ __forceinline__ void finish_row(const QueryArgs& a, const uint32_t id) {
+    const RowSums r = a.sums[id];
     if (r.cnt == 0) return;
-    const GridParams* gp = a.gp;
-    const float4 q = __ldg(&a.qpts[i]);
-    const uint32_t id = __float_as_uint(q.w);
     const long long n = r.cnt;
     long long M[6];
     M[0] = n * r.s[3] - (long long)r.s[0] * r.s[0];
@@ -483,26 +494,15 @@ __device__ __forceinline__ void finish_row(const QueryArgs& a, const uint64_t i)
     M[3] = n * r.s[6] - (long long)r.s[2] * r.s[0];
     M[4] = n * r.s[7] - (long long)r.s[2] * r.s[1];
     M[5] = n * r.s[8] - (long long)r.s[2] * r.s[2];
-    const int32_t qraw[3] = {__float2int_rz(q.x) + __ldg(&gp->minx), __float2int_rz(q.y) + __ldg(&gp->miny),
-                             __float2int_rz(q.z) + __ldg(&gp->minz)};
+    const int32_t qraw[3] = {__ldg(&a.x[id]), __ldg(&a.y[id]), __ldg(&a.z[id])};
     nbg_finish_row(a.grp, a.tf, a.ex, id, (int)n, M, qraw);
 }
 
-// Autotuning sample: runs of `run` consecutive blocks of 128 rows, run g
-// starting at row g*stride (neighbouring blocks share cells, as in a full
-// launch, so the sample sees the full launch's cache behaviour).
-template <int KS>
-__global__ void __launch_bounds__(128) knn_select_sample_kernel(const QueryArgs a, uint64_t stride,
-                                                                unsigned run) {
-    const uint64_t i = (blockIdx.x / run) * stride + (blockIdx.x % run) * 128ull + threadIdx.x;
-    if (i < a.n) select_row<KS>(a, i);
-}
-
-__global__ void __launch_bounds__(128) knn_finish_kernel(const QueryArgs a) {
+__global__ void __launch_bounds__(128, 6) knn_finish_kernel(const QueryArgs a) {
     uint64_t i = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x;
     if (i >= (a.rows ? a.nq : a.n)) return;
-    if (a.rows) i = __ldg(&a.rows[i]);
-    finish_row(a, i);
+    if (a.rows) i = a.id0 >= 0 ? (uint64_t)a.id0 + i : __float_as_uint(__ldg(&a.qpts[__ldg(&a.rows[i])]).w);
+    finish_row(a, (uint32_t)i);
 }
 
 // ---------------------------------------------------------------------------
@@ -549,7 +549,7 @@ __global__ void __launch_bounds__(128) knn_select_queue_kernel(const BatchJob* _
     }
 }
 
-__global__ void __launch_bounds__(128) knn_finish_queue_kernel(const BatchJob* __restrict__ jobs,
+__global__ void __launch_bounds__(128, 6) knn_finish_queue_kernel(const BatchJob* __restrict__ jobs,
                                                                int njobs, uint64_t items,
                                                                unsigned long long* head) {
     uint64_t item;
@@ -557,7 +557,7 @@ __global__ void __launch_bounds__(128) knn_finish_queue_kernel(const BatchJob* _
     while (next_item(jobs, njobs, items, head, item, j)) {
         const QueryArgs& a = jobs[j].q;
         const uint64_t i = (item - jobs[j].first) * 128u + threadIdx.x;
-        if (i < a.n) finish_row(a, i);
+        if (i < a.n) finish_row(a, (uint32_t)i);
     }
 }
 
@@ -1311,6 +1311,10 @@ int launch_query(Context* ctx, const QueryLaunch& ql, cudaStream_t stream) {
     la.q.rows = ql.sums ? ql.rows : nullptr;  // the fused kernel answers every row
     la.q.nq = ql.sums ? ql.nrows : 0;
     la.q.retry_rows = ql.retry_rows;
+    la.q.x = ql.tile->x;
+    la.q.y = ql.tile->y;
+    la.q.z = ql.tile->z;
+    la.q.id0 = ql.id0;
     la.stream = stream;
     if (ctx && ctx->fork) {
         la.fork = ctx->fork;
@@ -1398,51 +1402,6 @@ int build_id_chunks(Context* ctx, const Tile* t, const uint64_t* bounds, int nch
     if (!e) e = cudaStreamSynchronize(st);
     ctx_free(ctx, tmp, std::max<size_t>(tmp_bytes, 16));
     return e ? fail(ctx, NBG_ERR_CUDA, std::string("row chunks: ") + cudaGetErrorString(e)) : NBG_OK;
-}
-
-struct SampleArgs {
-    QueryArgs q;
-    uint64_t stride;
-    unsigned blocks;
-    unsigned run;
-    cudaStream_t stream;
-};
-
-template <int KS>
-struct SampleLauncher {
-    using Args = SampleArgs;
-    static int run(const SampleArgs& s) {
-        if (!s.blocks) return NBG_OK;
-        knn_select_sample_kernel<KS><<<s.blocks, 128, 0, s.stream>>>(s.q, s.stride, s.run);
-        NBG_LAUNCHED(1);
-        return cudaGetLastError() == cudaSuccess ? NBG_OK : NBG_ERR_CUDA;
-    }
-};
-
-int launch_select_sample(Context* ctx, const QueryLaunch& ql, uint64_t stride, unsigned blocks,
-                         unsigned run, cudaStream_t stream) {
-    (void)ctx;
-    SampleArgs s{};
-    s.q.gv = grid_view(ql.tile);
-    s.q.qpts = ql.tile->sorted;
-    s.q.gp = ql.tile->gp;
-    s.q.n = ql.tile->n;
-    s.q.K = ql.K;
-    s.q.rmax = ql.rmax;
-    s.q.grp = ql.grp;
-    s.q.tf = ql.tile->tf;
-    s.q.ex = ql.ex;
-    s.q.exact_rows = ql.exact_rows;
-    s.q.counters = ql.counters;
-    s.q.ties = ql.ties;
-    s.q.tie_cap = ql.tie_cap;
-    s.q.sums = ql.sums;
-    s.q.row_k = ql.row_k;
-    s.stride = stride;
-    s.blocks = blocks;
-    s.run = std::max(1u, run);
-    s.stream = stream;
-    return dispatch_slots<SampleLauncher>(ql.K, s);
 }
 
 int launch_select_queue(Context* ctx, int K, const BatchJob* jobs, int njobs, uint64_t items,
