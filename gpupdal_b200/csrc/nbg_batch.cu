@@ -11,7 +11,7 @@
 //              and the launches are captured in a CUDA graph, replayed while the
 //              batch's job arrays and counts are unchanged.
 // 3. replicas  the tiles' KD replicas, all as one forest (one level-synchronous
-//              build for every tile), once the queue has drained
+//              build for every tile), beside the queue
 // 4. exact     per tile: the tie-order resolver, then the search replay for
 //              the rows it hands on, as in nbg_run
 // Each tile owns disjoint slices of the row-sum, tie and replay lists and
@@ -220,14 +220,35 @@ extern "C" int nbg_run_batch(nbg_context* h, const nbg_batch_item* items, int32_
     // ---- grids (no host synchronisation), then one read of every shape
     cudaEventRecord(B->ev[0], user);
     cudaStreamWaitEvent(st, B->ev[0], 0);
+    // A tile's build is a chain of launches too short to fill the GPU: tiles in
+    // turn on three streams, which `st` joins (24 tiles: 3.1 -> 2.1 ms)
+    cudaStream_t lanes[3] = {st, ctx->side, ctx->fork};
+    auto open_lanes = [&]() {
+        cudaEventRecord(ctx->fev[0], st);
+        cudaStreamWaitEvent(ctx->side, ctx->fev[0], 0);
+        cudaStreamWaitEvent(ctx->fork, ctx->fev[0], 0);
+    };
+    auto join_lanes = [&]() {
+        cudaEventRecord(ctx->fev[1], ctx->side);
+        cudaEventRecord(ctx->fev[2], ctx->fork);
+        cudaStreamWaitEvent(st, ctx->fev[1], 0);
+        cudaStreamWaitEvent(st, ctx->fev[2], 0);
+    };
+    int turn = 0;
+    open_lanes();
     for (int i : live) {
         Tile* t = &items[i].tile->t;
         if (t->grid_valid && t->grid_fixed == t->fixed_cell &&
             (t->fixed_cell || (Ks[i] <= 2 * t->grid_k1 && 2 * Ks[i] >= t->grid_k1)))
             continue;
         t->grid_valid = false;
-        rc = build_grid_async(ctx, t, Ks[i], st);
-        if (rc) return fail(ctx, rc, "grid build failed");
+        rc = build_grid_async(ctx, t, Ks[i], lanes[turn++ % 3]);
+        if (rc) break;
+    }
+    join_lanes();
+    if (rc) {
+        cudaStreamSynchronize(st);
+        return fail(ctx, rc, "grid build failed");
     }
     std::vector<GridParams> gps(nl);
     for (int j = 0; j < nl; ++j)
@@ -260,14 +281,20 @@ extern "C" int nbg_run_batch(nbg_context* h, const nbg_batch_item* items, int32_
     // (16.6M points, knn 8, 16 and 32): 38.5 ms when every tile took the two-pass
     // queue, 30.5 ms with these
     std::vector<int> select(n_items, 0);
+    open_lanes();
     for (int i : live) {
         Tile* t = &items[i].tile->t;
         const int k = B->retry_cap ? select_kernel(t, Ks[i], false) : 0;
         select[i] = k >= 8 && t->clumps ? 32 : (k == 2 && slots_for_k(Ks[i]) <= 18 ? 2 : 0);
         if (select[i] == 32) {
-            rc = ensure_clumps(ctx, t, st);
-            if (rc) return fail(ctx, rc, "clump order");
+            rc = ensure_clumps(ctx, t, lanes[turn++ % 3]);
+            if (rc) break;
         }
+    }
+    join_lanes();
+    if (rc) {
+        cudaStreamSynchronize(st);
+        return fail(ctx, rc, "clump order");
     }
     auto class_of = [&](int i) { return slots_for_k(Ks[i]) * 64 + select[i]; };
     std::vector<int> order(live);
@@ -381,13 +408,20 @@ extern "C" int nbg_run_batch(nbg_context* h, const nbg_batch_item* items, int32_
             if (r) return r;
         }
         // rows handed back (their sums slots hold 0: the finish pass skips them)
-        for (const Cls& c : classes) {
-            if (!c.select) continue;
-            const int r = launch_retry_batch(slots_for_k(c.K), B->jobs + c.begin, c.count, ctx->sm_count, s);
-            if (r) return r;
-        }
-        return launch_finish_queue(ctx, B->jobs + nl, nl, fin_items, B->heads + classes.size(), s,
-                                   reserve);
+        // on the fork stream, queued first: long searches, beside the finish pass
+        // (2.2 of 5.7 ms of both, 24 tiles)
+        cudaError_t e = cudaEventRecord(ctx->fev[0], s);
+        if (!e) e = cudaStreamWaitEvent(ctx->fork, ctx->fev[0], 0);
+        if (e) return NBG_ERR_CUDA;
+        int r = NBG_OK;
+        for (const Cls& c : classes)
+            if (c.select && !r)
+                r = launch_retry_batch(slots_for_k(c.K), B->jobs + c.begin, c.count, ctx->sm_count, ctx->fork);
+        if (!r)
+            r = launch_finish_queue(ctx, B->jobs + nl, nl, fin_items, B->heads + classes.size(), s, reserve);
+        e = cudaEventRecord(ctx->fev[1], ctx->fork);
+        if (!e) e = cudaStreamWaitEvent(s, ctx->fev[1], 0);
+        return r ? r : e ? NBG_ERR_CUDA : NBG_OK;
     };
     const bool graph = (flags & NBG_BATCH_GRAPH) != 0;
     if (graph && (!B->exec || B->key != key)) {
@@ -413,26 +447,27 @@ extern "C" int nbg_run_batch(nbg_context* h, const nbg_batch_item* items, int32_
         }
         B->key = key;
     }
-    // ---- the queue on st, then the KD replicas of its tiles as one forest.
-    // The forest's level passes are many short launches with host
-    // synchronisations between levels: beside the persistent queue kernels,
-    // which hold every resident block slot, each waited for free slots (the
-    // forest of 256 tiles took longer than the queue itself); after the queue
-    // they have the whole GPU.
+    // ---- the queue on st and, beside it on the side stream, the KD replicas of
+    // its tiles as one forest: the select passes leave the memory idle, and the
+    // side stream's priority gives the build's short launches the block slots
+    // they wait for (after the queue -> beside it: 24 tiles of 16.6M points 26.6
+    // -> 25.3 ms, 72 tiles 49.0 -> 47.1 ms)
     cudaEventRecord(B->ev[2], st);
-    int qrc = graph ? (cudaGraphLaunch(B->exec, st) == cudaSuccess ? NBG_OK : NBG_ERR_CUDA) : record(st);
+    cudaEventRecord(ctx->xev[0], st);
+    cudaStreamWaitEvent(ctx->side, ctx->xev[0], 0);
+    const int qrc = graph ? (cudaGraphLaunch(B->exec, st) == cudaSuccess ? NBG_OK : NBG_ERR_CUDA) : record(st);
     cudaEventRecord(B->ev[3], st);
-    cudaError_t qe = cudaStreamSynchronize(st);
-    if (qrc || qe != cudaSuccess) return fail(ctx, NBG_ERR_CUDA, "batch queue launch failed");
     float kd_ms = 0;
-    if (!kd_tiles.empty()) {
-        cudaEventRecord(ctx->ev[8], st);
-        rc = kd_ensure_many(ctx, kd_tiles.data(), (int)kd_tiles.size(), st);
-        if (rc) return rc;
-        cudaEventRecord(ctx->ev[9], st);
-        if (cudaStreamSynchronize(st) != cudaSuccess) return fail(ctx, NBG_ERR_CUDA, "batch KD replicas");
-        cudaEventElapsedTime(&kd_ms, ctx->ev[8], ctx->ev[9]);
+    if (!qrc && !kd_tiles.empty()) {
+        cudaEventRecord(ctx->ev[8], ctx->side);
+        rc = kd_ensure_many(ctx, kd_tiles.data(), (int)kd_tiles.size(), ctx->side);
+        cudaEventRecord(ctx->ev[9], ctx->side);
+        if (cudaStreamSynchronize(ctx->side) != cudaSuccess && !rc) rc = fail(ctx, NBG_ERR_CUDA, "batch KD replicas");
+        if (!rc) cudaEventElapsedTime(&kd_ms, ctx->ev[8], ctx->ev[9]);
     }
+    const cudaError_t qe = cudaStreamSynchronize(st);
+    if (qrc || qe != cudaSuccess) return fail(ctx, NBG_ERR_CUDA, "batch queue launch failed");
+    if (rc) return rc;
     // ---- exact rows per tile
     std::vector<uint32_t> cnt((size_t)nl * kCounters);
     cudaMemcpyAsync(cnt.data(), B->counters, cnt.size() * 4, cudaMemcpyDeviceToHost, st);
