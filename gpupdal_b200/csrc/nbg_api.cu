@@ -38,12 +38,6 @@ static int cuda_fail(Context* c, cudaError_t e, const char* what) {
     return fail(c, NBG_ERR_CUDA, std::string(what) + ": " + cudaGetErrorString(e));
 }
 
-#define NBG_TRY(call, what)                               \
-    do {                                                  \
-        cudaError_t e__ = (call);                         \
-        if (e__ != cudaSuccess) return cuda_fail(ctx, e__, what); \
-    } while (0)
-
 std::atomic<uint64_t> g_launches{0};
 
 static size_t round_bytes(size_t bytes) { return bytes == 0 ? 256 : ((bytes + 255) / 256) * 256; }
@@ -598,12 +592,19 @@ int ensure_grid(Context* ctx, Tile* t, int k1, cudaStream_t stream, int32_t cell
         return NBG_OK;
     const int32_t saved = t->fixed_cell;
     t->fixed_cell = fixed;
-    int rc = build_grid(ctx, t, k1, stream);
+    bool small = grid_small(t);
+    int rc = NBG_OK;
+    for (;;) {
+        rc = small ? build_grid_small(ctx, t, k1, stream) : build_grid(ctx, t, k1, stream);
+        cudaError_t e = cudaSuccess;
+        if (!rc) e = cudaMemcpyAsync(&t->host_gp, t->gp, sizeof(GridParams), cudaMemcpyDeviceToHost, stream);
+        if (!rc && !e) e = cudaStreamSynchronize(stream);
+        if (e) rc = NBG_ERR_CUDA;
+        if (rc || !small || !(t->host_gp.cap_hit & 2u)) break;
+        small = false;  // more cells than one block should walk
+    }
     t->fixed_cell = saved;
     if (rc) return fail(ctx, rc, "grid build failed");
-    NBG_TRY(cudaMemcpyAsync(&t->host_gp, t->gp, sizeof(GridParams), cudaMemcpyDeviceToHost, stream),
-            "grid params");
-    NBG_TRY(cudaStreamSynchronize(stream), "grid build");
     const GridParams& g = t->host_gp;
     if ((int64_t)g.maxx - g.minx >= (1 << 24) || (int64_t)g.maxy - g.miny >= (1 << 24) ||
         (int64_t)g.maxz - g.minz >= (1 << 24))

@@ -242,7 +242,8 @@ extern "C" int nbg_run_batch(nbg_context* h, const nbg_batch_item* items, int32_
             (t->fixed_cell || (Ks[i] <= 2 * t->grid_k1 && 2 * Ks[i] >= t->grid_k1)))
             continue;
         t->grid_valid = false;
-        rc = build_grid_async(ctx, t, Ks[i], lanes[turn++ % 3]);
+        cudaStream_t lane = lanes[turn++ % 3];
+        rc = grid_small(t) ? build_grid_small(ctx, t, Ks[i], lane) : build_grid_async(ctx, t, Ks[i], lane);
         if (rc) break;
     }
     join_lanes();

@@ -153,6 +153,9 @@ int build_grid(Context* ctx, Tile* t, int k1, cudaStream_t stream);
 // Grid for neighbour count k1 (or a fixed cell edge), rebuilt only when needed.
 int ensure_grid(Context* ctx, Tile* t, int k1, cudaStream_t stream, int32_t cell = 0);
 int build_grid_async(Context* ctx, Tile* t, int k1, cudaStream_t stream);
+// The same in one launch, for the tiles grid_small names.
+bool grid_small(const Tile* t);
+int build_grid_small(Context* ctx, Tile* t, int k1, cudaStream_t stream);
 
 int fail(Context* c, int code, const std::string& msg);
 // Sets the context's error message (thread-safe).
