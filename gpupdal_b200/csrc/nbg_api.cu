@@ -1253,7 +1253,7 @@ extern "C" int nbg_run(nbg_context* h, nbg_tile* th, const nbg_stage_opts* stage
             cudaEventRecord(ctx->xev[1], ctx->side);
             cudaStreamWaitEvent(stream, ctx->xev[1], 0);
         }
-        // With the single-pass select the tie list is complete once its
+        // With the selects that fork the tie list is complete once their
         // handed-back rows are answered on the fork stream: the tie rows are
         // ordered there (count read on the device) beside the finish pass
         // instead of after it.

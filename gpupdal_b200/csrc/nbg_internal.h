@@ -66,8 +66,8 @@ struct Context {
     // query kernels run on the caller's stream
     cudaStream_t side = nullptr;
     cudaEvent_t xev[2];
-    // normal-priority stream for the single-pass select's handed-back rows,
-    // answered beside the finish pass of the other rows (fev: fork and join)
+    // normal-priority stream for the rows the single-pass and group selects hand
+    // back, answered beside the finish pass of the other rows (fev: fork and join)
     cudaStream_t fork = nullptr;
     cudaEvent_t fev[4];
     // device blocks released by earlier calls, kept for reuse by size
@@ -183,14 +183,14 @@ struct QueryLaunch {
     const uint32_t* rows = nullptr;  // split form only: sorted positions to answer (null: all)
     uint64_t nrows = 0;
     int64_t id0 = -1;  // when `rows` are the positions of ids [id0, id0 + nrows)
-    // group select (split form): rows handed back to the per-thread select
-    // (capacity: the rows answered; null: the per-thread select for every row)
+    // single-pass and group selects (split form): the rows they hand back
+    // (capacity: the rows answered; null: the two-pass select for every row)
     uint32_t* retry_rows = nullptr;
     int group = 0;
     float margin0 = 0.25f;
     // when set, the launch records `done` once every row is answered and
-    // leaves `stream` free for the next launch (the single-pass select's
-    // handed-back rows may still run on the context's fork stream); when
+    // leaves `stream` free for the next launch (handed-back rows may still run
+    // on the context's fork stream); when
     // null, every row is answered in `stream` order
     cudaEvent_t done = nullptr;
 };

@@ -1329,7 +1329,7 @@ int launch_query(Context* ctx, const QueryLaunch& ql, cudaStream_t stream) {
     la.sms = ctx ? ctx->sm_count : 148;
     la.ob = loc_offset_bits(ql.tile->host_gp.cell);
     const int rc = dispatch_slots<KnnLauncher>(ql.K, la);
-    // the forked single-pass launch records `done` itself, on the fork stream
+    // a forked launch records `done` itself, on the fork stream
     if (!rc && ql.done && !query_forks(ctx, ql) && cudaEventRecord(ql.done, stream) != cudaSuccess)
         return NBG_ERR_CUDA;
     return rc;

@@ -333,10 +333,10 @@ class Tile:
                                                    int(fixed_cell)))
 
     def set_select(self, kernel=0, first_margin=0.5):
-        """Select kernel (nbg_tile_set_select): 0 two-pass ring search
-        (default), 1 the same in block-local Morton order, 2 single-pass ring
-        search, 8 / 16 / 32 queries sharing one candidate list; results are
-        identical."""
+        """Select kernel (nbg_tile_set_select): 0 two-pass ring search, 1 the
+        same in block-local Morton order, 2 single-pass ring search, 8 / 16 / 32
+        queries sharing one candidate list; results are identical.  A tile
+        left alone takes the library's choice of 0, 2 and 32."""
         self.ctx._check(self.ctx.lib.nbg_tile_set_select(self.ctx.h, self.h, int(kernel),
                                                          float(first_margin)))
 
