@@ -84,7 +84,6 @@ struct StageGroup {
     const double* optimal_knn;     // device, may be null
     const double* optimal_radius;  // device, may be null
     uint32_t* resolve_count;       // rows the fast eigensolver handed to the chain (may be null)
-    int32_t no_eigen;              // every stage reads the neighbour count only
 };
 
 // The KD replica's nodes as the tie-order resolver reads them: a child's
@@ -589,7 +588,6 @@ __device__ inline void nbg_finish_row_d(const StageGroup& g, const Transform& tf
     if (nnb == 0) zero = true;
     double ev[3] = {0, 0, 0}, V[9] = {0, 0, 0, 0, 0, 0, 0, 0, 0};
     int ok = 1;
-    if (g.no_eigen) zero = true;
     if (!zero) {
         if (nonfinite) ok = 0;
         else if (g.sign_exact) ok = nbg_eigen_chain(C, ev, V);
@@ -672,11 +670,6 @@ __device__ inline void nbg_finish_row_d(const StageGroup& g, const Transform& tf
             const double smax = fmax(a0, fmax(a1, a2));
             const double thr = fmax(smax * (double)(float)st.t1, 2.2250738585072014e-308);
             nbg_store(st, id, 0, (double)((a0 >= thr) + (a1 >= thr) + (a2 >= thr)));
-        } else if (st.kind == NBG_STAGE_OUTLIER) {
-            // OutlierFilter.cpp:80-96: an inlier has more than size_t(min_k)
-            // points (itself included) within the radius; a negative min_k
-            // converts to a count no row exceeds
-            st.aux[id] = (st.ip >= 0 && nnb > st.ip) ? 0.0 : 1.0;
         } else if (st.kind == NBG_STAGE_EIGENVALUES) {
             if (zero) { nbg_append_exception(ex, id, sidx, NBG_ROW_ZERO_COV); continue; }
             if (!ok) { nbg_append_exception(ex, id, sidx, NBG_ROW_EIGEN_FAIL); continue; }

@@ -244,7 +244,6 @@ int run_consumer(Context* ctx, Tile* t, const nbg_stage_opts& o, int stage_index
         g.st[0] = st;
         g.st[0].aux = flag;
         g.st[0].ip = o.min_k;
-        g.no_eigen = 1;
         RadiusLaunch rl;
         rl.tile = t;
         rl.grp = g;

@@ -1005,6 +1005,8 @@ __global__ void __launch_bounds__(128) knn_stride_kernel(const StrideArgs sa) {
 // rounding of the coordinates) is dropped; every other candidate is tested
 // with the reference's FP64 distance.  Sums are int64 (exact while the
 // neighbourhood's sum of squared offsets stays below 2^63 raw units^2).
+// With COUNT only the number of points is kept (what the outlier flag reads).
+template <bool COUNT>
 struct RadiusFn {
     float qx, qy, qz;
     int32_t qraw[3];
@@ -1029,6 +1031,8 @@ struct RadiusFn {
             acc = __dadd_rn(acc, __dmul_rn(df, df));
         }
         if (!(acc < rr)) return;
+        ++cnt;
+        if constexpr (COUNT) return;
         s1x += ix;
         s1y += iy;
         s1z += iz;
@@ -1038,7 +1042,6 @@ struct RadiusFn {
         szx += (long long)iz * ix;
         szy += (long long)iz * iy;
         szz += (long long)iz * iz;
-        ++cnt;
     }
 };
 
@@ -1059,6 +1062,10 @@ __device__ __forceinline__ double m_entry(long long n, long long sab, long long 
     return (double)((__int128)n * sab - (__int128)sa * sb);
 }
 
+// Bound by the latency of the scan's loads and divergent loops: the counting
+// form without the sums, the covariance and the eigensolve holds few registers
+// and keeps more warps in flight (4M mixture points, radius 1: 2.48 -> 1.41 ms).
+template <bool COUNT>
 __global__ void __launch_bounds__(128) knn_radius_kernel(const RadiusArgs a) {
     const uint64_t i = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x;
     if (i >= a.n) return;
@@ -1072,7 +1079,7 @@ __global__ void __launch_bounds__(128) knn_radius_kernel(const RadiusArgs a) {
     qc.cx = qc.qx / g.cell;
     qc.cy = qc.qy / g.cell;
     qc.cz = qc.qz / g.cell;
-    RadiusFn f;
+    RadiusFn<COUNT> f;
     f.qx = q.x;
     f.qy = q.y;
     f.qz = q.z;
@@ -1091,6 +1098,13 @@ __global__ void __launch_bounds__(128) knn_radius_kernel(const RadiusArgs a) {
     if (st.kind != NBG_STAGE_NORMAL && (long long)f.cnt < (long long)a.min_k) {
         nbg_append_exception(a.ex, id, a.grp.stage_index[0], NBG_ROW_RADIUS_FEW,
                              (uint16_t)min(f.cnt, 65535u));
+        return;
+    }
+    if constexpr (COUNT) {
+        // OutlierFilter.cpp:80-96: an inlier has more than size_t(min_k) points
+        // (itself included) within the radius; a negative min_k converts to a
+        // count no row exceeds
+        st.aux[id] = (st.ip >= 0 && (int)min(f.cnt, 0x7FFFFFFFu) > st.ip) ? 0.0 : 1.0;
         return;
     }
     const long long n = f.cnt;
@@ -1117,7 +1131,9 @@ int launch_radius(Context* ctx, const RadiusLaunch& rl, cudaStream_t stream) {
     a.dout = rr_raw > 0.0 ? (unsigned long long)ceil(rr_raw * (1.0 + 1e-5)) + 2ull : 0ull;
     a.r_raw = sqrt((double)a.dout);
     a.min_k = rl.min_k;
-    knn_radius_kernel<<<(unsigned)((t->n + 127) / 128), 128, 0, stream>>>(a);
+    const unsigned blocks = (unsigned)((t->n + 127) / 128);
+    if (rl.grp.st[0].kind == NBG_STAGE_OUTLIER) knn_radius_kernel<true><<<blocks, 128, 0, stream>>>(a);
+    else knn_radius_kernel<false><<<blocks, 128, 0, stream>>>(a);
     NBG_LAUNCHED(1);
     return cudaGetLastError() == cudaSuccess ? NBG_OK : NBG_ERR_CUDA;
 }
