@@ -801,6 +801,7 @@ static int run_pipelined(Context* ctx, Tile* t, int K, int select, const StageGr
             tl.ex = sink;
             tl.ties = ctx->ties + b[c];
             tl.nties = nties;
+            tl.of_rows = rows_c;
             tl.kd = kd_order(t);
             tl.exact_rows = ctx->exact_rows + b[c];
             tl.counters = cnt_dev;

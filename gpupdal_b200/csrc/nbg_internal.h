@@ -210,6 +210,7 @@ struct TieLaunch {
     ExceptionSink ex;
     const uint2* ties;
     uint32_t nties;
+    uint64_t of_rows = 0;  // rows of the query that listed them (0: the tile's)
     KdOrder kd;
     uint32_t* exact_rows;  // rows the resolver hands to the search replay
     uint32_t* counters;

@@ -670,20 +670,32 @@ __global__ void __launch_bounds__(128) knn_retry_kernel(const QueryArgs a) {
 struct TieFn {
     float qx, qy, qz;
     uint32_t kk;
-    int less;
+    int s1x, s1y, s1z, sxx, syx, syy, szx, szy, szz, less;
     int gcnt;
     uint32_t gid[TIE_CAP];
     int gd[TIE_CAP][3];
-    uint32_t* row;  // ids of the strictly closer points
+    uint32_t* row;  // neighbour-set export: ids of the strictly closer points
     int K;
     __device__ __forceinline__ unsigned long long limit() const {
         return (unsigned long long)(kk - KEY_BASE);
+    }
+    __device__ __forceinline__ void add(int ix, int iy, int iz) {
+        s1x += ix;
+        s1y += iy;
+        s1z += iz;
+        sxx += ix * ix;
+        syx += iy * ix;
+        syy += iy * iy;
+        szx += iz * ix;
+        szy += iz * iy;
+        szz += iz * iz;
     }
     __device__ __forceinline__ void operator()(const float4 p) {
         const float dx = p.x - qx, dy = p.y - qy, dz = p.z - qz;
         const uint32_t key = dist_key(dx, dy, dz);
         if (key < kk) {
-            if (less < K) row[less] = __float_as_uint(p.w);
+            add(small_int(dx), small_int(dy), small_int(dz));
+            if (row && less < K) row[less] = __float_as_uint(p.w);
             ++less;
         } else if (key == kk) {
             if (gcnt < TIE_CAP) {
@@ -697,9 +709,9 @@ struct TieFn {
     }
 };
 
-// One tie row r of a.ties, one thread: the neighbour-set export, which needs
-// the members' order (rows that only need sums: warp_tie).
-__device__ __forceinline__ void tie_ids_row(const TieArgs& a, uint32_t r) {
+// One tie row r of a.ties by one thread: the neighbour-set export, and the sums
+// where tie rows are many (many_ties, nbg_rows.cu; where they are few: warp_tie).
+__device__ __forceinline__ void tie_row(const TieArgs& a, uint32_t r) {
     const uint2 e = a.ties[r];
     const uint32_t id = e.x;
     const uint32_t kk = KEY_BASE + (e.y & 0xFFFFFFu);
@@ -719,9 +731,10 @@ __device__ __forceinline__ void tie_ids_row(const TieArgs& a, uint32_t r) {
     f.qy = (float)qc.qy;
     f.qz = (float)qc.qz;
     f.kk = kk;
+    f.s1x = f.s1y = f.s1z = f.sxx = f.syx = f.syy = f.szx = f.szy = f.szz = 0;
     f.less = 0;
     f.gcnt = 0;
-    f.row = a.ids_out + (uint64_t)id * a.K;
+    f.row = a.ids_out ? a.ids_out + (uint64_t)id * a.K : nullptr;
     f.K = K;
     for (int ring = 0; ring <= R; ++ring) scan_shell(a.gv, g, qc, ring, f);
     const int m = K - f.less;
@@ -745,36 +758,110 @@ __device__ __forceinline__ void tie_ids_row(const TieArgs& a, uint32_t r) {
         }
         d64[t] = acc;
     }
-    // members at equal FP64 distance are taken in the search's visiting order
+    // Members at equal FP64 distance are taken in the search's visiting order.
+    // Without a neighbour-id export only their offsets reach the sums: when every
+    // member at the m-th smallest FP64 distance has the same offsets (duplicate
+    // points, most of a lidar tile's tie groups), any of them gives the same
+    // sums, and the row needs no walk down the tree.  (The test is per row: a
+    // member skipped as "equivalent" in a pairwise walk would stand in for its
+    // twin in later comparisons with the other members and break the order.)
+    bool any_order = f.row == nullptr;
+    if (any_order) {
+        double v = 0.0;  // the m-th smallest FP64 distance
+        for (int t = 0; t < f.gcnt; ++t) {
+            int less = 0, le = 0;
+            for (int u = 0; u < f.gcnt; ++u) {
+                less += d64[u] < d64[t];
+                le += d64[u] <= d64[t];
+            }
+            if (less < m && m <= le) v = d64[t];
+        }
+        int ref = -1;
+        for (int t = 0; t < f.gcnt && any_order; ++t) {
+            if (d64[t] != v) continue;
+            if (ref < 0) ref = t;
+            else if (f.gd[t][0] != f.gd[ref][0] || f.gd[t][1] != f.gd[ref][1] ||
+                     f.gd[t][2] != f.gd[ref][2])
+                any_order = false;
+        }
+    }
     uint32_t taken = 0;
     for (int j = 0; j < m; ++j) {
         int best = -1;
         for (int t = 0; t < f.gcnt; ++t) {
             if ((taken >> t) & 1u) continue;
             if (best < 0 || d64[t] < d64[best] ||
-                (d64[t] == d64[best] &&
+                (d64[t] == d64[best] && !any_order &&
                  kd_meets_first(a.kd, q64, __ldg(&a.kd.kpos[a.kd.base + f.gid[t]]),
                                 __ldg(&a.kd.kpos[a.kd.base + f.gid[best]]))))
                 best = t;
         }
         taken |= 1u << best;
-        f.row[f.less + j] = f.gid[best];
+        f.add(f.gd[best][0], f.gd[best][1], f.gd[best][2]);
+        if (f.row) f.row[f.less + j] = f.gid[best];
     }
-    uint32_t* row = f.row;
-    for (int s = 1; s < K; ++s) {
-        const uint32_t v = row[s];
-        int t = s - 1;
-        while (t >= 0 && row[t] > v) {
-            row[t + 1] = row[t];
-            --t;
+    if (f.row) {
+        uint32_t* row = f.row;
+        for (int s = 1; s < K; ++s) {
+            const uint32_t v = row[s];
+            int t = s - 1;
+            while (t >= 0 && row[t] > v) {
+                row[t + 1] = row[t];
+                --t;
+            }
+            row[t + 1] = v;
         }
-        row[t + 1] = v;
+        return;
     }
+    const long long n = K;
+    long long M[6];
+    M[0] = n * f.sxx - (long long)f.s1x * f.s1x;
+    M[1] = n * f.syx - (long long)f.s1y * f.s1x;
+    M[2] = n * f.syy - (long long)f.s1y * f.s1y;
+    M[3] = n * f.szx - (long long)f.s1z * f.s1x;
+    M[4] = n * f.szy - (long long)f.s1z * f.s1y;
+    M[5] = n * f.szz - (long long)f.s1z * f.s1z;
+    nbg_finish_row(a.grp, a.tf, a.ex, id, (int)n, M, qraw);
 }
 
-__global__ void __launch_bounds__(128) knn_tie_ids_kernel(const TieArgs a) {
-    const uint32_t r = blockIdx.x * blockDim.x + threadIdx.x;
-    if (r < a.nties) tie_ids_row(a, r);
+// A thread per tie row (the count as in knn_tie_kernel).  With `least` the launch
+// stands beside that of the warp form, and the one whose range holds the count
+// answers the rows.
+__global__ void __launch_bounds__(128) knn_tie_thread_kernel(const TieArgs a, const uint32_t* count, uint32_t least) {
+    const uint32_t nt = count ? min(*count, a.nties) : a.nties;
+    if (nt < least) return;
+    for (uint32_t r = blockIdx.x * blockDim.x + threadIdx.x; r < nt; r += gridDim.x * blockDim.x) tie_row(a, r);
+}
+
+// The same over many tiles: jobs[j]'s rows are entries first[j] .. first[j+1]-1
+// of the launch.
+__global__ void __launch_bounds__(128) knn_tie_thread_batch_kernel(const TieArgs* __restrict__ jobs,
+                                                                   const uint64_t* __restrict__ first, int njobs) {
+    const uint64_t t = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x;
+    if (t >= first[njobs]) return;
+    int lo = 0, hi = njobs;  // the job whose range holds t
+    while (hi - lo > 1) {
+        const int mid = (lo + hi) >> 1;
+        if (first[mid] <= t) lo = mid;
+        else hi = mid;
+    }
+    tie_row(jobs[lo], (uint32_t)(t - first[lo]));
+}
+
+int launch_tie_threads(const TieArgs& a, const uint32_t* count, uint32_t least, int sms, cudaStream_t stream) {
+    // (a count read on the device may be far below the capacity: rows in strides)
+    const uint64_t all = ((uint64_t)a.nties + 127) / 128;
+    const unsigned blocks = (unsigned)(count ? std::min<uint64_t>(all, (uint64_t)sms * 16) : all);
+    knn_tie_thread_kernel<<<blocks, 128, 0, stream>>>(a, count, least);
+    NBG_LAUNCHED(1);
+    return cudaGetLastError() == cudaSuccess ? NBG_OK : NBG_ERR_CUDA;
+}
+
+int launch_tie_threads_batch(const TieArgs* jobs, const uint64_t* first, int njobs, uint64_t rows,
+                             cudaStream_t stream) {
+    knn_tie_thread_batch_kernel<<<(unsigned)((rows + 127) / 128), 128, 0, stream>>>(jobs, first, njobs);
+    NBG_LAUNCHED(1);
+    return cudaGetLastError() == cudaSuccess ? NBG_OK : NBG_ERR_CUDA;
 }
 
 static TieArgs tie_args(const TieLaunch& tl) {
@@ -792,6 +879,7 @@ static TieArgs tie_args(const TieLaunch& tl) {
     a.ex = tl.ex;
     a.ties = tl.ties;
     a.nties = tl.nties;
+    a.of_rows = tl.of_rows ? tl.of_rows : tl.tile->n;
     a.kd = tl.kd;
     a.exact_rows = tl.exact_rows;
     a.counters = tl.counters;
@@ -810,10 +898,7 @@ int launch_ties(Context* ctx, const TieLaunch& tl, cudaStream_t stream) {
 
 int launch_ties_counted(Context* ctx, const TieLaunch& tl, const uint32_t* count, cudaStream_t stream) {
     if (!tl.nties) return NBG_OK;
-    if (!tl.ids_out) return launch_tie_rows(tie_args(tl), count, ctx ? ctx->sm_count : 148, stream);
-    knn_tie_ids_kernel<<<(tl.nties + 127) / 128, 128, 0, stream>>>(tie_args(tl));
-    NBG_LAUNCHED(1);
-    return cudaGetLastError() == cudaSuccess ? NBG_OK : NBG_ERR_CUDA;
+    return launch_tie_rows(tie_args(tl), count, ctx ? ctx->sm_count : 148, stream);
 }
 
 int launch_ties_many(Context* ctx, const TieLaunch* tls, int count, cudaStream_t stream) {

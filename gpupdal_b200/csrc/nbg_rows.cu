@@ -12,7 +12,8 @@
 //                     the lanes and merged into the sorted list the lanes hold
 //   tie rows          strictly closer points are summed; a member of the group at
 //                     the K-th distance goes to the lane of its number, and every
-//                     lane ranks its member by (FP64 distance, visiting order)
+//                     lane ranks its member by (FP64 distance, visiting order);
+//                     a tile whose ties are many gives a thread each (many_ties)
 // The FP64 epilogue of a row is not warp work: a warp answers up to 32 rows,
 // keeps row j's sums in lane j, and then every lane finishes its own row.
 #include <algorithm>
@@ -432,9 +433,10 @@ __device__ __forceinline__ void warp_tie_rows(const TieArgs& a, uint32_t r0, uin
 }
 
 // Tie rows counted on the device (a.nties: the list's capacity), or a.nties
-// rows when `count` is null.
-__global__ void __launch_bounds__(kRowThreads) knn_tie_kernel(const TieArgs a, const uint32_t* count) {
+// rows when `count` is null; `most` rows or more are left to the thread form.
+__global__ void __launch_bounds__(kRowThreads) knn_tie_kernel(const TieArgs a, const uint32_t* count, uint32_t most) {
     const uint32_t nt = count ? min(*count, a.nties) : a.nties;
+    if (nt >= most) return;
     const uint32_t rpw = rows_per_warp(nt);
     const uint32_t warp = (blockIdx.x * blockDim.x + threadIdx.x) >> 5, warps = gridDim.x * (blockDim.x >> 5);
     for (uint32_t r0 = warp * rpw; r0 < nt; r0 += warps * rpw) warp_tie_rows(a, r0, min(rpw, nt - r0));
@@ -462,6 +464,22 @@ __global__ void __launch_bounds__(kRowThreads) knn_tie_batch_kernel(const TieArg
 // ---- launches -----------------------------------------------------------------
 static constexpr uint64_t kRowBlocksPerSm = 16;
 
+// nbg_query.cu: a thread per row
+int launch_tie_threads(const TieArgs& a, const uint32_t* count, uint32_t least, int sms, cudaStream_t stream);
+int launch_tie_threads_batch(const TieArgs* jobs, const uint64_t* first, int njobs, uint64_t rows,
+                             cudaStream_t stream);
+
+// From this many of a launch's `rows` up, its tie rows get a thread each, below a
+// warp each.  A warp's lanes read one row's points side by side and leave no
+// tail, but sort, rank and sum across lanes; neighbouring threads of a dense
+// list walk the same cells.  Thread / warp, K = 17, ms: scattered ties (2 % of a
+// cloud with duplicates) 0.48 / 0.23 for 44k rows of 2M, 1.15 / 1.09 for 350k of
+// 16M; a raster's (8 %) 0.30 / 0.47 for 82k of 1M; a lattice's (all) 0.23 / 0.19
+// for 20k, 0.24 / 0.41 for 50k, 2.4 / 8.2 for 1M.
+uint32_t many_ties(int sms, uint64_t rows) {
+    return (uint32_t)std::max<uint64_t>((uint64_t)sms * 256, rows / 16);
+}
+
 int launch_retry_finish(const QueryArgs& q, int slots, int sms, cudaStream_t stream) {
     const uint64_t rows = q.nq;  // the most there can be
     const unsigned blocks =
@@ -485,19 +503,30 @@ int launch_retry_batch(int slots, const BatchJob* jobs, int njobs, int sms, cuda
 }
 
 int launch_tie_rows(const TieArgs& a, const uint32_t* count, int sms, cudaStream_t stream) {
+    const uint32_t many = many_ties(sms, a.of_rows);
+    if (a.ids_out) return launch_tie_threads(a, count, 0, sms, stream);
+    if (a.nties >= many) {
+        const int rc = launch_tie_threads(a, count, many, sms, stream);
+        if (rc || !count) return rc;
+    }
     const unsigned blocks =
         (unsigned)std::max<uint64_t>(1, std::min<uint64_t>(((uint64_t)a.nties + 3) / 4, (uint64_t)sms * kRowBlocksPerSm));
-    knn_tie_kernel<<<blocks, kRowThreads, 0, stream>>>(a, count);
+    knn_tie_kernel<<<blocks, kRowThreads, 0, stream>>>(a, count, many);
     NBG_LAUNCHED(1);
     return cudaGetLastError() == cudaSuccess ? NBG_OK : NBG_ERR_CUDA;
 }
 
 int launch_tie_batch(Context* ctx, const std::vector<TieArgs>& jobs, cudaStream_t stream) {
     uint64_t total = 0;
-    for (const TieArgs& j : jobs) total += j.nties;
+    uint64_t rows = 0;
+    for (const TieArgs& j : jobs) {
+        total += j.nties;
+        rows += j.of_rows;
+    }
     if (!total) return NBG_OK;
     const uint64_t warps = (uint64_t)ctx->sm_count * kRowBlocksPerSm * (kRowThreads / 32);
-    const uint32_t run = (uint32_t)std::min<uint64_t>(32, std::max<uint64_t>(1, total / warps));
+    const bool threads = total >= many_ties(ctx->sm_count, rows);
+    const uint32_t run = threads ? 1u : (uint32_t)std::min<uint64_t>(32, std::max<uint64_t>(1, total / warps));
     std::vector<uint64_t> first(1, 0);
     for (const TieArgs& j : jobs) first.push_back(first.back() + (j.nties + run - 1) / run);
     TieArgs* djobs = nullptr;
@@ -508,7 +537,9 @@ int launch_tie_batch(Context* ctx, const std::vector<TieArgs>& jobs, cudaStream_
     // pageable sources: both copies complete before they return
     if (!rc) rc = host_to_device(ctx, djobs, jobs.data(), jb, stream);
     if (!rc) rc = host_to_device(ctx, dfirst, first.data(), fb, stream);
-    if (!rc) {
+    if (!rc && threads) {
+        rc = launch_tie_threads_batch(djobs, dfirst, (int)jobs.size(), total, stream);
+    } else if (!rc) {
         const uint64_t runs = first.back();
         knn_tie_batch_kernel<<<(unsigned)((runs * 32 + kRowThreads - 1) / kRowThreads), kRowThreads, 0, stream>>>(
             djobs, dfirst, (int)jobs.size(), runs, run);

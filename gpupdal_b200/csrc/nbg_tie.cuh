@@ -57,6 +57,7 @@ struct TieArgs {
     ExceptionSink ex;
     const uint2* ties;
     uint32_t nties;
+    uint64_t of_rows;  // rows of the query that listed them
     KdOrder kd;
     uint32_t* exact_rows;
     uint32_t* counters;
