@@ -38,7 +38,7 @@ int slots_for_k(int K);
 int launch_loc_batch(int K, const BatchJob* jobs, int njobs, uint64_t items, cudaStream_t stream);
 uint32_t located_offset_bits(const Tile* t);
 int launch_group_batch(int slots, const BatchJob* jobs, int njobs, uint64_t items, cudaStream_t stream);
-int launch_retry_batch(int slots, const BatchJob* jobs, int njobs, int sms, cudaStream_t stream);
+int launch_retry_batch(int slots, const BatchJob* jobs, int njobs, uint64_t rows, int sms, cudaStream_t stream);
 
 static constexpr int kCounters = 64;  // u32 counters per tile
 
@@ -417,7 +417,8 @@ extern "C" int nbg_run_batch(nbg_context* h, const nbg_batch_item* items, int32_
         int r = NBG_OK;
         for (const Cls& c : classes)
             if (c.select && !r)
-                r = launch_retry_batch(slots_for_k(c.K), B->jobs + c.begin, c.count, ctx->sm_count, ctx->fork);
+                r = launch_retry_batch(slots_for_k(c.K), B->jobs + c.begin, c.count, 128 * c.items, ctx->sm_count,
+                                       ctx->fork);
         if (!r)
             r = launch_finish_queue(ctx, B->jobs + nl, nl, fin_items, B->heads + classes.size(), s, reserve);
         e = cudaEventRecord(ctx->fev[1], ctx->fork);

@@ -210,6 +210,18 @@ __device__ __forceinline__ int job_of(const BatchJob* __restrict__ jobs, int njo
     return lo;
 }
 
+// Rows that the jobs' selects have handed back, in every thread of the block.
+__device__ __forceinline__ uint32_t retry_total(const BatchJob* __restrict__ jobs, int njobs) {
+    __shared__ uint32_t s_total;
+    if (threadIdx.x == 0) s_total = 0;
+    __syncthreads();
+    uint32_t n = 0;
+    for (int j = threadIdx.x; j < njobs; j += blockDim.x) n += jobs[j].q.counters[6];
+    if (n) atomicAdd(&s_total, n);
+    __syncthreads();
+    return s_total;
+}
+
 // What a select kernel reads of a job, in registers (the job lies in memory the
 // kernel's own stores might alias).
 __device__ __forceinline__ QueryArgs select_args(const BatchJob& j) {

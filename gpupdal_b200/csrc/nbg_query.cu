@@ -183,8 +183,9 @@ __global__ void __launch_bounds__(128) knn_fused_kernel(const QueryArgs a) {
 }
 
 // Split form, pass 1 + pass 2: the row's exact neighbourhood sums, at its point
-// id (cnt = 0 marks a row handed to the exact path).
-template <int KS>
+// id (cnt = 0 marks a row handed to the exact path).  With FINISH the row is
+// finished in place instead (a handed-back row, whose slot holds cnt = 0).
+template <int KS, bool FINISH = false>
 __device__ __forceinline__ void select_row(const QueryArgs& a, const uint64_t i) {
     const GridParams g = *a.gp;
     const float4 q = __ldg(&a.qpts[i]);
@@ -196,9 +197,11 @@ __device__ __forceinline__ void select_row(const QueryArgs& a, const uint64_t i)
         const int32_t qraw[3] = {__float2int_rz(q.x) + g.minx, __float2int_rz(q.y) + g.miny,
                                  __float2int_rz(q.z) + g.minz};
         nbg_finish_row(a.grp, a.tf, a.ex, id, 0, M, qraw);
-        RowSums z;
-        z.cnt = 0;
-        a.sums[id] = z;
+        if (!FINISH) {
+            RowSums z;
+            z.cnt = 0;
+            a.sums[id] = z;
+        }
         return;
     }
     QueryCell qc;
@@ -215,14 +218,23 @@ __device__ __forceinline__ void select_row(const QueryArgs& a, const uint64_t i)
     out.cnt = 0;
     if (!select_kth<KS>(a, g, qc, q, K, R, kk, tie)) {
         defer_row(a, id, tie, kk, R);
-        a.sums[id] = out;
+        if (!FINISH) a.sums[id] = out;
         return;
     }
     Pass2Fn f2{q.x, q.y, q.z, kk, 0, 0, 0, 0, 0, 0, 0, 0, 0, 0};
     for (int r = 0; r <= R; ++r) scan_shell(a.gv, g, qc, r, f2);
     if (f2.cnt != K) {
         defer_row(a, id, false, kk, R);
-        a.sums[id] = out;
+        if (!FINISH) a.sums[id] = out;
+        return;
+    }
+    if (FINISH) {
+        const long long n = f2.cnt;
+        const long long M[6] = {n * f2.sxx - (long long)f2.s1x * f2.s1x, n * f2.syx - (long long)f2.s1y * f2.s1x,
+                                n * f2.syy - (long long)f2.s1y * f2.s1y, n * f2.szx - (long long)f2.s1z * f2.s1x,
+                                n * f2.szy - (long long)f2.s1z * f2.s1y, n * f2.szz - (long long)f2.s1z * f2.s1z};
+        const int32_t qraw[3] = {qc.qx + g.minx, qc.qy + g.miny, qc.qz + g.minz};
+        nbg_finish_row(a.grp, a.tf, a.ex, id, (int)n, M, qraw);
         return;
     }
     out.s[0] = f2.s1x;
@@ -666,6 +678,50 @@ __global__ void __launch_bounds__(128) knn_retry_kernel(const QueryArgs a) {
         ids_row<KS>(a, __ldg(&a.rows[r]));
     }
 }
+
+// Rows handed back, finished in place, a thread per row where they are many
+// (a.nq_dev of them; fewer than `least` are left to knn_retry_finish_kernel).
+template <int KS>
+__global__ void __launch_bounds__(128) knn_retry_thread_kernel(const QueryArgs a, uint32_t least) {
+    const uint32_t nr = *a.nq_dev;
+    if (nr < least) return;
+    for (uint32_t r = blockIdx.x * blockDim.x + threadIdx.x; r < nr; r += gridDim.x * blockDim.x)
+        select_row<KS, true>(a, __ldg(&a.rows[r]));
+}
+
+// The same for the tiles of a batch: job blockIdx.y's rows.
+template <int KS>
+__global__ void __launch_bounds__(128) knn_retry_thread_batch_kernel(const BatchJob* __restrict__ jobs, int njobs,
+                                                                     uint32_t least) {
+    if (retry_total(jobs, njobs) < least) return;
+    const QueryArgs& a = jobs[blockIdx.y].q;
+    const uint32_t nr = a.counters[6];
+    for (uint32_t r = blockIdx.x * blockDim.x + threadIdx.x; r < nr; r += gridDim.x * blockDim.x)
+        select_row<KS, true>(a, a.retry_rows[r]);
+}
+
+struct RetryArgs {
+    QueryArgs q;
+    const BatchJob* jobs;  // or the jobs of a batch
+    int njobs;
+    uint32_t least;
+    unsigned blocks;  // (per job)
+    cudaStream_t stream;
+};
+
+template <int KS>
+struct RetryLauncher {
+    using Args = RetryArgs;
+    static int run(const RetryArgs& r) {
+        if (r.jobs)
+            knn_retry_thread_batch_kernel<KS>
+                <<<dim3(r.blocks, (unsigned)r.njobs), 128, 0, r.stream>>>(r.jobs, r.njobs, r.least);
+        else
+            knn_retry_thread_kernel<KS><<<r.blocks, 128, 0, r.stream>>>(r.q, r.least);
+        NBG_LAUNCHED(1);
+        return cudaGetLastError() == cudaSuccess ? NBG_OK : NBG_ERR_CUDA;
+    }
+};
 
 struct TieFn {
     float qx, qy, qz;
@@ -1267,6 +1323,18 @@ bool located_keys_fit(const Tile* t) {
     const GridParams& g = t->host_gp;
     const double mean = (double)t->n / ((double)g.gx * (double)g.gy);
     return (double)(1u << loc_offset_bits(g.cell)) >= 4.0 * mean;
+}
+
+// (slots = K + 1 of the widest row)
+int launch_retry_threads(const QueryArgs& q, int slots, uint32_t least, int sms, cudaStream_t stream) {
+    const unsigned blocks = (unsigned)std::min<uint64_t>((q.nq + 127) / 128, (uint64_t)sms * 16);
+    return dispatch_slots<RetryLauncher>(slots - 1, RetryArgs{q, nullptr, 0, least, blocks, stream});
+}
+
+int launch_retry_threads_batch(int slots, const BatchJob* jobs, int njobs, uint32_t least, int sms,
+                               cudaStream_t stream) {
+    const unsigned blocks = (unsigned)std::max<uint64_t>(4, (uint64_t)sms * 16 / (uint64_t)njobs);
+    return dispatch_slots<RetryLauncher>(slots - 1, RetryArgs{QueryArgs{}, jobs, njobs, least, blocks, stream});
 }
 
 struct LaunchArgs {

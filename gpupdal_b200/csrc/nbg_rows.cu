@@ -9,7 +9,8 @@
 // columns up together, then read its points 32 at a time.
 //   handed-back rows  candidates below the current (K+1)-th distance are
 //                     gathered in shared memory and, 32 at a time, sorted across
-//                     the lanes and merged into the sorted list the lanes hold
+//                     the lanes and merged into the sorted list the lanes hold; a
+//                     thread each where they are many (many_retries)
 //   tie rows          strictly closer points are summed; a member of the group at
 //                     the K-th distance goes to the lane of its number, and every
 //                     lane ranks its member by (FP64 distance, visiting order);
@@ -309,15 +310,18 @@ __device__ __forceinline__ void retry_finish_rows(const QueryArgs& a, const uint
 }
 
 template <int NR>
-__global__ void __launch_bounds__(kRowThreads) knn_retry_finish_kernel(const QueryArgs a) {
+__global__ void __launch_bounds__(kRowThreads) knn_retry_finish_kernel(const QueryArgs a, uint32_t most) {
     __shared__ uint32_t s_gather[kRowThreads / 32][64];
+    if (*a.nq_dev >= most) return;  // (a thread each)
     retry_finish_rows<NR>(a, a.rows, *a.nq_dev, s_gather);
 }
 
 // The same for the tiles of a batch: job blockIdx.y's rows.
 template <int NR>
-__global__ void __launch_bounds__(kRowThreads) knn_retry_batch_kernel(const BatchJob* __restrict__ jobs) {
+__global__ void __launch_bounds__(kRowThreads) knn_retry_batch_kernel(const BatchJob* __restrict__ jobs, int njobs,
+                                                                      uint32_t most) {
     __shared__ uint32_t s_gather[kRowThreads / 32][64];
+    if (most != 0xFFFFFFFFu && retry_total(jobs, njobs) >= most) return;
     const QueryArgs& a = jobs[blockIdx.y].q;
     retry_finish_rows<NR>(a, a.retry_rows, a.counters[6], s_gather);
 }
@@ -468,36 +472,68 @@ static constexpr uint64_t kRowBlocksPerSm = 16;
 int launch_tie_threads(const TieArgs& a, const uint32_t* count, uint32_t least, int sms, cudaStream_t stream);
 int launch_tie_threads_batch(const TieArgs* jobs, const uint64_t* first, int njobs, uint64_t rows,
                              cudaStream_t stream);
+int launch_retry_threads(const QueryArgs& q, int slots, uint32_t least, int sms, cudaStream_t stream);
+int launch_retry_threads_batch(int slots, const BatchJob* jobs, int njobs, uint32_t least, int sms,
+                               cudaStream_t stream);
 
 // From this many of a launch's `rows` up, its tie rows get a thread each, below a
 // warp each.  A warp's lanes read one row's points side by side and leave no
 // tail, but sort, rank and sum across lanes; neighbouring threads of a dense
 // list walk the same cells.  Thread / warp, K = 17, ms: scattered ties (2 % of a
 // cloud with duplicates) 0.48 / 0.23 for 44k rows of 2M, 1.15 / 1.09 for 350k of
-// 16M; a raster's (8 %) 0.30 / 0.47 for 82k of 1M; a lattice's (all) 0.23 / 0.19
-// for 20k, 0.24 / 0.41 for 50k, 2.4 / 8.2 for 1M.
+// 16M; 7 % of a batch whose density falls with distance 10.1 / 6.8; a raster's
+// (8 %) 0.30 / 0.47 for 82k of 1M; a lattice's (all) 0.23 / 0.19 for 20k, 0.24 / 0.41
+// for 50k, 2.4 / 8.2 for 1M.
 uint32_t many_ties(int sms, uint64_t rows) {
-    return (uint32_t)std::max<uint64_t>((uint64_t)sms * 256, rows / 16);
+    return (uint32_t)std::max<uint64_t>((uint64_t)sms * 256, rows / 13);
+}
+
+// The same for the rows a select hands back: few of them are the hard rows, far
+// from one another, with a long tail; when a fifth of a large tile is handed back
+// the select as a whole did not fit it, and neighbouring threads walk the same
+// cells again.  Whole calls, thread / warp, ms: 1 - 2 % of 4M mixture points 13.5 /
+// 12.6 (K = 65) and 8.7 / 8.6 (K = 33); 17 % of 500k points far apart in raw units
+// 18.9 / 12.7; 29 % of 1M points whose density falls with distance 160 / 197; 39 %
+// of 500k far points 22.8 / 42.6; all of a 1M wall 24.4 / 31.5, of a 100k one 1.1 /
+// 1.8; 77 % of 100k far points 20.0 / 22.2, 35 % of them 19.4 / 11.1.  A thread's
+// list costs in proportion to its slots, a warp's by the third register at most:
+// from 65 slots up half the rows (K = 65, 500k far points: 32 % 43.8 / 35.4, 39 %
+// 93 / 85, all 182 / 219).
+uint32_t many_retries(int sms, int slots, uint64_t rows) {
+    return (uint32_t)std::max<uint64_t>((uint64_t)sms * 512, slots > 64 ? rows / 2 : rows / 5);
 }
 
 int launch_retry_finish(const QueryArgs& q, int slots, int sms, cudaStream_t stream) {
     const uint64_t rows = q.nq;  // the most there can be
+    const uint32_t many = many_retries(sms, slots, rows);
+    if (rows >= many) {
+        const int rc = launch_retry_threads(q, slots, many, sms, stream);
+        if (rc) return rc;
+    }
     const unsigned blocks =
         (unsigned)std::max<uint64_t>(1, std::min<uint64_t>((rows + 3) / 4, (uint64_t)sms * kRowBlocksPerSm));
-    if (slots <= 32) knn_retry_finish_kernel<1><<<blocks, kRowThreads, 0, stream>>>(q);
-    else if (slots <= 64) knn_retry_finish_kernel<2><<<blocks, kRowThreads, 0, stream>>>(q);
-    else knn_retry_finish_kernel<3><<<blocks, kRowThreads, 0, stream>>>(q);
+    if (slots <= 32) knn_retry_finish_kernel<1><<<blocks, kRowThreads, 0, stream>>>(q, many);
+    else if (slots <= 64) knn_retry_finish_kernel<2><<<blocks, kRowThreads, 0, stream>>>(q, many);
+    else knn_retry_finish_kernel<3><<<blocks, kRowThreads, 0, stream>>>(q, many);
     NBG_LAUNCHED(1);
     return cudaGetLastError() == cudaSuccess ? NBG_OK : NBG_ERR_CUDA;
 }
 
-int launch_retry_batch(int slots, const BatchJob* jobs, int njobs, int sms, cudaStream_t stream) {
+// `rows`: the rows of the jobs' tiles.
+int launch_retry_batch(int slots, const BatchJob* jobs, int njobs, uint64_t rows, int sms, cudaStream_t stream) {
     if (!njobs) return NBG_OK;
+    uint32_t many = many_retries(sms, slots, rows);
+    if (rows >= many) {
+        const int rc = launch_retry_threads_batch(slots, jobs, njobs, many, sms, stream);
+        if (rc) return rc;
+    } else {
+        many = 0xFFFFFFFFu;  // (there cannot be as many)
+    }
     const dim3 grid((unsigned)std::max<uint64_t>(4, (uint64_t)sms * kRowBlocksPerSm / (uint64_t)njobs),
                     (unsigned)njobs);
-    if (slots <= 32) knn_retry_batch_kernel<1><<<grid, kRowThreads, 0, stream>>>(jobs);
-    else if (slots <= 64) knn_retry_batch_kernel<2><<<grid, kRowThreads, 0, stream>>>(jobs);
-    else knn_retry_batch_kernel<3><<<grid, kRowThreads, 0, stream>>>(jobs);
+    if (slots <= 32) knn_retry_batch_kernel<1><<<grid, kRowThreads, 0, stream>>>(jobs, njobs, many);
+    else if (slots <= 64) knn_retry_batch_kernel<2><<<grid, kRowThreads, 0, stream>>>(jobs, njobs, many);
+    else knn_retry_batch_kernel<3><<<grid, kRowThreads, 0, stream>>>(jobs, njobs, many);
     NBG_LAUNCHED(1);
     return cudaGetLastError() == cudaSuccess ? NBG_OK : NBG_ERR_CUDA;
 }
