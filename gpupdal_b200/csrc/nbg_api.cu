@@ -1432,12 +1432,32 @@ static std::pair<int, int> tuning_class(const Tile* t, int K) {
 // its keys hold a column; the group select sorts batches and wins above.  A chunk
 // holds a fraction of each clump, so the group select's bounds are loose there
 // (6M stress records, K = 17: 18.8 ms against 17.4 with the two-pass search).
+//
+// Both hand back what their keys cannot hold, so a tile most of whose points
+// lie where they cannot is left to the others.  The grid counts those points:
+//   in full columns     the single pass (1M points whose density falls with distance,
+//                       K = 9, 45 %: 54 / 73 / 31; ordinary clouds 0 - 2 %)
+//   few to a cell       the single pass again, which looks two rings far (a wall of
+//                       1M points, 128 cells a point: 18.6 / 24.3 / 9.5; a cube of
+//                       points, 3 cells a point: 1.87 / 1.95 / 3.53)
+//   in thin columns     the group select (500k points far apart in raw units, K = 33,
+//                       10 %: 55 / 73 / 59, 48 %: 59 / 76 / 77; K = 65, 9 %: 94 / 107 /
+//                       85, 85 %: 155 / 171 / 186)
+//   in heavy columns    the group select (200k points in nested clusters, K = 9, 76 %:
+//                       209 / 189 / 290; 26 % at most where density falls with distance)
+// The last two from 100k points up: below, the few handed-back rows there are find
+// idle warps (50k nested: 57 / 26 / 21).
 int select_kernel(const Tile* t, int K, bool chunks) {
     if (t->group >= 0) return t->group;
     if (!t->clumps) return 0;
+    const GridParams& g = t->host_gp;
+    const uint64_t n = t->n;
     const int slots = slots_for_k(K);
-    if ((slots <= 14 || (slots <= 18 && (chunks || t->n >= 16000000))) && located_keys_fit(t)) return 2;
-    return chunks && slots < 50 ? 0 : 32;
+    if ((slots <= 14 || (slots <= 18 && (chunks || n >= 16000000))) && located_keys_fit(t) && g.in_full <= n / 20 &&
+        g.cells <= 8 * n)
+        return 2;
+    if (chunks && slots < 50) return 0;
+    return n >= 100000 && (g.in_thin > n / 10 || g.in_heavy > n / 2) ? 0 : 32;
 }
 
 // A tile the caller did not tune takes the context's cached choice for its

@@ -26,7 +26,24 @@ struct GridParams {
     int32_t tgx;       // columns are laid out in 64 x 64 tiles, tgx tiles a row (0: row by row)
     uint32_t nslots;   // column slots of that layout (tiles at the edge are padded)
     float r1;          // radius holding one point at the tile's planar density
+    // which select kernel fits (select_kernel): points in columns of more than
+    // full, fewer than thin and more than heavy points, and the columns' cells
+    uint32_t full, thin, heavy;
+    uint32_t in_full, in_thin, in_heavy;
+    uint32_t cells;
 };
+
+// Offset bits of the single-pass select's keys for cell edge c: the squared
+// distance field (27 - ob bits) holds (2.2 c)^2, the search's reach at ring 2.
+__host__ __device__ inline uint32_t loc_offset_bits(int32_t c) {
+    const double e = c < 1 ? 1.0 : (double)c, need = 4.84 * e * e;
+    int bits = 1;
+    while (bits < 27 && (double)(1u << bits) < need) ++bits;
+    return bits > 21 ? 6u : bits < 11 ? 16u : (uint32_t)(27 - bits);
+}
+
+// Margins of the group select's keys: half of them for long lists (WarpShape).
+__host__ __device__ inline int group_max_margin(int slots) { return slots > 40 ? 1447 : 2047; }
 
 // Slot of column (cx, cy) in the layout of the columns' runs of cells: Morton
 // order inside 64 x 64 tiles, so that consecutive cells (and the points in

@@ -123,6 +123,14 @@ __device__ GridParams grid_config(const int32_t* bb, uint64_t n, int k1, float c
     const uint64_t tx = ((uint64_t)g.gx + 63) / 64, ty = ((uint64_t)g.gy + 63) / 64;
     g.tgx = tx * ty * 4096 <= cols_cap ? (int32_t)tx : 0;
     g.nslots = g.tgx ? (uint32_t)(tx * ty * 4096) : g.ncols;
+    // a full column's offsets pass the single-pass select's keys, and a thin
+    // one's k1 nearest lie (at its own planar density) beyond 0.8 of the group
+    // select's
+    g.full = 1u << loc_offset_bits(g.cell);
+    const double m = 0.8 * group_max_margin(k1 + 1);
+    g.thin = (uint32_t)fmin(4.0e9, k1 * c * c / (3.14159265358979 * m * m));
+    g.heavy = (uint32_t)fmin(4.0e9, 256.0 * fmax(1.0, (double)n / (double)g.ncols));
+    g.in_full = g.in_thin = g.in_heavy = g.cells = 0;
     return g;
 }
 
@@ -166,13 +174,13 @@ __global__ void col_extent_kernel(const GridParams* __restrict__ gpp,
     }
 }
 
-__global__ void col_base_kernel(const GridParams* __restrict__ gpp, const uint32_t* __restrict__ ext,
+__global__ void col_base_kernel(GridParams* gpp, const uint32_t* __restrict__ ext,
                                 int4* __restrict__ colinfo, uint32_t* __restrict__ table_size) {
     const GridParams g = *gpp;
     for (uint32_t c = blockIdx.x * blockDim.x + threadIdx.x; c <= g.ncols;
          c += gridDim.x * blockDim.x) {
         if (c < g.ncols) colinfo[c].x = (int)ext[column_slot(g, c % (uint32_t)g.gx, c / (uint32_t)g.gx)];
-        else *table_size = ext[g.nslots];
+        else *table_size = gpp->cells = ext[g.nslots];
     }
 }
 
@@ -221,6 +229,40 @@ __global__ void cell_scatter_kernel(const int32_t* __restrict__ x, const int32_t
     }
 }
 
+// The counts of GridParams over the columns this thread takes; all threads of
+// its block take part.
+__device__ __forceinline__ void count_columns(const GridParams& g, const int4* colinfo, const uint32_t* cstart,
+                                              uint32_t entries, uint32_t first, uint32_t step, GridParams* gp) {
+    uint32_t v[3] = {0, 0, 0};
+    for (uint32_t c = first; c < g.ncols; c += step) {
+        const int4 ci = colinfo[c];
+        // (a column beyond a table that is too small, which is built again)
+        if (ci.z < ci.y || (uint64_t)(uint32_t)ci.x + (uint32_t)(ci.z - ci.y) + 1 > entries) continue;
+        const uint32_t p = cstart[(uint32_t)ci.x + (uint32_t)(ci.z - ci.y) + 1u] - cstart[(uint32_t)ci.x];
+        v[0] += p > g.full ? p : 0u;
+        v[1] += p < g.thin ? p : 0u;
+        v[2] += p > g.heavy ? p : 0u;
+    }
+    uint32_t* to = &gp->in_full;
+#pragma unroll
+    for (int k = 0; k < 3; ++k) {
+        const uint32_t r = __reduce_add_sync(0xffffffffu, v[k]);
+        if ((threadIdx.x & 31) == 0 && r) atomicAdd(&to[k], r);
+    }
+}
+
+// The scatter's cursors start at the cells' first points; and the columns'
+// counts, which want the same prefix.
+__global__ void __launch_bounds__(256) cell_cursor_kernel(const uint32_t* __restrict__ cstart,
+                                                          uint32_t* __restrict__ cursor, uint64_t count,
+                                                          const int4* __restrict__ colinfo, GridParams* gpp) {
+    const uint32_t i0 = blockIdx.x * blockDim.x + threadIdx.x, step = gridDim.x * blockDim.x;
+    for (uint64_t i = i0; i < count / 4; i += step) ((uint4*)cursor)[i] = ((const uint4*)cstart)[i];
+    if (i0 < (count & 3u)) cursor[(count & ~3ull) + i0] = cstart[(count & ~3ull) + i0];
+    const GridParams g = *gpp;
+    count_columns(g, colinfo, cstart, (uint32_t)min(count - 1, (uint64_t)0xFFFFFFFFu), i0, step, gpp);
+}
+
 // Exclusive prefix sums of v[0 .. count) in place (and into w), by one block of
 // kSmallThreads; returns the total in every thread.  `part` is shared, one
 // word a warp.
@@ -261,7 +303,7 @@ __device__ uint32_t block_scan(uint32_t* v, uint32_t* w, uint32_t count, uint32_
 // a block should walk, or than the table holds, sets bit 2 of cap_hit and is
 // left to the other builds.
 //
-// Bound by the phases' latency, not by work: thirteen launches and a read of the
+// Bound by the phases' latency, not by work: fourteen launches and a read of the
 // table size between them are what it saves (figures at grid_small).
 __global__ void __launch_bounds__(kSmallThreads) grid_small_kernel(
     const int32_t* x, const int32_t* y, const int32_t* z, const uint32_t n, int k1, float cell_factor,
@@ -322,7 +364,7 @@ __global__ void __launch_bounds__(kSmallThreads) grid_small_kernel(
     }
     __syncthreads();
     const uint32_t total = block_scan(ext, nullptr, g.nslots + 1, part);
-    if (tid == 0) *table_size = total;
+    if (tid == 0) *table_size = gp->cells = total;
     if (total > entries || total > kSmallSlots) {  // (as *gp says to the host)
         if (tid == 0) gp->cap_hit = g.cap_hit | 2u;
         return;
@@ -347,6 +389,7 @@ __global__ void __launch_bounds__(kSmallThreads) grid_small_kernel(
     }
     __syncthreads();
     block_scan(cstart, cursor, total + 1, part);
+    count_columns(g, colinfo, cstart, total, tid, kSmallThreads, gp);
     for (uint32_t i = tid; i < n; i += kSmallThreads) {
         if (keys[i] == 0xFFFFFFFFu) continue;
         const uint32_t pos = atomicAdd(&cursor[keys[i]], 1u);
@@ -586,17 +629,16 @@ int build_grid(Context* ctx, Tile* t, int k1, cudaStream_t stream) {
     if (cub::DeviceScan::ExclusiveSum(t->grid_tmp, tmp, t->cstart, t->cstart, (int)(T + 1),
                                       stream))
         return NBG_ERR_CUDA;
-    if (cudaMemcpyAsync(t->cursor, t->cstart, ((size_t)T + 1) * sizeof(uint32_t),
-                        cudaMemcpyDeviceToDevice, stream))
-        return NBG_ERR_CUDA;
+    cell_cursor_kernel<<<grid_blocks(T / 4, 256, sms), 256, 0, stream>>>(t->cstart, t->cursor, (uint64_t)T + 1,
+                                                                         t->colinfo, t->gp);
     cell_scatter_kernel<<<sb, 256, 0, stream>>>(t->x, t->y, t->z, n, t->gp, t->keys, t->cursor,
                                                 t->sorted);
-    // bbox (2), config, col init, zrange, extent, scan (2), bases, count, scan (2), scatter
-    NBG_LAUNCHED(13);
+    // bbox (2), config, col init, zrange, extent, scan (2), bases, count, scan (2), cursors, scatter
+    NBG_LAUNCHED(14);
     return cudaGetLastError() == cudaSuccess ? NBG_OK : NBG_ERR_CUDA;
 }
 
-// One block's build against thirteen launches and two reads by the host: 30 us
+// One block's build against fourteen launches and two reads by the host: 30 us
 // against 87 up to 2000 points, 42 / 86 at 4000, 56 / 84 at 8000, 65 / 86 at
 // 12000, 77 / 89 at 16000 (a call's time as before there), 140 / 88 at 32000.  A
 // cell edge fixed by a radius may give any number of columns: not here.
@@ -650,12 +692,11 @@ int build_grid_async(Context* ctx, Tile* t, int k1, cudaStream_t stream) {
     if (cub::DeviceScan::ExclusiveSum(t->grid_tmp, tmp, t->cstart, t->cstart, (int)(entries + 1),
                                       stream))
         return NBG_ERR_CUDA;
-    if (cudaMemcpyAsync(t->cursor, t->cstart, (size_t)(entries + 1) * sizeof(uint32_t),
-                        cudaMemcpyDeviceToDevice, stream))
-        return NBG_ERR_CUDA;
+    cell_cursor_kernel<<<grid_blocks(entries / 4, 256, sms), 256, 0, stream>>>(t->cstart, t->cursor, entries + 1,
+                                                                               t->colinfo, t->gp);
     cell_scatter_kernel<<<sb, 256, 0, stream>>>(t->x, t->y, t->z, n, t->gp, t->keys, t->cursor,
                                                 t->sorted);
-    NBG_LAUNCHED(13);
+    NBG_LAUNCHED(14);
     t->table_size = entries;
     return cudaGetLastError() == cudaSuccess ? NBG_OK : NBG_ERR_CUDA;
 }

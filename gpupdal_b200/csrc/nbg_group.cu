@@ -149,7 +149,7 @@ struct WarpShape {
     static constexpr int kIdxBits = KS > 40 ? 11 : 10;
     static constexpr uint32_t kCap = 1u << kIdxBits;
     static constexpr uint32_t kD2Max = (1u << (32 - kIdxBits)) - 1u;  // first distance past the field
-    static constexpr int kMaxMargin = KS > 40 ? 1447 : 2047;          // kMaxMargin^2 < kD2Max
+    static constexpr int kMaxMargin = KS > 40 ? 1447 : 2047;  // (group_max_margin) its square < kD2Max
     static constexpr uint32_t kMemClumps = (KS + 31) / 32;  // clumps whose points bound the search
     static constexpr size_t kBufBytes = (size_t)kBatch * 32 * 4;
     static constexpr size_t kStageBytes = 3 * 64 * 4;

@@ -1307,18 +1307,9 @@ static int dispatch_slots(int K, typename Launcher<10>::Args args) {
     return NBG_ERR_INVALID;
 }
 
-// Offset bits of the single-pass select's keys for cell edge c: the squared
-// distance field (27 - ob bits) holds (2.2 c)^2, the search's reach at ring 2.
-static uint32_t loc_offset_bits(int32_t c) {
-    const double need = 4.84 * (double)std::max(c, 1) * (double)std::max(c, 1);
-    int bits = 1;
-    while (bits < 27 && (double)(1u << bits) < need) ++bits;
-    return (uint32_t)std::min(16, std::max(6, 27 - bits));
-}
-
 // The single-pass select's offset field holds a column of four times the
-// tile's mean population: fuller columns are rare then, and their rows few
-// enough to hand back.
+// tile's mean population (where the columns are unlike, select_kernel also asks
+// for the points in fuller ones).
 bool located_keys_fit(const Tile* t) {
     const GridParams& g = t->host_gp;
     const double mean = (double)t->n / ((double)g.gx * (double)g.gy);
