@@ -235,7 +235,7 @@ __device__ __forceinline__ void count_columns(const GridParams& g, const int4* c
                                               uint32_t entries, uint32_t first, uint32_t step, GridParams* gp) {
     uint32_t v[3] = {0, 0, 0};
     for (uint32_t c = first; c < g.ncols; c += step) {
-        const int4 ci = colinfo[c];
+        const int4 ci = __ldcg(&colinfo[c]);
         // (a column beyond a table that is too small, which is built again)
         if (ci.z < ci.y || (uint64_t)(uint32_t)ci.x + (uint32_t)(ci.z - ci.y) + 1 > entries) continue;
         const uint32_t p = cstart[(uint32_t)ci.x + (uint32_t)(ci.z - ci.y) + 1u] - cstart[(uint32_t)ci.x];
