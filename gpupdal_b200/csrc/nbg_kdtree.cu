@@ -61,6 +61,7 @@ static constexpr int KD_BSTACK = 13;
 // points up; a smaller build would end after the query, which then waits for it.
 static constexpr int kKdBesideBlocksPerSm = 4;
 static constexpr uint64_t kKdBesideMinPoints = 16000000;
+static constexpr uint32_t KD_WARP_RUN = 2048;  // points of a run at the cut that one warp reads
 static constexpr int KD_RETRY = -100;  // kd_build: redo with room for every node
 static constexpr int KD_STACK = 96;
 static constexpr int KD_CAP = 66;
@@ -495,7 +496,9 @@ __global__ void __launch_bounds__(KD_THREADS) kd_classify_kernel(const KdLevel l
                     mn[1][d] = min(mn[1][d], in && v >= t2 ? c[d] : INT32_MAX);
                     mx[1][d] = max(mx[1][d], in && v >= t2 ? c[d] : INT32_MIN);
                 }
-                if (in && v >= t1 && v < t2)  // at the cut: few
+                // at the cut: few (a ninth of all points costs as much lane by lane
+                // as reduced over the warp first)
+                if (in && v >= t1 && v < t2)
 #pragma unroll
                     for (int d = 0; d < 3; ++d) {
                         atomicMin(&s_ext[3 + d], c[d]);
@@ -629,14 +632,38 @@ __device__ __forceinline__ void kd_tile_map(const KdSeg* segs, KdSplit* sp, uint
     }
 }
 
+// Extents of the points [from, mid) (v: least x, y, z, then greatest) and [mid, to)
+// (the next six), in every lane of a warp that takes every `step`-th from
+// `first` (its lanes' consecutive).
+__device__ __forceinline__ void kd_run_extents(const KdLevel& lv, uint32_t from, uint32_t mid, uint32_t to,
+                                               uint32_t first, uint32_t step, int32_t (&v)[12]) {
+#pragma unroll
+    for (int k = 0; k < 12; ++k) v[k] = k % 6 < 3 ? INT32_MAX : INT32_MIN;
+#pragma unroll 4
+    for (uint32_t i = from + first; i < to; i += step) {
+        const int32_t c[3] = {__ldcg(&lv.rx[i]), __ldcg(&lv.ry[i]), __ldcg(&lv.rz[i])};
+#pragma unroll
+        for (int d = 0; d < 3; ++d) {
+            v[d] = min(v[d], i < mid ? c[d] : INT32_MAX);
+            v[3 + d] = max(v[3 + d], i < mid ? c[d] : INT32_MIN);
+            v[6 + d] = min(v[6 + d], i < mid ? INT32_MAX : c[d]);
+            v[9 + d] = max(v[9 + d], i < mid ? INT32_MIN : c[d]);
+        }
+    }
+#pragma unroll
+    for (int k = 0; k < 12; ++k)
+        v[k] = k % 6 < 3 ? __reduce_min_sync(0xffffffffu, v[k]) : __reduce_max_sync(0xffffffffu, v[k]);
+}
+
 // The misplaced pairs of a tile: every load of the thread's pairs is issued
 // before any store (each position belongs to exactly one pair of the level, so
 // the loads never read what a store of this launch writes), which keeps the
 // dependent position -> coordinate loads of all the thread's items in flight
 // together instead of one item at a time.  After pass 2 the last block splits
-// the segments and plans the next level.
+// the segments and plans the next level (the bound keeps its registers from
+// costing the swaps a resident block).
 template <int PASS>
-__global__ void __launch_bounds__(KD_THREADS) kd_swap_kernel(const KdLevel lv) {
+__global__ void __launch_bounds__(KD_THREADS, PASS == 1 ? 4 : 3) kd_swap_kernel(const KdLevel lv) {
     const uint32_t ntiles = lv.st->tiles;
     if (!ntiles) return;
     constexpr int ITEMS = 4;
@@ -685,15 +712,66 @@ __global__ void __launch_bounds__(KD_THREADS) kd_swap_kernel(const KdLevel lv) {
     }
     if (PASS == 1 || !kd_last_block(lv.st)) return;
     // ---- split the segments, plan the next level
-    __shared__ uint32_t s_next;
+    __shared__ uint32_t s_next, s_who, s_run[3];
+    __shared__ int32_t s_rext[12];
     if (threadIdx.x == 0) s_next = 0;
     __syncthreads();
     const uint32_t S = lv.st->segs;
-    for (uint32_t s = threadIdx.x; s < S; s += KD_THREADS) {
-        const KdSeg sg = lv.segs[s];
-        const KdSplit p = lv.sp[s];
+    const int lane = threadIdx.x & 31;
+    for (uint32_t s0 = 0; s0 < S; s0 += KD_THREADS) {
+        const uint32_t s = s0 + threadIdx.x;
+        const KdSeg sg = lv.segs[min(s, S - 1)];
+        const KdSplit p = lv.sp[min(s, S - 1)];
         const uint32_t count = sg.end - sg.begin;
         const uint32_t index = kd_split_index(count, p.L, p.eq);
+        // the split falls among the points at the cut: the extents of the two
+        // parts of that run, read by a warp, or (a long run) by the block
+        const bool in_run = s < S && index > p.L && index < p.L + p.eq;
+        int32_t run[12];
+#pragma unroll
+        for (int k = 0; k < 12; ++k) run[k] = k % 6 < 3 ? INT32_MAX : INT32_MIN;
+        const uint32_t from = sg.begin + p.L, mid = sg.begin + index, to = from + p.eq;
+        if (__syncthreads_or(in_run)) {
+            for (unsigned m = __ballot_sync(0xffffffffu, in_run && p.eq <= KD_WARP_RUN); m; m &= m - 1) {
+                const int src = __ffs(m) - 1;
+                int32_t v[12];
+                kd_run_extents(lv, __shfl_sync(0xffffffffu, from, src), __shfl_sync(0xffffffffu, mid, src),
+                               __shfl_sync(0xffffffffu, to, src), lane, 32u, v);
+                if (lane == src)
+#pragma unroll
+                    for (int k = 0; k < 12; ++k) run[k] = v[k];
+            }
+            bool wait = in_run && p.eq > KD_WARP_RUN;
+            while (__syncthreads_or(wait)) {
+                if (threadIdx.x == 0) s_who = KD_THREADS;
+                if (threadIdx.x < 12) s_rext[threadIdx.x] = threadIdx.x % 6 < 3 ? INT32_MAX : INT32_MIN;
+                __syncthreads();
+                if (wait) atomicMin(&s_who, threadIdx.x);
+                __syncthreads();
+                const bool mine = wait && s_who == threadIdx.x;
+                if (mine) {
+                    s_run[0] = from;
+                    s_run[1] = mid;
+                    s_run[2] = to;
+                }
+                __syncthreads();
+                int32_t v[12];
+                kd_run_extents(lv, s_run[0], s_run[1], s_run[2], threadIdx.x, KD_THREADS, v);
+                if (lane == 0)
+#pragma unroll
+                    for (int k = 0; k < 12; ++k) {
+                        if (k % 6 < 3) atomicMin(&s_rext[k], v[k]);
+                        else atomicMax(&s_rext[k], v[k]);
+                    }
+                __syncthreads();
+                if (mine) {
+                    wait = false;
+#pragma unroll
+                    for (int k = 0; k < 12; ++k) run[k] = s_rext[k];
+                }
+            }
+        }
+        if (s >= S) continue;
         const uint32_t cid = atomicAdd(&lv.st->nodes, 2u);
         if (cid + 2 > lv.N.cap) {
             atomicAdd(&lv.st->errors, 1u);
@@ -701,30 +779,17 @@ __global__ void __launch_bounds__(KD_THREADS) kd_swap_kernel(const KdLevel lv) {
         }
         kd_write_children(lv.N, sg.node, cid, p.f, sg.begin, sg.begin + index, sg.end, sg.pad);
         // the children's extents: the points at the cut go to one side, or (the
-        // split falls among them) their range is read
+        // split falls among them) to both
         int32_t mn[2][3], mx[2][3];
-        for (int d = 0; d < 3; ++d) {
-            mn[0][d] = p.mn[0][d];
-            mx[0][d] = p.mx[0][d];
-            mn[1][d] = p.mn[2][d];
-            mx[1][d] = p.mx[2][d];
-        }
-        if (index == p.L || index == p.L + p.eq) {
-            const int side = index == p.L ? 1 : 0;
-            for (int d = 0; d < 3; ++d) {
-                mn[side][d] = min(mn[side][d], p.mn[1][d]);
-                mx[side][d] = max(mx[side][d], p.mx[1][d]);
+        const int at = index == p.L ? 1 : 0;
+#pragma unroll
+        for (int d = 0; d < 3; ++d)
+#pragma unroll
+            for (int side = 0; side < 2; ++side) {
+                mn[side][d] = min(p.mn[2 * side][d], in_run ? run[6 * side + d] : side == at ? p.mn[1][d] : INT32_MAX);
+                mx[side][d] =
+                    max(p.mx[2 * side][d], in_run ? run[6 * side + 3 + d] : side == at ? p.mx[1][d] : INT32_MIN);
             }
-        } else {
-            for (uint32_t i = sg.begin + p.L; i < sg.begin + p.L + p.eq; ++i) {
-                const int side = i < sg.begin + index ? 0 : 1;
-                const int32_t c[3] = {__ldcg(&lv.rx[i]), __ldcg(&lv.ry[i]), __ldcg(&lv.rz[i])};
-                for (int d = 0; d < 3; ++d) {
-                    mn[side][d] = min(mn[side][d], c[d]);
-                    mx[side][d] = max(mx[side][d], c[d]);
-                }
-            }
-        }
         for (int side = 0; side < 2; ++side) {
             const uint32_t node = cid + side;
             for (int d = 0; d < 3; ++d) {
