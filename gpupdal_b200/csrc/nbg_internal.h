@@ -274,7 +274,6 @@ int kd_neighbor_rows(Context* ctx, Tile* t, int K, const uint32_t* rows, uint32_
 KdOrder kd_order(const Tile* t);
 bool kd_built(const Tile* t);
 void kd_free(Context* ctx, Tile* t);
-uint64_t kd_bytes(uint64_t n);
 int kd_export(Context* ctx, Tile* t, uint32_t* vind, uint32_t* nnodes, int32_t* c1, int32_t* c2,
               int32_t* feat, double* dlo, double* dhi, uint32_t* nb, uint32_t* ne, uint32_t cap,
               cudaStream_t st);

@@ -1411,8 +1411,6 @@ static void kd_release(Context* ctx, KdForest* kd, void* p) {
         }
 }
 
-uint64_t kd_bytes(uint64_t n) { return n * 28 + (n / 16 + 1024) * 68; }
-
 static void kd_forest_free(Context* ctx, KdForest* f) {
     for (auto& b : f->blocks) ctx_free(ctx, b.first, b.second);
     delete f;
@@ -1646,7 +1644,7 @@ static int kd_build(Context* ctx, KdForest* kd, Tile* const* tiles, cudaStream_t
         if (rc) return rc;
     }
     // divlow / divhigh from the children's extents
-    kd_div_kernel<<<grid_for(ctx, kd->node_cap / 8), 256, 0, st>>>(kd->state, kd->c1, kd->c2, kd->feat, kd->bmin,
+    kd_div_kernel<<<grid_for(ctx, kd->node_cap / 16), 256, 0, st>>>(kd->state, kd->c1, kd->c2, kd->feat, kd->bmin,
                                                                    kd->bmax, kd->tfs, kd->ntree, kd->dlo, kd->dhi,
                                                                    kd->node_cap);
     NBG_LAUNCHED(1);
@@ -1714,23 +1712,24 @@ int kd_ensure_many(Context* ctx, Tile* const* tiles, int count, cudaStream_t st,
     if (!rc) rc = kd_alloc(ctx, (void**)&kd->counters, 64, kd);
     if (!rc) rc = kd_alloc(ctx, (void**)&kd->tfs, (size_t)T * sizeof(Transform), kd);
     if (!rc) rc = kd_alloc(ctx, (void**)&kd->bases, (size_t)T * 8, kd);
-    if (!rc) rc = kd_alloc_nodes(ctx, kd, (uint32_t)(n / 16 + 1024 + 2 * (uint64_t)T));
-    if (!rc) {
-        rc = kd_build(ctx, kd, todo.data(), st);
-        if (rc == KD_RETRY) {
-            // a very uneven tree outgrew the node or subtree lists: build it again
-            // with room for every node it can have
-            kd_release(ctx, kd, kd->small);
-            kd->small_cap = (uint32_t)(n + T);
-            rc = kd_alloc(ctx, (void**)&kd->small, (size_t)kd->small_cap * sizeof(KdSeg), kd);
-            if (!rc)
-                rc = kd_alloc_nodes(ctx, kd, (uint32_t)std::min<uint64_t>(2 * n + 64 + 2 * (uint64_t)T, UINT32_MAX));
-            if (!rc) rc = kd_build(ctx, kd, todo.data(), st);
-            if (rc == KD_RETRY) {
-                set_err(ctx, "KD replica build ran out of node capacity");
-                rc = NBG_ERR_UNSUPPORTED;
-            }
+    // room for leaves of 16 points on average (ordinary clouds, and clusters nested
+    // at every scale, have 50 to 70 to a leaf)
+    if (!rc) rc = kd_alloc_nodes(ctx, kd, (uint32_t)(n / 8 + 1024 + 2 * (uint64_t)T));
+    if (!rc) rc = kd_build(ctx, kd, todo.data(), st);
+    while (rc == KD_RETRY) {
+        // a more uneven tree outgrew the node or subtree lists: build it again with
+        // twice the room, up to one for every point
+        const uint64_t nodes = std::min<uint64_t>(2 * n + 64 + 2 * (uint64_t)T, UINT32_MAX), smalls = n + T;
+        if (kd->node_cap >= nodes && kd->small_cap >= smalls) {
+            set_err(ctx, "KD replica build ran out of node capacity");
+            rc = NBG_ERR_UNSUPPORTED;
+            break;
         }
+        kd_release(ctx, kd, kd->small);
+        kd->small_cap = (uint32_t)std::min<uint64_t>(2 * (uint64_t)kd->small_cap, smalls);
+        rc = kd_alloc(ctx, (void**)&kd->small, (size_t)kd->small_cap * sizeof(KdSeg), kd);
+        if (!rc) rc = kd_alloc_nodes(ctx, kd, (uint32_t)std::min<uint64_t>(2 * (uint64_t)kd->node_cap, nodes));
+        if (!rc) rc = kd_build(ctx, kd, todo.data(), st);
     }
     if (rc) {
         kd_forest_free(ctx, kd);

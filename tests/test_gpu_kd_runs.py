@@ -1,7 +1,9 @@
 """The KD replica where a segment's split falls among points at its cut (odd
 columns of a raster, coincident points), at the level passes (segments above
 4096 points): runs read by one warp and by all, several a level, in short and
-long tiles; and trees of very uneven leaves.  The exported tree equals the
+long tiles; and trees of uneven leaves,
+one of them past the room that the nodes get at first
+(of those the point order is compared).  The exported tree equals the
 oracle's."""
 import numpy as np
 import pytest
@@ -31,12 +33,18 @@ def _cloud(kind):
         s = np.exp(rng.uniform(0, np.log(8e6), 50_000))
         d = rng.normal(size=(3, 50_000))
         return tuple(np.round(d / np.linalg.norm(d, axis=0) * s))
+    if kind.startswith("peeled"):  # places whose splits take off one point at a time
+        places, bits, pile = (1024, 14, 101) if kind == "peeled" else (2048, 13, 88)
+        arms = [np.eye(3, dtype=np.int64)[d] << k for d in range(3) for k in range(1, bits - 1 if d == 0 else 23)]
+        one = np.concatenate((arms, np.zeros((pile, 3), np.int64)))
+        at = np.arange(places)[:, None] * np.array((1 << bits, 0, 0))
+        return tuple((at[:, None] + one[None]).reshape(-1, 3).T)
     w, h, flat = {"raster": (101, 99, False), "flat": (201, 203, True), "wide": (601, 401, False),
                   "long tiles": (1801, 1601, False)}[kind]
     return _raster(w, h, flat=flat)
 
 
-@pytest.mark.parametrize("kind", ("raster", "flat", "wide", "long tiles", "coincident", "stack", "columns", "nested"))
+@pytest.mark.parametrize("kind", ("raster", "flat", "wide", "long tiles", "coincident", "stack", "columns", "nested", "peeled", "peeled more"))
 def test_kd_replica_with_runs_at_the_cut(nbg, port, kind):
     xyz = [np.ascontiguousarray(v).astype(np.int32) for v in _cloud(kind)]
     tile = nbg.tile(*xyz)
@@ -44,6 +52,9 @@ def test_kd_replica_with_runs_at_the_cut(nbg, port, kind):
     tile.free()
     want = port.tree(*(U.syn.to_double(v) for v in xyz)).export()
     assert np.array_equal(vind.astype(np.uint64), want["vind"]), "point order"
+    if kind.startswith("peeled"):  # past an eighth of the points, where the nodes' room is doubled
+        assert (len(want["child1"]) > len(vind) // 8 + 1024) == (kind == "peeled more")
+        return  # (more nodes than the export holds)
     inner, winner = nodes["child1"] >= 0, want["child1"] >= 0
     cuts = [sorted(zip(*(t[k][m].tolist() for k in ("divfeat", "divlow", "divhigh")))) for t, m in
             ((nodes, inner), (want, winner))]
