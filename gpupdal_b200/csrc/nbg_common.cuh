@@ -304,7 +304,7 @@ __device__ __forceinline__ double nbg_pos_hypot(double x, double y) {
 
 // a: symmetric 3x3 (a00,a10,a11,a20,a21,a22 lower triangle).  Returns 1 on
 // success.  eval ascending; evec[c*3+r].
-static __device__ __noinline__ int nbg_eigen_chain_call(const double low[6], double eval[3], double evec[9]) {
+__device__ __forceinline__ int nbg_eigen_chain_inline(const double low[6], double eval[3], double evec[9]) {
     double m00 = low[0], m10 = low[1], m11 = low[2], m20 = low[3], m21 = low[4], m22 = low[5];
     double scale = fmax(fmax(fmax(fabs(m00), fabs(m10)), fmax(fabs(m11), fabs(m20))),
                         fmax(fabs(m21), fabs(m22)));
@@ -420,10 +420,19 @@ static __device__ __noinline__ int nbg_eigen_chain_call(const double low[6], dou
     return ok;
 }
 
+static __device__ __noinline__ int nbg_eigen_chain_call(const double low[6], double eval[3], double evec[9]) {
+    return nbg_eigen_chain_inline(low, eval, evec);
+}
+
 // A call, not inlined: few rows take the chain, and with its four copies in a
 // finish kernel the common path waited for instructions.  The arrays are
-// copied around the call, so that the caller's stay in registers.
+// copied around the call, so that the caller's stay in registers.  INLINE for
+// the radius kernel, where the call costs the scan more than the copies do (1M
+// terrain points, normals, radius 1: 0.97 -> 0.87 ms; the fused kNN kernel is the
+// other way round, 500k points 0.89 against 0.97).
+template <bool INLINE = false>
 __device__ __forceinline__ int nbg_eigen_chain(const double low[6], double eval[3], double evec[9]) {
+    if (INLINE) return nbg_eigen_chain_inline(low, eval, evec);
     double c[6], e[3], v[9];
 #pragma unroll
     for (int i = 0; i < 6; ++i) c[i] = low[i];
@@ -596,6 +605,7 @@ __device__ __forceinline__ void nbg_store(const StageDev& st, uint32_t id, int d
 
 // Md = n*S2 - S1*S1^T of the neighbours' raw offsets (exact integers, as
 // doubles), lower triangle m00, m10, m11, m20, m21, m22.
+template <bool INLINE = false>
 __device__ inline void nbg_finish_row_d(const StageGroup& g, const Transform& tf,
                                         const ExceptionSink& ex, uint32_t id, int nnb,
                                         const double Md[6], const int32_t qraw[3]) {
@@ -619,10 +629,10 @@ __device__ inline void nbg_finish_row_d(const StageGroup& g, const Transform& tf
     int ok = 1;
     if (!zero) {
         if (nonfinite) ok = 0;
-        else if (g.sign_exact) ok = nbg_eigen_chain(C, ev, V);
+        else if (g.sign_exact) ok = nbg_eigen_chain<INLINE>(C, ev, V);
         else if (!nbg_eigen_fast(C, ev, V)) {
             if (g.resolve_count) atomicAdd(g.resolve_count, 1u);
-            ok = nbg_eigen_chain(C, ev, V);
+            ok = nbg_eigen_chain<INLINE>(C, ev, V);
         }
     }
     double p[3] = {ref_coord(qraw[0], tf.scale[0], tf.offset[0]),
@@ -649,7 +659,7 @@ __device__ inline void nbg_finish_row_d(const StageGroup& g, const Transform& tf
                 if (!g.sign_exact &&
                     fabs(dot) <= 1e-12 * (fabs(dx) + fabs(dy) + fabs(dz))) {
                     double ev2[3], V2[9];
-                    if (nbg_eigen_chain(C, ev2, V2)) {
+                    if (nbg_eigen_chain<INLINE>(C, ev2, V2)) {
                         n0 = V2[0]; n1 = V2[1]; n2 = V2[2];
                         dot = __dadd_rn(__dadd_rn(__dmul_rn(dx, n0), __dmul_rn(dy, n1)),
                                         __dmul_rn(dz, n2));
@@ -660,7 +670,7 @@ __device__ inline void nbg_finish_row_d(const StageGroup& g, const Transform& tf
                 // horizontal normal: same rule as above, the chain's sign stands
                 if (!g.sign_exact && fabs(n2) <= 1e-12) {
                     double ev2[3], V2[9];
-                    if (nbg_eigen_chain(C, ev2, V2)) { n0 = V2[0]; n1 = V2[1]; n2 = V2[2]; }
+                    if (nbg_eigen_chain<INLINE>(C, ev2, V2)) { n0 = V2[0]; n1 = V2[1]; n2 = V2[2]; }
                 }
                 if (n2 < 0) { n0 = -n0; n1 = -n1; n2 = -n2; }
             }
@@ -690,7 +700,7 @@ __device__ inline void nbg_finish_row_d(const StageGroup& g, const Transform& tf
             }
             if (zero && any) {
                 double e2[3], V2[9];
-                if (nbg_eigen_chain(C, e2, V2)) { a0 = fabs(e2[0]); a1 = fabs(e2[1]); a2 = fabs(e2[2]); }
+                if (nbg_eigen_chain<INLINE>(C, e2, V2)) { a0 = fabs(e2[0]); a1 = fabs(e2[1]); a2 = fabs(e2[2]); }
             } else if (!zero && ok) {
                 a0 = fabs(ev[0]);
                 a1 = fabs(ev[1]);

@@ -1252,7 +1252,7 @@ __global__ void __launch_bounds__(128) knn_radius_kernel(const RadiusArgs a) {
     const double Md[6] = {m_entry(n, f.sxx, f.s1x, f.s1x), m_entry(n, f.syx, f.s1y, f.s1x),
                           m_entry(n, f.syy, f.s1y, f.s1y), m_entry(n, f.szx, f.s1z, f.s1x),
                           m_entry(n, f.szy, f.s1z, f.s1y), m_entry(n, f.szz, f.s1z, f.s1z)};
-    nbg_finish_row_d(a.grp, a.tf, a.ex, id, (int)min(f.cnt, 0x7FFFFFFFu), Md, f.qraw);
+    nbg_finish_row_d<true>(a.grp, a.tf, a.ex, id, (int)min(f.cnt, 0x7FFFFFFFu), Md, f.qraw);
 }
 
 int launch_radius(Context* ctx, const RadiusLaunch& rl, cudaStream_t stream) {
