@@ -36,9 +36,10 @@ struct GridParams {
 // Offset bits of the single-pass select's keys for cell edge c: the squared
 // distance field (27 - ob bits) holds (2.2 c)^2, the search's reach at ring 2.
 __host__ __device__ inline uint32_t loc_offset_bits(int32_t c) {
-    const double e = c < 1 ? 1.0 : (double)c, need = 4.84 * e * e;
+    const uint64_t e = c < 1 ? 1u : c > 8192 ? 8192u : (uint64_t)c;
+    const uint64_t need = (484u * e * e + 99u) / 100u;  // bits: the least with 2^bits >= need
     int bits = 1;
-    while (bits < 27 && (double)(1u << bits) < need) ++bits;
+    while (bits < 27 && (1ull << bits) < need) ++bits;
     return bits > 21 ? 6u : bits < 11 ? 16u : (uint32_t)(27 - bits);
 }
 

@@ -127,9 +127,9 @@ __device__ GridParams grid_config(const int32_t* bb, uint64_t n, int k1, float c
     // one's k1 nearest lie (at its own planar density) beyond 0.8 of the group
     // select's
     g.full = 1u << loc_offset_bits(g.cell);
-    const double m = 0.8 * group_max_margin(k1 + 1);
-    g.thin = (uint32_t)fmin(4.0e9, k1 * c * c / (3.14159265358979 * m * m));
-    g.heavy = (uint32_t)fmin(4.0e9, 256.0 * fmax(1.0, (double)n / (double)g.ncols));
+    const float m = 0.8f * (float)group_max_margin(k1 + 1), cf = (float)g.cell;
+    g.thin = (uint32_t)fminf(4.0e9f, (float)k1 * cf * cf / (3.14159265f * m * m));
+    g.heavy = (uint32_t)fminf(4.0e9f, 256.0f * fmaxf(1.0f, (float)n / (float)g.ncols));
     g.in_full = g.in_thin = g.in_heavy = g.cells = 0;
     return g;
 }
