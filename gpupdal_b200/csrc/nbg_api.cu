@@ -559,7 +559,7 @@ extern "C" int nbg_tile_set_select(nbg_context* h, nbg_tile* th, int32_t select_
     if (!valid_select(select_kernel))
         return fail(&h->c, NBG_ERR_INVALID, "select kernel must be 0, 1, 2, 8, 16 or 32");
     if (!(first_margin > 0.0f && first_margin <= 16.0f))
-        return fail(&h->c, NBG_ERR_INVALID, "first margin must be in (0, 16] cell edges");
+        return fail(&h->c, NBG_ERR_INVALID, "first margin must be in (0, 16]");
     std::lock_guard<std::mutex> lock(h->c.mu);
     th->t.group = select_kernel;
     th->t.margin0 = first_margin;

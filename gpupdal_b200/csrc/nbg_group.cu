@@ -234,7 +234,8 @@ __device__ __forceinline__ void group_warp(const QueryArgs& a, const uint64_t s0
     if (S::kMemClumps == 3) mem0 -= (c0 >> 1) & 1u;
     mem0 = min(mem0, nclumps - want);
     const uint32_t own = c0 >> 5;  // the block a walk starts with
-    const int mcap = (int)(margin0 * 8.0f * g.r1 * sqrtf((float)a.K)) + 1;
+    // (beyond 3 kMaxMargin it limits neither a margin nor a round's span)
+    const int mcap = (int)fminf(margin0 * 8.0f * g.r1 * sqrtf((float)a.K), 3.0f * S::kMaxMargin) + 1;
     bool again = false;      // the lane's list started over: members are not in it
     bool in = !done;         // takes part in the current round
     bool members = true;     // (uniform) the current list is the members'
