@@ -689,15 +689,17 @@ __global__ void __launch_bounds__(128) knn_retry_thread_kernel(const QueryArgs a
         select_row<KS, true>(a, __ldg(&a.rows[r]));
 }
 
-// The same for the tiles of a batch: job blockIdx.y's rows.
+// The same for the tiles of a batch: blockIdx.y's jobs, gridDim.y apart.
 template <int KS>
 __global__ void __launch_bounds__(128) knn_retry_thread_batch_kernel(const BatchJob* __restrict__ jobs, int njobs,
                                                                      uint32_t least) {
     if (retry_total(jobs, njobs) < least) return;
-    const QueryArgs& a = jobs[blockIdx.y].q;
-    const uint32_t nr = a.counters[6];
-    for (uint32_t r = blockIdx.x * blockDim.x + threadIdx.x; r < nr; r += gridDim.x * blockDim.x)
-        select_row<KS, true>(a, a.retry_rows[r]);
+    for (int j = blockIdx.y; j < njobs; j += gridDim.y) {
+        const QueryArgs& a = jobs[j].q;
+        const uint32_t nr = a.counters[6];
+        for (uint32_t r = blockIdx.x * blockDim.x + threadIdx.x; r < nr; r += gridDim.x * blockDim.x)
+            select_row<KS, true>(a, a.retry_rows[r]);
+    }
 }
 
 struct RetryArgs {
@@ -705,7 +707,7 @@ struct RetryArgs {
     const BatchJob* jobs;  // or the jobs of a batch
     int njobs;
     uint32_t least;
-    unsigned blocks;  // (per job)
+    dim3 grid;
     cudaStream_t stream;
 };
 
@@ -714,10 +716,9 @@ struct RetryLauncher {
     using Args = RetryArgs;
     static int run(const RetryArgs& r) {
         if (r.jobs)
-            knn_retry_thread_batch_kernel<KS>
-                <<<dim3(r.blocks, (unsigned)r.njobs), 128, 0, r.stream>>>(r.jobs, r.njobs, r.least);
+            knn_retry_thread_batch_kernel<KS><<<r.grid, 128, 0, r.stream>>>(r.jobs, r.njobs, r.least);
         else
-            knn_retry_thread_kernel<KS><<<r.blocks, 128, 0, r.stream>>>(r.q, r.least);
+            knn_retry_thread_kernel<KS><<<r.grid, 128, 0, r.stream>>>(r.q, r.least);
         NBG_LAUNCHED(1);
         return cudaGetLastError() == cudaSuccess ? NBG_OK : NBG_ERR_CUDA;
     }
@@ -1322,13 +1323,15 @@ bool located_keys_fit(const Tile* t) {
 // (slots = K + 1 of the widest row)
 int launch_retry_threads(const QueryArgs& q, int slots, uint32_t least, int sms, cudaStream_t stream) {
     const unsigned blocks = (unsigned)std::min<uint64_t>((q.nq + 127) / 128, (uint64_t)sms * 16);
-    return dispatch_slots<RetryLauncher>(slots - 1, RetryArgs{q, nullptr, 0, least, blocks, stream});
+    return dispatch_slots<RetryLauncher>(slots - 1, RetryArgs{q, nullptr, 0, least, dim3(blocks), stream});
 }
+
+dim3 retry_batch_grid(int njobs, int sms);  // nbg_rows.cu
 
 int launch_retry_threads_batch(int slots, const BatchJob* jobs, int njobs, uint32_t least, int sms,
                                cudaStream_t stream) {
-    const unsigned blocks = (unsigned)std::max<uint64_t>(4, (uint64_t)sms * 16 / (uint64_t)njobs);
-    return dispatch_slots<RetryLauncher>(slots - 1, RetryArgs{QueryArgs{}, jobs, njobs, least, blocks, stream});
+    return dispatch_slots<RetryLauncher>(
+        slots - 1, RetryArgs{QueryArgs{}, jobs, njobs, least, retry_batch_grid(njobs, sms), stream});
 }
 
 struct LaunchArgs {

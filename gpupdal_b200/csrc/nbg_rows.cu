@@ -316,14 +316,16 @@ __global__ void __launch_bounds__(kRowThreads) knn_retry_finish_kernel(const Que
     retry_finish_rows<NR>(a, a.rows, *a.nq_dev, s_gather);
 }
 
-// The same for the tiles of a batch: job blockIdx.y's rows.
+// The same for the tiles of a batch: blockIdx.y's jobs, gridDim.y apart.
 template <int NR>
 __global__ void __launch_bounds__(kRowThreads) knn_retry_batch_kernel(const BatchJob* __restrict__ jobs, int njobs,
                                                                       uint32_t most) {
     __shared__ uint32_t s_gather[kRowThreads / 32][64];
     if (most != 0xFFFFFFFFu && retry_total(jobs, njobs) >= most) return;
-    const QueryArgs& a = jobs[blockIdx.y].q;
-    retry_finish_rows<NR>(a, a.retry_rows, a.counters[6], s_gather);
+    for (int j = blockIdx.y; j < njobs; j += gridDim.y) {
+        const QueryArgs& a = jobs[j].q;
+        retry_finish_rows<NR>(a, a.retry_rows, a.counters[6], s_gather);
+    }
 }
 
 // One tie row by a warp (see tie_row): the sums over its K points, in every
@@ -525,6 +527,13 @@ int launch_retry_finish(const QueryArgs& q, int slots, int sms, cudaStream_t str
     return cudaGetLastError() == cudaSuccess ? NBG_OK : NBG_ERR_CUDA;
 }
 
+// Blocks for a batch's jobs, at least four a job; more jobs than fill the GPU so
+// take turns (gridDim.y ends at 65535).
+dim3 retry_batch_grid(int njobs, int sms) {
+    const unsigned y = (unsigned)std::min<uint64_t>((uint64_t)njobs, (uint64_t)sms * kRowBlocksPerSm / 4);
+    return dim3((unsigned)((uint64_t)sms * kRowBlocksPerSm / y), y);
+}
+
 // `rows`: the rows of the jobs' tiles.
 int launch_retry_batch(int slots, const BatchJob* jobs, int njobs, uint64_t rows, int sms, cudaStream_t stream) {
     if (!njobs) return NBG_OK;
@@ -535,8 +544,7 @@ int launch_retry_batch(int slots, const BatchJob* jobs, int njobs, uint64_t rows
     } else {
         many = 0xFFFFFFFFu;  // (there cannot be as many)
     }
-    const dim3 grid((unsigned)std::max<uint64_t>(4, (uint64_t)sms * kRowBlocksPerSm / (uint64_t)njobs),
-                    (unsigned)njobs);
+    const dim3 grid = retry_batch_grid(njobs, sms);
     if (slots <= 32) knn_retry_batch_kernel<1><<<grid, kRowThreads, 0, stream>>>(jobs, njobs, many);
     else if (slots <= 64) knn_retry_batch_kernel<2><<<grid, kRowThreads, 0, stream>>>(jobs, njobs, many);
     else knn_retry_batch_kernel<3><<<grid, kRowThreads, 0, stream>>>(jobs, njobs, many);
