@@ -342,10 +342,8 @@ __device__ __forceinline__ bool warp_tie(const TieArgs& a, const GridParams& g, 
     int less = 0;
     uint32_t gcnt = 0, gid = 0;  // the group's size; this lane's member
     int g0 = 0, g1 = 0, g2 = 0;
-    // (a group of more than 32 goes to the search replay: nothing more is read)
-    for (int r = 0; r <= R && gcnt <= 32u; ++r)
+    for (int r = 0; r <= R; ++r)
         warp_ring(a.gv, g, qc, r, (unsigned long long)(kk - KEY_BASE), [&](const float4 p, bool in) {
-            if (gcnt > 32u) return;
             const float dx = p.x - qx, dy = p.y - qy, dz = p.z - qz;
             const uint32_t key = in ? dist_key(dx, dy, dz) : 0xFFFFFFFFu;
             if (key < kk) {
@@ -353,11 +351,8 @@ __device__ __forceinline__ bool warp_tie(const TieArgs& a, const GridParams& g, 
                 ++less;
             }
             unsigned b = __ballot_sync(kAll, key == kk);
-            if (gcnt + __popc(b) > 32u) {
-                gcnt = 33;
-                return;
-            }
-            while (b) {  // the lane of the member's number takes it
+            // (past 32 the row goes to the search replay)
+            while (b && gcnt <= 32u) {  // the lane of the member's number takes it
                 const int src = __ffs(b) - 1;
                 b &= b - 1;
                 const float mx = __shfl_sync(kAll, dx, src), my = __shfl_sync(kAll, dy, src),
