@@ -1423,15 +1423,22 @@ static std::pair<int, int> tuning_class(const Tile* t, int K) {
 // The library's choice for a tile nobody tuned.  Whole calls on fresh tiles, ms,
 // per-thread two-pass (0) / single pass (2) / group (32):
 //   K = 9    2M mixture 3.02 / 2.41 / 2.90     16M stress 25.2 / 19.3 / 25.6
-//   K = 17   2M mixture 3.55 / 3.39 / 3.04     32M stress 56.0 / 50.4 / 53.3
+//   K = 14   2M mixture 3.37 / 3.03 / 3.08     16M mixture 22.3 / 19.9 / 21.3
+//   K = 17, 128 points / m^2:
+//      stress    2M 4.54 / 4.09 / 3.73   8M 15.6 / 13.6 / 13.6   16M 29.4 / 25.9 / 26.5   32M 57.7 / 50.2 / 53.3
+//      mixture   2M 4.58 / 3.87 / 3.51   8M 15.4 / 13.1 / 12.8   16M 28.7 / 24.8 / 25.0   32M 56.0 / 48.0 / 50.2
+//      terrain   2M 4.12 / 3.76 / 2.68   8M 14.3 / 12.9 /  8.4   16M 27.1 / 24.7 / 16.1   32M 54.8 / 49.9 / 33.1
 //   K = 25   2M mixture 4.73 / 5.25 / 3.69     2M stress  5.58 / 5.18 / 4.46
 //   K = 33   2M mixture 6.76 / 15.6 / 4.50     300k terrain 1.47 / 3.5 / 0.93
 // The single pass pays one min/max per list slot and candidate and wins while the
 // list is short (from 16M points also at 18 slots: the replica built beside it
 // gets more of the SMs than beside the group select's shared memory), as long as
-// its keys hold a column; the group select sorts batches and wins above.  A chunk
-// holds a fraction of each clump, so the group select's bounds are loose there
-// (6M stress records, K = 17: 18.8 ms against 17.4 with the two-pass search).
+// its keys hold a column; the group select sorts batches and wins above.  On bare
+// ground, where its clumps are flat, it wins by far: at 18 slots a tile of less than a
+// cell to 25 points takes it at any size (ground has 0.014 to 0.024 cells a point,
+// the mixed clouds 0.09 to 0.45).  A chunk holds a fraction of each clump, so the
+// group select's bounds are loose there (6M stress records, K = 17: 18.8 ms against
+// 17.4 with the two-pass search).
 //
 // Both hand back what their keys cannot hold, so a tile most of whose points
 // lie where they cannot is left to the others.  The grid counts those points:
@@ -1453,8 +1460,8 @@ int select_kernel(const Tile* t, int K, bool chunks) {
     const GridParams& g = t->host_gp;
     const uint64_t n = t->n;
     const int slots = slots_for_k(K);
-    if ((slots <= 14 || (slots <= 18 && (chunks || n >= 16000000))) && located_keys_fit(t) && g.in_full <= n / 20 &&
-        g.cells <= 8 * n)
+    if ((slots <= 14 || (slots <= 18 && (chunks || (n >= 16000000 && g.cells >= n / 25)))) && located_keys_fit(t) &&
+        g.in_full <= n / 20 && g.cells <= 8 * n)
         return 2;
     if (chunks && slots < 50) return 0;
     return n >= 100000 && (g.in_thin > n / 10 || g.in_heavy > n / 2) ? 0 : 32;
