@@ -28,12 +28,10 @@
 
 namespace nbg {
 
-// `reserve`: resident blocks per SM the persistent launch leaves free, so that
-// the KD replica build on the side stream runs beside it instead of after it.
 int launch_select_queue(Context* ctx, int K, const BatchJob* jobs, int njobs, uint64_t items,
-                        unsigned long long* head, cudaStream_t stream, int reserve);
+                        unsigned long long* head, cudaStream_t stream);
 int launch_finish_queue(Context* ctx, const BatchJob* jobs, int njobs, uint64_t items,
-                        unsigned long long* head, cudaStream_t stream, int reserve);
+                        unsigned long long* head, cudaStream_t stream);
 int slots_for_k(int K);
 int launch_loc_batch(int K, const BatchJob* jobs, int njobs, uint64_t items, cudaStream_t stream);
 uint32_t located_offset_bits(const Tile* t);
@@ -379,15 +377,12 @@ extern "C" int nbg_run_batch(nbg_context* h, const nbg_batch_item* items, int32_
     cudaMemsetAsync(B->counters, 0, (size_t)nl * kCounters * sizeof(uint32_t), st);
     rc = host_to_device(ctx, B->jobs, jobs.data(), jobs.size() * sizeof(BatchJob), st);
     if (rc) return rc;
-    // tiles whose KD replica is built after the queue
+    // tiles whose KD replica is built beside the queue
     std::vector<Tile*> kd_tiles;
     for (int i : live)
         if (items[i].tile->t.n > 100 && !kd_built(&items[i].tile->t)) kd_tiles.push_back(&items[i].tile->t);
-    // the persistent launches take every resident block slot
-    const int reserve = 0;
     // ---- the queue launches, captured once per batch shape
     std::vector<uint64_t> key;
-    key.push_back((uint64_t)reserve);
     key.push_back((uint64_t)(uintptr_t)B->jobs);
     key.push_back(fin_items);
     key.push_back((uint64_t)nl);
@@ -405,7 +400,7 @@ extern "C" int nbg_run_batch(nbg_context* h, const nbg_batch_item* items, int32_
             int r = c.select == 32 ? launch_group_batch(slots_for_k(c.K), j, c.count, c.items, s)
                     : c.select == 2
                         ? launch_loc_batch(c.K, j, c.count, c.items, s)
-                        : launch_select_queue(ctx, c.K, j, c.count, c.items, B->heads + k, s, reserve);
+                        : launch_select_queue(ctx, c.K, j, c.count, c.items, B->heads + k, s);
             if (r) return r;
         }
         // rows handed back (their sums slots hold 0: the finish pass skips them)
@@ -420,7 +415,7 @@ extern "C" int nbg_run_batch(nbg_context* h, const nbg_batch_item* items, int32_
                 r = launch_retry_batch(slots_for_k(c.K), B->jobs + c.begin, c.count, 128 * c.items, ctx->sm_count,
                                        ctx->fork);
         if (!r)
-            r = launch_finish_queue(ctx, B->jobs + nl, nl, fin_items, B->heads + classes.size(), s, reserve);
+            r = launch_finish_queue(ctx, B->jobs + nl, nl, fin_items, B->heads + classes.size(), s);
         e = cudaEventRecord(ctx->fev[1], ctx->fork);
         if (!e) e = cudaStreamWaitEvent(s, ctx->fev[1], 0);
         return r ? r : e ? NBG_ERR_CUDA : NBG_OK;

@@ -609,7 +609,6 @@ struct QueueArgs {
     unsigned long long* head;
     int sms;
     cudaStream_t stream;
-    int reserve;  // resident blocks per SM left to kernels of other streams
 };
 
 template <int KS>
@@ -619,7 +618,7 @@ struct QueueLauncher {
         int per_sm = 0;
         cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, knn_select_queue_kernel<KS>, 128, 0);
         const uint64_t grid =
-            std::min<uint64_t>(q.items, (uint64_t)q.sms * std::max(per_sm - q.reserve, 1));
+            std::min<uint64_t>(q.items, (uint64_t)q.sms * std::max(per_sm, 1));
         if (!grid) return NBG_OK;
         knn_select_queue_kernel<KS><<<(unsigned)grid, 128, 0, q.stream>>>(q.jobs, q.njobs, q.items,
                                                                            q.head);
@@ -1571,9 +1570,9 @@ int build_id_chunks(Context* ctx, const Tile* t, const uint64_t* bounds, int nch
 }
 
 int launch_select_queue(Context* ctx, int K, const BatchJob* jobs, int njobs, uint64_t items,
-                        unsigned long long* head, cudaStream_t stream, int reserve) {
+                        unsigned long long* head, cudaStream_t stream) {
     return dispatch_slots<QueueLauncher>(
-        K, QueueArgs{jobs, njobs, items, head, ctx->sm_count, stream, reserve});
+        K, QueueArgs{jobs, njobs, items, head, ctx->sm_count, stream});
 }
 
 int launch_loc_batch(int K, const BatchJob* jobs, int njobs, uint64_t items, cudaStream_t stream) {
@@ -1583,11 +1582,11 @@ int launch_loc_batch(int K, const BatchJob* jobs, int njobs, uint64_t items, cud
 uint32_t located_offset_bits(const Tile* t) { return loc_offset_bits(t->host_gp.cell); }
 
 int launch_finish_queue(Context* ctx, const BatchJob* jobs, int njobs, uint64_t items,
-                        unsigned long long* head, cudaStream_t stream, int reserve) {
+                        unsigned long long* head, cudaStream_t stream) {
     int per_sm = 0;
     cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, knn_finish_queue_kernel, 128, 0);
     const uint64_t grid =
-        std::min<uint64_t>(items, (uint64_t)ctx->sm_count * std::max(per_sm - reserve, 1));
+        std::min<uint64_t>(items, (uint64_t)ctx->sm_count * std::max(per_sm, 1));
     if (!grid) return NBG_OK;
     knn_finish_queue_kernel<<<(unsigned)grid, 128, 0, stream>>>(jobs, njobs, items, head);
     NBG_LAUNCHED(1);
