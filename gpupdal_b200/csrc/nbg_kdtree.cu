@@ -1112,6 +1112,9 @@ __global__ void __launch_bounds__(KD_BTHREADS, 2) kd_block_build_kernel(
 __global__ void kd_div_kernel(const KdState* st, const int32_t* c1, const int32_t* c2, const int32_t* feat,
                               const int32_t* bmin, const int32_t* bmax, const Transform* tfs,
                               const int32_t* ntree, double* dlo, double* dhi, uint32_t cap) {
+    // (a build out of room is made again: a number drawn past the capacity's last
+    // pair has a place but no node in it)
+    if (st->errors) return;
     const uint32_t nodes = min(st->nodes, cap);
     for (uint32_t node = blockIdx.x * blockDim.x + threadIdx.x; node < nodes; node += gridDim.x * blockDim.x) {
         if (c1[node] < 0) continue;

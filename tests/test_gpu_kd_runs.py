@@ -61,3 +61,17 @@ def test_kd_replica_with_runs_at_the_cut(nbg, port, kind):
     assert cuts[0] == cuts[1], "split planes"
     leaves = sorted(zip(nodes["begin"][~inner].tolist(), nodes["end"][~inner].tolist()))
     assert leaves == sorted(zip(want["left"][~winner].tolist(), want["right"][~winner].tolist())), "leaves"
+
+
+def test_a_build_out_of_room_reads_no_node_it_did_not_write(nbg):
+    """The nodes' room ends between the two nodes of a pair: the first has a
+    place but is not written.  The context's cache is given blocks of the nodes'
+    size that hold large numbers, which a reader would take for children."""
+    xyz = [np.ascontiguousarray(v).astype(np.int32) for v in _cloud("peeled more")]
+    stale = [nbg.tile(*[np.full(40_000, 2_000_000_000, np.int32)] * 3) for _ in range(4)]
+    for tile in stale:
+        tile.free()
+    tile = nbg.tile(*xyz)
+    vind, _ = nbg.kd_export(tile)
+    assert np.array_equal(np.sort(vind), np.arange(len(vind)))
+    tile.free()
