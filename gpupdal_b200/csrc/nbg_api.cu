@@ -1305,7 +1305,8 @@ extern "C" int nbg_run(nbg_context* h, nbg_tile* th, const nbg_stage_opts* stage
         if (cnt[0] || nties) {
             if (!ties_queued) cudaEventRecord(ctx->ev[4], stream);
             rc = kd_ensure(ctx, t, stream);
-            if (!rc && nties && !ties_queued) {
+            // (a queued launch leaves many rows to the thread form)
+            if (!rc && nties && (!ties_queued || nties >= many_ties(ctx->sm_count, n))) {
                 TieLaunch tl;
                 tl.tile = t;
                 tl.K = K;
@@ -1465,6 +1466,16 @@ int select_kernel(const Tile* t, int K, bool chunks) {
         return 2;
     if (chunks && slots < 50) return 0;
     return n >= 100000 && (g.in_thin > n / 10 || g.in_heavy > n / 2) ? 0 : 32;
+}
+
+// A tile somebody tuned may have been given a select that does not fit it; on the
+// library's choice many rows come back where the single pass finds few points to a
+// cell, or the group select's keys thin or heavy columns (ordinary clouds: 0.01 - 0.5
+// cells a point, at most 0.01 % in thin columns, none in heavy ones).
+bool may_hand_back_many(const Tile* t, int select) {
+    const GridParams& g = t->host_gp;
+    if (t->group >= 0) return true;
+    return select == 2 ? g.in_full > t->n / 20 || g.cells > t->n : g.in_thin > t->n / 1000 || g.in_heavy;
 }
 
 // A tile the caller did not tune takes the context's cached choice for its

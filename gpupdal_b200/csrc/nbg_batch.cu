@@ -36,7 +36,8 @@ int slots_for_k(int K);
 int launch_loc_batch(int K, const BatchJob* jobs, int njobs, uint64_t items, cudaStream_t stream);
 uint32_t located_offset_bits(const Tile* t);
 int launch_group_batch(int slots, const BatchJob* jobs, int njobs, uint64_t items, cudaStream_t stream);
-int launch_retry_batch(int slots, const BatchJob* jobs, int njobs, uint64_t rows, int sms, cudaStream_t stream);
+int launch_retry_batch(int slots, const BatchJob* jobs, int njobs, uint64_t rows, bool may_be_many, int sms,
+                       cudaStream_t stream);
 
 static constexpr int kCounters = 64;  // u32 counters per tile
 
@@ -315,6 +316,7 @@ extern "C" int nbg_run_batch(nbg_context* h, const nbg_batch_item* items, int32_
         int K, select;
         int begin, count;
         uint64_t items;
+        bool many;  // may_hand_back_many of a tile
     };
     std::vector<Cls> classes;
     uint64_t fin_items = 0;
@@ -346,7 +348,7 @@ extern "C" int nbg_run_batch(nbg_context* h, const nbg_batch_item* items, int32_
         q.sums = B->sums + row0[i];
         const uint64_t blocks = (t->n + 127) / 128;
         if (classes.empty() || class_of(order[j - 1]) != class_of(i))
-            classes.push_back(Cls{Ks[i], select[i], j, 0, 0});
+            classes.push_back(Cls{Ks[i], select[i], j, 0, 0, false});
         Cls& c = classes.back();
         jobs[j].q = q;
         jobs[j].first = c.items;
@@ -354,6 +356,7 @@ extern "C" int nbg_run_batch(nbg_context* h, const nbg_batch_item* items, int32_
         jobs[j].margin = t->margin0;
         c.items += blocks;
         c.count += 1;
+        c.many = c.many || may_hand_back_many(t, select[i]);
         jobs[nl + j].q = q;
         jobs[nl + j].first = fin_items;
         fin_items += blocks;
@@ -387,7 +390,7 @@ extern "C" int nbg_run_batch(nbg_context* h, const nbg_batch_item* items, int32_
     key.push_back(fin_items);
     key.push_back((uint64_t)nl);
     for (const Cls& c : classes) {
-        key.push_back((uint64_t)slots_for_k(c.K) * 64 + (uint64_t)c.select);
+        key.push_back(((uint64_t)slots_for_k(c.K) * 64 + (uint64_t)c.select) * 2 + (c.many ? 1 : 0));
         key.push_back((uint64_t)c.begin);
         key.push_back((uint64_t)c.count);
         key.push_back(c.items);
@@ -412,8 +415,8 @@ extern "C" int nbg_run_batch(nbg_context* h, const nbg_batch_item* items, int32_
         int r = NBG_OK;
         for (const Cls& c : classes)
             if (c.select && !r)
-                r = launch_retry_batch(slots_for_k(c.K), B->jobs + c.begin, c.count, 128 * c.items, ctx->sm_count,
-                                       ctx->fork);
+                r = launch_retry_batch(slots_for_k(c.K), B->jobs + c.begin, c.count, 128 * c.items, c.many,
+                                       ctx->sm_count, ctx->fork);
         if (!r)
             r = launch_finish_queue(ctx, B->jobs + nl, nl, fin_items, B->heads + classes.size(), s);
         e = cudaEventRecord(ctx->fev[1], ctx->fork);

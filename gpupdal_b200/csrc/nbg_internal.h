@@ -218,15 +218,20 @@ struct TieLaunch {
     const double* row_k = nullptr;
 };
 int launch_ties(Context* ctx, const TieLaunch& tl, cudaStream_t stream);
+// From this many of a query's `rows` up its tie rows get a thread each.
+uint32_t many_ties(int sms, uint64_t rows);
 // The same with the row count read on the device: min(*count, tl.nties) rows
 // (tl.nties: the list's capacity), so the launch can be queued before the
-// query that fills the list has finished.
+// query that fills the list has finished.  A count of many_ties() or more is
+// left to launch_ties, once the caller has read it.
 int launch_ties_counted(Context* ctx, const TieLaunch& tl, const uint32_t* count, cudaStream_t stream);
 // The select kernel a launch over `t` (its grid built) with K neighbours takes:
 // the tile's own setting, else the library's choice.  `chunks`: the launches
 // answer the rows of id-range chunks.
 int select_kernel(const Tile* t, int K, bool chunks);
 bool located_keys_fit(const Tile* t);
+// False for a tile whose grid says that this select hands few rows back.
+bool may_hand_back_many(const Tile* t, int select);
 // The clump order of the tile's current grid (group select).
 int ensure_clumps(Context* ctx, Tile* t, cudaStream_t stream);
 // True when launch_query answers `q`'s handed-back rows on the context's fork

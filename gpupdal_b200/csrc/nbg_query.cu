@@ -880,13 +880,10 @@ __device__ __forceinline__ void tie_row(const TieArgs& a, uint32_t r) {
     nbg_finish_row(a.grp, a.tf, a.ex, id, (int)n, M, qraw);
 }
 
-// A thread per tie row (the count as in knn_tie_kernel).  With `least` the launch
-// stands beside that of the warp form, and the one whose range holds the count
-// answers the rows.
-__global__ void __launch_bounds__(128) knn_tie_thread_kernel(const TieArgs a, const uint32_t* count, uint32_t least) {
-    const uint32_t nt = count ? min(*count, a.nties) : a.nties;
-    if (nt < least) return;
-    for (uint32_t r = blockIdx.x * blockDim.x + threadIdx.x; r < nt; r += gridDim.x * blockDim.x) tie_row(a, r);
+// A thread per tie row.
+__global__ void __launch_bounds__(128) knn_tie_thread_kernel(const TieArgs a) {
+    const uint32_t r = blockIdx.x * blockDim.x + threadIdx.x;
+    if (r < a.nties) tie_row(a, r);
 }
 
 // The same over many tiles: jobs[j]'s rows are entries first[j] .. first[j+1]-1
@@ -904,11 +901,8 @@ __global__ void __launch_bounds__(128) knn_tie_thread_batch_kernel(const TieArgs
     tie_row(jobs[lo], (uint32_t)(t - first[lo]));
 }
 
-int launch_tie_threads(const TieArgs& a, const uint32_t* count, uint32_t least, int sms, cudaStream_t stream) {
-    // (a count read on the device may be far below the capacity: rows in strides)
-    const uint64_t all = ((uint64_t)a.nties + 127) / 128;
-    const unsigned blocks = (unsigned)(count ? std::min<uint64_t>(all, (uint64_t)sms * 16) : all);
-    knn_tie_thread_kernel<<<blocks, 128, 0, stream>>>(a, count, least);
+int launch_tie_threads(const TieArgs& a, cudaStream_t stream) {
+    knn_tie_thread_kernel<<<(a.nties + 127) / 128, 128, 0, stream>>>(a);
     NBG_LAUNCHED(1);
     return cudaGetLastError() == cudaSuccess ? NBG_OK : NBG_ERR_CUDA;
 }
@@ -946,7 +940,7 @@ static TieArgs tie_args(const TieLaunch& tl) {
 // nbg_rows.cu
 int launch_tie_rows(const TieArgs& a, const uint32_t* count, int sms, cudaStream_t stream);
 int launch_tie_batch(Context* ctx, const std::vector<TieArgs>& jobs, cudaStream_t stream);
-int launch_retry_finish(const QueryArgs& q, int slots, int sms, cudaStream_t stream);
+int launch_retry_finish(const QueryArgs& q, int slots, bool may_be_many, int sms, cudaStream_t stream);
 
 int launch_ties(Context* ctx, const TieLaunch& tl, cudaStream_t stream) {
     return launch_ties_counted(ctx, tl, nullptr, stream);
@@ -1344,6 +1338,7 @@ struct LaunchArgs {
     float margin0 = 0.25f;
     int sms = 148;
     uint32_t ob = 11;     // single-pass select: offset bits of a key
+    bool may_be_many = false;  // the handed-back rows (may_hand_back_many)
 };
 
 int launch_group_select(const QueryArgs& q, int slots, float margin0, cudaStream_t stream);
@@ -1380,7 +1375,7 @@ struct KnnLauncher {
             r.nq_dev = la.q.counters + 6;
             r.nq = rows;
             if (!la.fork) {
-                const int rc = launch_retry_finish(r, KS, la.sms, la.stream);
+                const int rc = launch_retry_finish(r, KS, la.may_be_many, la.sms, la.stream);
                 if (rc) return rc;
                 knn_finish_kernel<<<(unsigned)blocks, threads, 0, la.stream>>>(la.q);
                 NBG_LAUNCHED(1);
@@ -1392,7 +1387,7 @@ struct KnnLauncher {
             cudaError_t e = cudaEventRecord(la.fev[0], la.stream);
             if (!e) e = cudaStreamWaitEvent(la.fork, la.fev[0], 0);
             if (e) return NBG_ERR_CUDA;
-            const int rc = launch_retry_finish(r, KS, la.sms, la.fork);
+            const int rc = launch_retry_finish(r, KS, la.may_be_many, la.sms, la.fork);
             if (rc) return rc;
             knn_finish_kernel<<<(unsigned)blocks, threads, 0, la.stream>>>(la.q);
             NBG_LAUNCHED(1);
@@ -1493,6 +1488,7 @@ int launch_query(Context* ctx, const QueryLaunch& ql, cudaStream_t stream) {
     la.margin0 = ql.margin0;
     la.sms = ctx ? ctx->sm_count : 148;
     la.ob = loc_offset_bits(ql.tile->host_gp.cell);
+    la.may_be_many = may_hand_back_many(ql.tile, la.group);
     const int rc = dispatch_slots<KnnLauncher>(ql.K, la);
     // a forked launch records `done` itself, on the fork stream
     if (!rc && ql.done && !query_forks(ctx, ql) && cudaEventRecord(ql.done, stream) != cudaSuccess)

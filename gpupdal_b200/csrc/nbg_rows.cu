@@ -440,7 +440,7 @@ __device__ __forceinline__ void warp_tie_rows(const TieArgs& a, uint32_t r0, uin
 }
 
 // Tie rows counted on the device (a.nties: the list's capacity), or a.nties
-// rows when `count` is null; `most` rows or more are left to the thread form.
+// rows when `count` is null; a count of `most` or more is left to the thread form.
 __global__ void __launch_bounds__(kRowThreads) knn_tie_kernel(const TieArgs a, const uint32_t* count, uint32_t most) {
     const uint32_t nt = count ? min(*count, a.nties) : a.nties;
     if (nt >= most) return;
@@ -472,7 +472,7 @@ __global__ void __launch_bounds__(kRowThreads) knn_tie_batch_kernel(const TieArg
 static constexpr uint64_t kRowBlocksPerSm = 16;
 
 // nbg_query.cu: a thread per row
-int launch_tie_threads(const TieArgs& a, const uint32_t* count, uint32_t least, int sms, cudaStream_t stream);
+int launch_tie_threads(const TieArgs& a, cudaStream_t stream);
 int launch_tie_threads_batch(const TieArgs* jobs, const uint64_t* first, int njobs, uint64_t rows,
                              cudaStream_t stream);
 int launch_retry_threads(const QueryArgs& q, int slots, uint32_t least, int sms, cudaStream_t stream);
@@ -506,9 +506,10 @@ uint32_t many_retries(int sms, int slots, uint64_t rows) {
     return (uint32_t)std::max<uint64_t>((uint64_t)sms * 512, slots > 64 ? rows / 2 : rows / 5);
 }
 
-int launch_retry_finish(const QueryArgs& q, int slots, int sms, cudaStream_t stream) {
+// may_be_many: the thread form is launched too (an idle launch costs 3 us)
+int launch_retry_finish(const QueryArgs& q, int slots, bool may_be_many, int sms, cudaStream_t stream) {
     const uint64_t rows = q.nq;  // the most there can be
-    const uint32_t many = many_retries(sms, slots, rows);
+    const uint32_t many = may_be_many ? many_retries(sms, slots, rows) : 0xFFFFFFFFu;
     if (rows >= many) {
         const int rc = launch_retry_threads(q, slots, many, sms, stream);
         if (rc) return rc;
@@ -530,10 +531,11 @@ dim3 retry_batch_grid(int njobs, int sms) {
 }
 
 // `rows`: the rows of the jobs' tiles.
-int launch_retry_batch(int slots, const BatchJob* jobs, int njobs, uint64_t rows, int sms, cudaStream_t stream) {
+int launch_retry_batch(int slots, const BatchJob* jobs, int njobs, uint64_t rows, bool may_be_many, int sms,
+                       cudaStream_t stream) {
     if (!njobs) return NBG_OK;
     uint32_t many = many_retries(sms, slots, rows);
-    if (rows >= many) {
+    if (may_be_many && rows >= many) {
         const int rc = launch_retry_threads_batch(slots, jobs, njobs, many, sms, stream);
         if (rc) return rc;
     } else {
@@ -549,11 +551,7 @@ int launch_retry_batch(int slots, const BatchJob* jobs, int njobs, uint64_t rows
 
 int launch_tie_rows(const TieArgs& a, const uint32_t* count, int sms, cudaStream_t stream) {
     const uint32_t many = many_ties(sms, a.of_rows);
-    if (a.ids_out) return launch_tie_threads(a, count, 0, sms, stream);
-    if (a.nties >= many) {
-        const int rc = launch_tie_threads(a, count, many, sms, stream);
-        if (rc || !count) return rc;
-    }
+    if (a.ids_out || (!count && a.nties >= many)) return launch_tie_threads(a, stream);
     const unsigned blocks =
         (unsigned)std::max<uint64_t>(1, std::min<uint64_t>(((uint64_t)a.nties + 3) / 4, (uint64_t)sms * kRowBlocksPerSm));
     knn_tie_kernel<<<blocks, kRowThreads, 0, stream>>>(a, count, many);
