@@ -712,84 +712,20 @@ __global__ void __launch_bounds__(KD_THREADS, PASS == 1 ? 4 : 3) kd_swap_kernel(
     }
     if (PASS == 1 || !kd_last_block(lv.st)) return;
     // ---- split the segments, plan the next level
-    __shared__ uint32_t s_next, s_who, s_run[3];
+    __shared__ uint32_t s_next, s_runs, s_who, s_run[3];
     __shared__ int32_t s_rext[12];
-    if (threadIdx.x == 0) s_next = 0;
+    if (threadIdx.x == 0) s_next = s_runs = 0;
     __syncthreads();
     const uint32_t S = lv.st->segs;
-    const int lane = threadIdx.x & 31;
-    for (uint32_t s0 = 0; s0 < S; s0 += KD_THREADS) {
-        const uint32_t s = s0 + threadIdx.x;
-        const KdSeg sg = lv.segs[min(s, S - 1)];
-        const KdSplit p = lv.sp[min(s, S - 1)];
-        const uint32_t count = sg.end - sg.begin;
-        const uint32_t index = kd_split_index(count, p.L, p.eq);
-        // the split falls among the points at the cut: the extents of the two
-        // parts of that run, read by a warp, or (a long run) by the block
-        const bool in_run = s < S && index > p.L && index < p.L + p.eq;
-        int32_t run[12];
-#pragma unroll
-        for (int k = 0; k < 12; ++k) run[k] = k % 6 < 3 ? INT32_MAX : INT32_MIN;
-        const uint32_t from = sg.begin + p.L, mid = sg.begin + index, to = from + p.eq;
-        if (__syncthreads_or(in_run)) {
-            for (unsigned m = __ballot_sync(0xffffffffu, in_run && p.eq <= KD_WARP_RUN); m; m &= m - 1) {
-                const int src = __ffs(m) - 1;
-                int32_t v[12];
-                kd_run_extents(lv, __shfl_sync(0xffffffffu, from, src), __shfl_sync(0xffffffffu, mid, src),
-                               __shfl_sync(0xffffffffu, to, src), lane, 32u, v);
-                if (lane == src)
-#pragma unroll
-                    for (int k = 0; k < 12; ++k) run[k] = v[k];
-            }
-            bool wait = in_run && p.eq > KD_WARP_RUN;
-            while (__syncthreads_or(wait)) {
-                if (threadIdx.x == 0) s_who = KD_THREADS;
-                if (threadIdx.x < 12) s_rext[threadIdx.x] = threadIdx.x % 6 < 3 ? INT32_MAX : INT32_MIN;
-                __syncthreads();
-                if (wait) atomicMin(&s_who, threadIdx.x);
-                __syncthreads();
-                const bool mine = wait && s_who == threadIdx.x;
-                if (mine) {
-                    s_run[0] = from;
-                    s_run[1] = mid;
-                    s_run[2] = to;
-                }
-                __syncthreads();
-                int32_t v[12];
-                kd_run_extents(lv, s_run[0], s_run[1], s_run[2], threadIdx.x, KD_THREADS, v);
-                if (lane == 0)
-#pragma unroll
-                    for (int k = 0; k < 12; ++k) {
-                        if (k % 6 < 3) atomicMin(&s_rext[k], v[k]);
-                        else atomicMax(&s_rext[k], v[k]);
-                    }
-                __syncthreads();
-                if (mine) {
-                    wait = false;
-#pragma unroll
-                    for (int k = 0; k < 12; ++k) run[k] = s_rext[k];
-                }
-            }
-        }
-        if (s >= S) continue;
+    // children of a segment cut at `index`, with the extents of their points
+    auto split = [&](const KdSeg& sg, const KdSplit& p, uint32_t index, const int32_t (&mn)[2][3],
+                     const int32_t (&mx)[2][3]) {
         const uint32_t cid = atomicAdd(&lv.st->nodes, 2u);
         if (cid + 2 > lv.N.cap) {
             atomicAdd(&lv.st->errors, 1u);
-            continue;
+            return;
         }
         kd_write_children(lv.N, sg.node, cid, p.f, sg.begin, sg.begin + index, sg.end, sg.pad);
-        // the children's extents: the points at the cut go to one side, or (the
-        // split falls among them) to both
-        int32_t mn[2][3], mx[2][3];
-        const int at = index == p.L ? 1 : 0;
-#pragma unroll
-        for (int d = 0; d < 3; ++d)
-#pragma unroll
-            for (int side = 0; side < 2; ++side) {
-                mn[side][d] = min(p.mn[2 * side][d], in_run ? run[6 * side + d] : side == at ? p.mn[1][d] : INT32_MAX);
-                mx[side][d] =
-                    max(p.mx[2 * side][d], in_run ? run[6 * side + 3 + d] : side == at ? p.mx[1][d] : INT32_MIN);
-            }
         for (int side = 0; side < 2; ++side) {
             const uint32_t node = cid + side;
             for (int d = 0; d < 3; ++d) {
@@ -819,6 +755,90 @@ __global__ void __launch_bounds__(KD_THREADS, PASS == 1 ? 4 : 3) kd_swap_kernel(
                 }
             }
         }
+    };
+    for (uint32_t s = threadIdx.x; s < S; s += KD_THREADS) {
+        const KdSeg sg = lv.segs[s];
+        const KdSplit p = lv.sp[s];
+        const uint32_t index = kd_split_index(sg.end - sg.begin, p.L, p.eq);
+        if (index > p.L && index < p.L + p.eq) {  // among the points at the cut: below
+            s_runs = 1;
+            continue;
+        }
+        // the points at the cut go to one side
+        int32_t mn[2][3], mx[2][3];
+        for (int d = 0; d < 3; ++d) {
+            mn[0][d] = p.mn[0][d];
+            mx[0][d] = p.mx[0][d];
+            mn[1][d] = p.mn[2][d];
+            mx[1][d] = p.mx[2][d];
+        }
+        const int at = index == p.L ? 1 : 0;
+        for (int d = 0; d < 3; ++d) {
+            mn[at][d] = min(mn[at][d], p.mn[1][d]);
+            mx[at][d] = max(mx[at][d], p.mx[1][d]);
+        }
+        split(sg, p, index, mn, mx);
+    }
+    __syncthreads();
+    // segments whose split falls among the points at their cut: the extents of the
+    // two parts of that run, read by a warp, or (a long run) by the block
+    const int lane = threadIdx.x & 31;
+    for (uint32_t s0 = 0; s_runs && s0 < S; s0 += KD_THREADS) {
+        const uint32_t s = s0 + threadIdx.x;
+        const KdSeg sg = lv.segs[min(s, S - 1)];
+        const KdSplit p = lv.sp[min(s, S - 1)];
+        const uint32_t index = kd_split_index(sg.end - sg.begin, p.L, p.eq);
+        const bool in_run = s < S && index > p.L && index < p.L + p.eq;
+        const uint32_t from = sg.begin + p.L, mid = sg.begin + index, to = from + p.eq;
+        int32_t run[12];
+        for (unsigned m = __ballot_sync(0xffffffffu, in_run && p.eq <= KD_WARP_RUN); m; m &= m - 1) {
+            const int src = __ffs(m) - 1;
+            int32_t v[12];
+            kd_run_extents(lv, __shfl_sync(0xffffffffu, from, src), __shfl_sync(0xffffffffu, mid, src),
+                           __shfl_sync(0xffffffffu, to, src), lane, 32u, v);
+            if (lane == src)
+#pragma unroll
+                for (int k = 0; k < 12; ++k) run[k] = v[k];
+        }
+        bool wait = in_run && p.eq > KD_WARP_RUN;
+        while (__syncthreads_or(wait)) {
+            if (threadIdx.x == 0) s_who = KD_THREADS;
+            if (threadIdx.x < 12) s_rext[threadIdx.x] = threadIdx.x % 6 < 3 ? INT32_MAX : INT32_MIN;
+            __syncthreads();
+            if (wait) atomicMin(&s_who, threadIdx.x);
+            __syncthreads();
+            const bool mine = wait && s_who == threadIdx.x;
+            if (mine) {
+                s_run[0] = from;
+                s_run[1] = mid;
+                s_run[2] = to;
+            }
+            __syncthreads();
+            int32_t v[12];
+            kd_run_extents(lv, s_run[0], s_run[1], s_run[2], threadIdx.x, KD_THREADS, v);
+            if (lane == 0)
+#pragma unroll
+                for (int k = 0; k < 12; ++k) {
+                    if (k % 6 < 3) atomicMin(&s_rext[k], v[k]);
+                    else atomicMax(&s_rext[k], v[k]);
+                }
+            __syncthreads();
+            if (mine) {
+                wait = false;
+#pragma unroll
+                for (int k = 0; k < 12; ++k) run[k] = s_rext[k];
+            }
+        }
+        if (!in_run) continue;
+        int32_t mn[2][3], mx[2][3];
+#pragma unroll
+        for (int side = 0; side < 2; ++side)
+#pragma unroll
+            for (int d = 0; d < 3; ++d) {
+                mn[side][d] = min(p.mn[2 * side][d], run[6 * side + d]);
+                mx[side][d] = max(p.mx[2 * side][d], run[6 * side + 3 + d]);
+            }
+        split(sg, p, index, mn, mx);
     }
     __syncthreads();
     if (threadIdx.x == 0) lv.st->ticket = 0;
