@@ -37,9 +37,12 @@ struct GridParams {
 // distance field (27 - ob bits) holds (2.2 c)^2, the search's reach at ring 2.
 __host__ __device__ inline uint32_t loc_offset_bits(int32_t c) {
     const uint64_t e = c < 1 ? 1u : c > 8192 ? 8192u : (uint64_t)c;
-    const uint64_t need = (484u * e * e + 99u) / 100u;  // bits: the least with 2^bits >= need
-    int bits = 1;
-    while (bits < 27 && (1ull << bits) < need) ++bits;
+    const uint64_t need = (484u * e * e + 99u) / 100u;  // above 4
+#ifdef __CUDA_ARCH__
+    const int bits = 64 - __clzll((long long)(need - 1u));  // the least with 2^bits >= need
+#else
+    const int bits = 64 - __builtin_clzll(need - 1u);
+#endif
     return bits > 21 ? 6u : bits < 11 ? 16u : (uint32_t)(27 - bits);
 }
 

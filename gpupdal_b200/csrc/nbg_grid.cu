@@ -229,28 +229,6 @@ __global__ void cell_scatter_kernel(const int32_t* __restrict__ x, const int32_t
     }
 }
 
-// The counts of GridParams over the columns this thread takes; all threads of
-// its block take part.
-__device__ __forceinline__ void count_columns(const GridParams& g, const int4* colinfo, const uint32_t* cstart,
-                                              uint32_t entries, uint32_t first, uint32_t step, GridParams* gp) {
-    uint32_t v[3] = {0, 0, 0};
-    for (uint32_t c = first; c < g.ncols; c += step) {
-        const int4 ci = __ldcg(&colinfo[c]);
-        // (a column beyond a table that is too small, which is built again)
-        if (ci.z < ci.y || (uint64_t)(uint32_t)ci.x + (uint32_t)(ci.z - ci.y) + 1 > entries) continue;
-        const uint32_t p = cstart[(uint32_t)ci.x + (uint32_t)(ci.z - ci.y) + 1u] - cstart[(uint32_t)ci.x];
-        v[0] += p > g.full ? p : 0u;
-        v[1] += p < g.thin ? p : 0u;
-        v[2] += p > g.heavy ? p : 0u;
-    }
-    uint32_t* to = &gp->in_full;
-#pragma unroll
-    for (int k = 0; k < 3; ++k) {
-        const uint32_t r = __reduce_add_sync(0xffffffffu, v[k]);
-        if ((threadIdx.x & 31) == 0 && r) atomicAdd(&to[k], r);
-    }
-}
-
 // The scatter's cursors start at the cells' first points; and the columns'
 // counts, which want the same prefix.
 __global__ void __launch_bounds__(256) cell_cursor_kernel(const uint32_t* __restrict__ cstart,
@@ -260,7 +238,22 @@ __global__ void __launch_bounds__(256) cell_cursor_kernel(const uint32_t* __rest
     for (uint64_t i = i0; i < count / 4; i += step) ((uint4*)cursor)[i] = ((const uint4*)cstart)[i];
     if (i0 < (count & 3u)) cursor[(count & ~3ull) + i0] = cstart[(count & ~3ull) + i0];
     const GridParams g = *gpp;
-    count_columns(g, colinfo, cstart, (uint32_t)min(count - 1, (uint64_t)0xFFFFFFFFu), i0, step, gpp);
+    const uint64_t entries = count - 1;
+    uint32_t v[3] = {0, 0, 0};
+    for (uint32_t c = i0; c < g.ncols; c += step) {
+        const int4 ci = colinfo[c];
+        // (a column beyond a table that is too small, which is built again)
+        if (ci.z < ci.y || (uint64_t)(uint32_t)ci.x + (uint32_t)(ci.z - ci.y) + 1 > entries) continue;
+        const uint32_t p = cstart[(uint32_t)ci.x + (uint32_t)(ci.z - ci.y) + 1u] - cstart[(uint32_t)ci.x];
+        v[0] += p > g.full ? p : 0u;
+        v[1] += p < g.thin ? p : 0u;
+        v[2] += p > g.heavy ? p : 0u;
+    }
+#pragma unroll
+    for (int k = 0; k < 3; ++k) {
+        const uint32_t r = __reduce_add_sync(0xffffffffu, v[k]);
+        if ((threadIdx.x & 31) == 0 && r) atomicAdd(&gpp->in_full + k, r);
+    }
 }
 
 // Exclusive prefix sums of v[0 .. count) in place (and into w), by one block of
@@ -389,7 +382,19 @@ __global__ void __launch_bounds__(kSmallThreads) grid_small_kernel(
     }
     __syncthreads();
     block_scan(cstart, cursor, total + 1, part);
-    count_columns(g, colinfo, cstart, total, tid, kSmallThreads, gp);
+    // (of a small tile's counts select_kernel reads the full columns', for lists of
+    // up to 14 slots)
+    if (k1 < 14) {
+        uint32_t full = 0;
+        for (uint32_t c = tid; c < g.ncols; c += kSmallThreads) {
+            const int4 ci = __ldcg(&colinfo[c]);
+            // (beyond the table: extents whose sum passes 32 bits)
+            if (ci.z < ci.y || (uint64_t)(uint32_t)ci.x + (uint32_t)(ci.z - ci.y) + 1 > total) continue;
+            const uint32_t p = cstart[(uint32_t)ci.x + (uint32_t)(ci.z - ci.y) + 1u] - cstart[(uint32_t)ci.x];
+            full += p > g.full ? p : 0u;
+        }
+        if (full) atomicAdd(&gp->in_full, full);
+    }
     for (uint32_t i = tid; i < n; i += kSmallThreads) {
         if (keys[i] == 0xFFFFFFFFu) continue;
         const uint32_t pos = atomicAdd(&cursor[keys[i]], 1u);

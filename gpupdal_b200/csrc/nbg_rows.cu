@@ -312,8 +312,8 @@ __device__ __forceinline__ void retry_finish_rows(const QueryArgs& a, const uint
 template <int NR>
 __global__ void __launch_bounds__(kRowThreads) knn_retry_finish_kernel(const QueryArgs a, uint32_t most) {
     __shared__ uint32_t s_gather[kRowThreads / 32][64];
-    if (*a.nq_dev >= most) return;  // (a thread each)
-    retry_finish_rows<NR>(a, a.rows, *a.nq_dev, s_gather);
+    const uint32_t nr = *a.nq_dev;
+    if (nr < most) retry_finish_rows<NR>(a, a.rows, nr, s_gather);  // (else a thread each)
 }
 
 // The same for the tiles of a batch: blockIdx.y's jobs, gridDim.y apart.
