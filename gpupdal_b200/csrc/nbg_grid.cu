@@ -211,10 +211,10 @@ __global__ void cell_count_kernel(const int32_t* __restrict__ x, const int32_t* 
 }
 
 __global__ void cell_scatter_kernel(const int32_t* __restrict__ x, const int32_t* __restrict__ y,
-                                    const int32_t* __restrict__ z, uint64_t n,
-                                    const GridParams* __restrict__ gpp,
+                                    const int32_t* __restrict__ z, uint64_t n, GridParams* gpp,
                                     const uint32_t* __restrict__ keys, uint32_t* __restrict__ cursor,
-                                    float4* __restrict__ sorted) {
+                                    float4* __restrict__ sorted, const int4* __restrict__ colinfo,
+                                    const uint32_t* __restrict__ cstart, uint64_t entries) {
     const GridParams g = *gpp;
     for (uint64_t i = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x; i < n;
          i += (uint64_t)gridDim.x * blockDim.x) {
@@ -227,20 +227,12 @@ __global__ void cell_scatter_kernel(const int32_t* __restrict__ x, const int32_t
         r.w = __uint_as_float((uint32_t)i);
         sorted[pos] = r;
     }
-}
-
-// The scatter's cursors start at the cells' first points; and the columns'
-// counts, which want the same prefix.
-__global__ void __launch_bounds__(256) cell_cursor_kernel(const uint32_t* __restrict__ cstart,
-                                                          uint32_t* __restrict__ cursor, uint64_t count,
-                                                          const int4* __restrict__ colinfo, GridParams* gpp) {
-    const uint32_t i0 = blockIdx.x * blockDim.x + threadIdx.x, step = gridDim.x * blockDim.x;
-    for (uint64_t i = i0; i < count / 4; i += step) ((uint4*)cursor)[i] = ((const uint4*)cstart)[i];
-    if (i0 < (count & 3u)) cursor[(count & ~3ull) + i0] = cstart[(count & ~3ull) + i0];
-    const GridParams g = *gpp;
-    const uint64_t entries = count - 1;
+    // the counts of GridParams over the columns, beside the scatter: the warps
+    // that have any
+    const uint32_t first = blockIdx.x * blockDim.x + threadIdx.x;
+    if ((first & ~31u) >= g.ncols) return;
     uint32_t v[3] = {0, 0, 0};
-    for (uint32_t c = i0; c < g.ncols; c += step) {
+    for (uint32_t c = first; c < g.ncols; c += gridDim.x * blockDim.x) {
         const int4 ci = colinfo[c];
         // (a column beyond a table that is too small, which is built again)
         if (ci.z < ci.y || (uint64_t)(uint32_t)ci.x + (uint32_t)(ci.z - ci.y) + 1 > entries) continue;
@@ -250,9 +242,9 @@ __global__ void __launch_bounds__(256) cell_cursor_kernel(const uint32_t* __rest
         v[2] += p > g.heavy ? p : 0u;
     }
 #pragma unroll
-    for (int k = 0; k < 3; ++k) {
-        const uint32_t r = __reduce_add_sync(0xffffffffu, v[k]);
-        if ((threadIdx.x & 31) == 0 && r) atomicAdd(&gpp->in_full + k, r);
+    for (int q = 0; q < 3; ++q) {
+        const uint32_t r = __reduce_add_sync(0xffffffffu, v[q]);
+        if ((threadIdx.x & 31) == 0 && r) atomicAdd(&gpp->in_full + q, r);
     }
 }
 
@@ -296,7 +288,7 @@ __device__ uint32_t block_scan(uint32_t* v, uint32_t* w, uint32_t count, uint32_
 // a block should walk, or than the table holds, sets bit 2 of cap_hit and is
 // left to the other builds.
 //
-// Bound by the phases' latency, not by work: fourteen launches and a read of the
+// Bound by the phases' latency, not by work: thirteen launches and a read of the
 // table size between them are what it saves (figures at grid_small).
 __global__ void __launch_bounds__(kSmallThreads) grid_small_kernel(
     const int32_t* x, const int32_t* y, const int32_t* z, const uint32_t n, int k1, float cell_factor,
@@ -634,16 +626,17 @@ int build_grid(Context* ctx, Tile* t, int k1, cudaStream_t stream) {
     if (cub::DeviceScan::ExclusiveSum(t->grid_tmp, tmp, t->cstart, t->cstart, (int)(T + 1),
                                       stream))
         return NBG_ERR_CUDA;
-    cell_cursor_kernel<<<grid_blocks(T / 4, 256, sms), 256, 0, stream>>>(t->cstart, t->cursor, (uint64_t)T + 1,
-                                                                         t->colinfo, t->gp);
+    if (cudaMemcpyAsync(t->cursor, t->cstart, ((size_t)T + 1) * sizeof(uint32_t),
+                        cudaMemcpyDeviceToDevice, stream))
+        return NBG_ERR_CUDA;
     cell_scatter_kernel<<<sb, 256, 0, stream>>>(t->x, t->y, t->z, n, t->gp, t->keys, t->cursor,
-                                                t->sorted);
-    // bbox (2), config, col init, zrange, extent, scan (2), bases, count, scan (2), cursors, scatter
-    NBG_LAUNCHED(14);
+                                                t->sorted, t->colinfo, t->cstart, T);
+    // bbox (2), config, col init, zrange, extent, scan (2), bases, count, scan (2), scatter
+    NBG_LAUNCHED(13);
     return cudaGetLastError() == cudaSuccess ? NBG_OK : NBG_ERR_CUDA;
 }
 
-// One block's build against fourteen launches and two reads by the host: 30 us
+// One block's build against thirteen launches and two reads by the host: 30 us
 // against 87 up to 2000 points, 42 / 86 at 4000, 56 / 84 at 8000, 65 / 86 at
 // 12000, 77 / 89 at 16000 (a call's time as before there), 140 / 88 at 32000.  A
 // cell edge fixed by a radius may give any number of columns: not here.
@@ -697,11 +690,12 @@ int build_grid_async(Context* ctx, Tile* t, int k1, cudaStream_t stream) {
     if (cub::DeviceScan::ExclusiveSum(t->grid_tmp, tmp, t->cstart, t->cstart, (int)(entries + 1),
                                       stream))
         return NBG_ERR_CUDA;
-    cell_cursor_kernel<<<grid_blocks(entries / 4, 256, sms), 256, 0, stream>>>(t->cstart, t->cursor, entries + 1,
-                                                                               t->colinfo, t->gp);
+    if (cudaMemcpyAsync(t->cursor, t->cstart, (size_t)(entries + 1) * sizeof(uint32_t),
+                        cudaMemcpyDeviceToDevice, stream))
+        return NBG_ERR_CUDA;
     cell_scatter_kernel<<<sb, 256, 0, stream>>>(t->x, t->y, t->z, n, t->gp, t->keys, t->cursor,
-                                                t->sorted);
-    NBG_LAUNCHED(14);
+                                                t->sorted, t->colinfo, t->cstart, entries);
+    NBG_LAUNCHED(13);
     t->table_size = entries;
     return cudaGetLastError() == cudaSuccess ? NBG_OK : NBG_ERR_CUDA;
 }
