@@ -45,11 +45,14 @@ BYTES_PER_POINT = 20 + 8 * 7 + 1  # sorted xyz+id, id permutation, 7 f64 outputs
 # records), summarised under profiles/.
 QUERY_PROFILES = {
     0: {"kernel": "knn_select_kernel+knn_finish_kernel",
-        # (182.3 + 628.9) MB / 4e6
-        "traffic": 202.8, "lanes": 8.91, "issue": 0.793, "dram_pct": 0.54},
+        # select (209.9 + 227.0) + finish (345.3 + 323.9) MB / 4e6
+        "traffic": 276.5, "lanes": 8.87, "issue": 0.762, "dram_pct": 1.24},
     2: {"kernel": "knn_select_loc_kernel+knn_retry_finish_kernel+knn_finish_kernel",
-        # select (70.4 + 99.3) + handed-back rows (10.1 + 0.1) + finish (363.1 + 255.5) MB / 4e6
-        "traffic": 199.6, "lanes": 10.13, "issue": 0.662, "dram_pct": 0.58},
+        # select (208.4 + 226.4) + handed-back rows (11.8 + 0.9) + finish MB / 4e6
+        "traffic": 279.2, "lanes": 10.12, "issue": 0.652, "dram_pct": 1.43},
+    32: {"kernel": "knn_group_kernel+knn_retry_finish_kernel+knn_finish_kernel",
+         # select (214.8 + 230.9) + handed-back rows (8.3 + 0.4) + finish MB / 4e6
+         "traffic": 280.9, "lanes": 29.80, "issue": 0.603, "dram_pct": 1.56},
 }
 
 

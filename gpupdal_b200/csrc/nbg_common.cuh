@@ -163,7 +163,7 @@ struct QueryArgs {
     const uint32_t* rows = nullptr;  // split form: the sorted positions to answer (null: all n)
     uint64_t nq = 0;                 // entries of `rows`
     const uint32_t* nq_dev = nullptr;  // entries of `rows` read on the device (retry launches)
-    uint32_t* retry_rows = nullptr;    // group select: rows it hands to the per-thread select
+    uint32_t* retry_rows = nullptr;    // single-pass and group selects: rows they hand back
     // the points the rows index: gv.sorted, or the clump order of the group
     // select (rows and retry_rows then hold its slots), with the boxes of the
     // clumps (ClumpTree)

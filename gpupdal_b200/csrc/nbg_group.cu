@@ -212,7 +212,7 @@ __device__ __forceinline__ void group_warp(const QueryArgs& a, const uint64_t s0
     const uint32_t id = __float_as_uint(q.w);
     const int K = valid ? row_neighbours(a.row_k, a.K, a.n, id) : 0;
     const int qx = __float2int_rz(q.x), qy = __float2int_rz(q.y), qz = __float2int_rz(q.z);
-    bool retry = valid && K <= 0;  // rows without neighbours: the per-thread select
+    bool retry = valid && K <= 0;  // rows without neighbours: the retry launch
     bool done = K <= 0;
     TopK<KS> top;  // the last two slots are the K-th and (K+1)-th
     top.init(done ? 0 : KS - (K + 1));
@@ -410,7 +410,7 @@ __device__ __forceinline__ void group_warp(const QueryArgs& a, const uint64_t s0
             members = false;
         } else if (over) {
             // too many candidates: the lanes start over with the bounds they have
-            // now (a second time the per-thread select takes them)
+            // now (a second time the retry launch takes them)
             if (in && again) retry = done = true;
             if (in && !again) {
                 again = true;
@@ -433,7 +433,7 @@ __device__ __forceinline__ void group_warp(const QueryArgs& a, const uint64_t s0
                                fh0 + (float)m >= (float)(g.maxx - g.minx) && fh1 + (float)m >= (float)(g.maxy - g.miny) &&
                                fh2 + (float)m >= (float)(g.maxz - g.minz);
             if (!next_round && (whole || m >= S::kMaxMargin)) {
-                // fewer than K points in reach: the per-thread select decides
+                // fewer than K points in reach: the retry launch decides
                 if (in) retry = done = true;
                 next_round = true;
             }

@@ -45,14 +45,14 @@ struct Context {
     uint64_t used = 0;     // bytes held by tiles and scratch
     std::string err;
     std::mutex mu;   // held by every entry point that takes the context
-    std::mutex amu;  // the block cache below (the batched form's KD helper thread allocates too)
+    std::mutex amu;  // the block cache below (the server's workers allocate without `mu`)
     std::mutex emu;  // err
     // per-call scratch (grown on demand)
     uint32_t* exact_rows = nullptr;
     uint64_t exact_cap = 0;
     uint2* ties = nullptr;          // tie list of the query kernels
     uint64_t tie_cap = 0;
-    uint32_t* retry_rows = nullptr; // rows the group select hands to the per-thread select
+    uint32_t* retry_rows = nullptr; // rows the single-pass and group selects hand back
     uint64_t retry_cap = 0;
     RowSums* sums = nullptr;        // select -> finish hand-over
     uint64_t sums_cap = 0;

@@ -9,9 +9,9 @@
 // half of this worker's share of the queued points (split over the free
 // workers).  The
 // wave's requests are uploaded, their grids, KD replicas and outputs held on
-// the device, and all of them answered by ONE nbg_run_batch call: a
-// persistent kernel per neighbour-count class drains a device queue of
-// (tile, 128-query block) items across every request of the wave.  Each
+// the device, and all of them answered by ONE nbg_run_batch call: a launch
+// per class (neighbour slots, select kernel) answers the (tile, 128-query
+// block) items of every request of the wave.  Each
 // request's outputs are copied back into its own buffers and its tile freed
 // as the wave ends.  Requests that arrive while a wave runs are admitted into
 // the next free worker's wave (continuous batching: they wait for a worker
